@@ -73,14 +73,11 @@ __device__ __forceinline__ void inv_bf(u32 & x0, u32 & x1, u32 v, u32 vs, u32 p,
 struct TConst
 {
 	u32 p[AB_MAXKP], pinv[AB_MAXKP];
-	u32 one_s[AB_MAXKP];                 // floor(2^32 / p): Shoup constant of 1
-	u32 c32[AB_MAXKP], c32s[AB_MAXKP];   // 2^32 mod p and its Shoup constant
-	u32 c64[AB_MAXKP], c64s[AB_MAXKP];   // 2^64 mod p
-	u32 k95[AB_MAXKP];                   // -2^95 mod p (bias of the signed top limb)
-	u32 crt[AB_MAXKP], crts[AB_MAXKP];   // (2/n) 2^32 (M/p)^-1 mod p: scale and CRT weight of the inverse output
-	u32 fl[AB_MAXKP];                    // floor(2^60 / p): fixed-point 1/p of the CRT quotient estimate
-	u32 mk[AB_MAXKP][AB_MAXK];           // (M/p) mod 2^(32 L), L = K limbs
-	u32 negm[AB_MAXK];                   // -M mod 2^(32 L)
+	u32 enc[AB_MAXKP][3];                // s_k 2^(30 j) 2^32 mod p: encoding weights of a value's 30-bit pieces (encode_res)
+	u32 mk[AB_MAXKP][AB_MAXK];           // e_k M/p_k in radix 2^30, the top entry holding 32 bits (crt)
+	u32 mkh[AB_MAXKP];                   // bits above those 32
+	u32 negm[AB_MAXK], negmh;            // -M mod 2^(32 K) in the same form
+	u32 tinv, tsh;                       // quotient estimate of crt: 2^tsh 2^(32 + 30 (K-1)) / M, times 2^32
 	int K, KP, pck, lbase, ln;           // reference primes K, transform primes KP = K + 1
 	u32 n;                               // 2^ln
 	u32 R, H;                            // column pass: row length and row count of the 2-D layout
@@ -157,53 +154,6 @@ __device__ __forceinline__ Big<L> big_mul_u32(const Big<L> & a, u32 y)
 template <int L>
 __device__ __forceinline__ bool big_is_neg(const Big<L> & a) { return (a.l[L - 1] >> 31) != 0; }
 
-// arithmetic right shift by s, 0 < s < 32L.  s is the same in every thread
-// (it derives from the digit size), so the limb move is a uniform branch and
-// only the sub-limb part is a funnel shift.
-template <int L>
-__device__ __forceinline__ Big<L> big_sar(const Big<L> & a, int s)
-{
-	const u32 fill = big_is_neg<L>(a) ? 0xffffffffu : 0u;
-	u32 t[L + 1];
-#pragma unroll
-	for (int i = 0; i < L; ++i) t[i] = a.l[i];
-	t[L] = fill;
-	int ws = s >> 5;
-	while (ws > 0)
-	{
-#pragma unroll
-		for (int i = 0; i < L; ++i) t[i] = t[i + 1];
-		--ws;
-	}
-	const int bs = s & 31;
-	Big<L> r;
-	if (bs == 0)
-	{
-#pragma unroll
-		for (int i = 0; i < L; ++i) r.l[i] = t[i];
-	}
-	else
-	{
-#pragma unroll
-		for (int i = 0; i < L; ++i) r.l[i] = __funnelshift_r(t[i], t[i + 1], bs);
-	}
-	return r;
-}
-
-// v as L two's-complement limbs (v fits 32L bits)
-template <int L>
-__device__ __forceinline__ Big<L> big_from_i128(__int128 v)
-{
-	Big<L> r;
-	const u32 s = (v < 0) ? 0xffffffffu : 0u;
-#pragma unroll
-	for (int i = 0; i < L; ++i) r.l[i] = (i < 4) ? (u32)((unsigned __int128)v >> (32 * i)) : s;
-	return r;
-}
-
-template <int L>
-__device__ __forceinline__ u64 big_low64(const Big<L> & a) { return (u64)a.l[0] | ((u64)a.l[1] << 32); }
-
 // a 96-bit exact value (three limbs) sign-extended or truncated to L limbs
 template <int L>
 __device__ __forceinline__ Big<L> big_from_exact(u32 d0, u32 d1, u32 d2)
@@ -216,164 +166,126 @@ __device__ __forceinline__ Big<L> big_from_exact(u32 d0, u32 d1, u32 d2)
 }
 
 // ---------------------------------------------------------------- CRT
-// acc += y m (mod 2^(32L)): two carry chains, low halves then high halves.
+// Every forward image carries a factor s_k per prime (encode_res), chosen so
+// that the inverse output of a product, (n/2) 2^-32 s_k^2 V mod p_k, is already
+// the CRT coordinate of V: s_k^2 e_k = (2/n) 2^32 (M/p_k)^-1 mod p_k, with e_k
+// = 1, or the least non-residue mod p_k when that quotient is not a square.
+// So V = sum y_k e_k (M/p_k) - t M for ANY representative y_k of the inverse
+// output (here [0, 2p_k), as the lazy levels leave it): no product and no
+// reduction per residue.  t = round(S / M), S the sum: S / M lies within
+// |V| / M < 2^-18 of the integer t, so its top 32 bits decide t.
+//
+// S is summed in radix 2^30, one 64-bit column per limb: the integer
+// multiplier is what bounds the column pass (B200: IMAD 64, IMAD.HI and
+// IMAD.WIDE 32 per clock and SM), and 2^31 2^30 products of 6 primes fit a
+// column with no carry chain, so a limb product costs one IMAD.WIDE (2 units)
+// where a 32-bit limb costs a low and a high product (3).  Computed mod
+// 2^(32 L), where V fits.
 template <int L>
-__device__ __forceinline__ void big_mad_u32(u32 (&a)[L], u32 y, const u32 (&m)[AB_MAXK])
-{
-	if constexpr (L == 2)
-	{
-		asm("mad.lo.cc.u32 %0, %2, %3, %0;\n\t"
-		    "madc.lo.u32 %1, %2, %4, %1;\n\t"
-		    "mad.hi.u32 %1, %2, %3, %1;"
-		    : "+r"(a[0]), "+r"(a[1]) : "r"(y), "r"(m[0]), "r"(m[1]));
-	}
-	else if constexpr (L == 3)
-	{
-		asm("mad.lo.cc.u32 %0, %3, %4, %0;\n\t"
-		    "madc.lo.cc.u32 %1, %3, %5, %1;\n\t"
-		    "madc.lo.u32 %2, %3, %6, %2;\n\t"
-		    "mad.hi.cc.u32 %1, %3, %4, %1;\n\t"
-		    "madc.hi.u32 %2, %3, %5, %2;"
-		    : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]) : "r"(y), "r"(m[0]), "r"(m[1]), "r"(m[2]));
-	}
-	else if constexpr (L == 4)
-	{
-		asm("mad.lo.cc.u32 %0, %4, %5, %0;\n\t"
-		    "madc.lo.cc.u32 %1, %4, %6, %1;\n\t"
-		    "madc.lo.cc.u32 %2, %4, %7, %2;\n\t"
-		    "madc.lo.u32 %3, %4, %8, %3;\n\t"
-		    "mad.hi.cc.u32 %1, %4, %5, %1;\n\t"
-		    "madc.hi.cc.u32 %2, %4, %6, %2;\n\t"
-		    "madc.hi.u32 %3, %4, %7, %3;"
-		    : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]) : "r"(y), "r"(m[0]), "r"(m[1]), "r"(m[2]), "r"(m[3]));
-	}
-	else
-	{
-		static_assert(L == 5, "2 to 5 limbs");
-		asm("mad.lo.cc.u32 %0, %5, %6, %0;\n\t"
-		    "madc.lo.cc.u32 %1, %5, %7, %1;\n\t"
-		    "madc.lo.cc.u32 %2, %5, %8, %2;\n\t"
-		    "madc.lo.cc.u32 %3, %5, %9, %3;\n\t"
-		    "madc.lo.u32 %4, %5, %10, %4;\n\t"
-		    "mad.hi.cc.u32 %1, %5, %6, %1;\n\t"
-		    "madc.hi.cc.u32 %2, %5, %7, %2;\n\t"
-		    "madc.hi.cc.u32 %3, %5, %8, %3;\n\t"
-		    "madc.hi.u32 %4, %5, %9, %4;"
-		    : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4])
-		    : "r"(y), "r"(m[0]), "r"(m[1]), "r"(m[2]), "r"(m[3]), "r"(m[4]));
-	}
-}
-
-// Exact signed value V of a coefficient from its KP = L + 1 residues r_k in
-// [0, 2p_k), which hold (n/2) 2^-32 V (the unnormalised inverse transform of a
-// Montgomery pointwise product).  With y_k = r_k crt_k mod p_k in [0, p_k),
-// V = sum y_k (M/p_k) - t M, t = round(sum y_k / p_k): the sum of fractions
-// lies within |V|/M < 2^-18 of the integer t, so a 60-bit fixed-point estimate
-// decides t exactly.  Computed mod 2^(32L), where V fits.
-template <int L>
-__device__ __forceinline__ Big<L> crt(const TConst & c, const u32 (&r)[L + 1])
+__device__ __forceinline__ Big<L> crt(const TConst & c, const u32 (&y)[L + 1])
 {
 	constexpr int KP = L + 1;
-	u32 y[KP];
-	u64 est = 0;
+	u64 col[L];
 #pragma unroll
-	for (int k = 0; k < KP; ++k)
+	for (int j = 0; j < L; ++j)
 	{
-		const u32 p = c.p[k];
-		const u32 v = shoup(r[k], c.crt[k], c.crts[k], p);
-		y[k] = min(v, v - p);
-		est += (u64)y[k] * c.fl[k];
+		u64 s = (u64)y[0] * c.mk[0][j];
+#pragma unroll
+		for (int k = 1; k < KP; ++k) s += (u64)y[k] * c.mk[k][j];
+		col[j] = s;
 	}
-	const u32 t = (u32)((est + (1ull << 59)) >> 60);
-	u32 a[L];
+	// only e_3 = 11 of the class L = 4 needs a 33rd bit
+	if (L == 4) col[L - 1] += (u64)(y[3] * c.mkh[3]) << 32;
+	const u32 hi = (u32)((col[L - 1] + (col[L - 2] >> 30)) >> 32);
+	const u32 t = (__umulhi(hi, c.tinv) + (1u << (c.tsh - 1))) >> c.tsh;
 #pragma unroll
-	for (int i = 0; i < L; ++i) a[i] = 0;
-	big_mad_u32<L>(a, t, c.negm);
+	for (int j = 0; j < L; ++j) col[j] += (u64)t * c.negm[j];
+	col[L - 1] += (u64)(t * c.negmh) << 32;
 #pragma unroll
-	for (int k = 0; k < KP; ++k) big_mad_u32<L>(a, y[k], c.mk[k]);
+	for (int j = 1; j < L; ++j) col[j] += col[j - 1] >> 30;
 	Big<L> V;
 #pragma unroll
-	for (int i = 0; i < L; ++i) V.l[i] = a[i];
+	for (int i = 0; i < L - 1; ++i) V.l[i] = __funnelshift_r((u32)col[i] << 2, (u32)col[i + 1], 2 + 2 * i);
+	V.l[L - 1] = (u32)(col[L - 1] >> (2 * (L - 1)));
 	return V;
 }
 
-// Residue in [0, 3p) of the exact value (d0, d1, d2) (two's complement): d0 +
-// 2^32 d1 + 2^64 (d2 ^ 2^31) - 2^95.
-__device__ __forceinline__ u32 encode_res(const TConst & c, int k, u32 d0, u32 d1, u32 d2u)
+// The 30-bit pieces of an exact value (three limbs, |v| < 2^91): v = a0 +
+// 2^30 a1 + 2^60 a2, a2 signed.
+struct Pieces
 {
-	const u32 p = c.p[k], p2 = 2 * p;
-	const u32 a = d0 - __umulhi(d0, c.one_s[k]) * p;
-	const u32 b = shoup(d1, c.c32[k], c.c32s[k], p);
-	const u32 e = shoup(d2u, c.c64[k], c.c64s[k], p);
-	u32 s = red2(a + b, p2);
-	s = red2(s + e, p2);
-	return s + c.k95[k];
+	u32 a0, a1;
+	i32 a2;
+};
+__device__ __forceinline__ Pieces split30(u32 d0, u32 d1, u32 d2)
+{
+	constexpr u32 M30 = (1u << 30) - 1;
+	return Pieces{ d0 & M30, __funnelshift_r(d0, d1, 30) & M30, (i32)__funnelshift_r(d1, d2, 28) };
+}
+
+// s_k v mod p_k in (0, 3p): one Montgomery reduction of the 64-bit sum of the
+// weighted pieces (its high word lies in (-p/2, p)).
+__device__ __forceinline__ u32 encode_res(const TConst & c, int k, const Pieces & a)
+{
+	const u32 p = c.p[k];
+	u64 s = (u64)a.a0 * c.enc[k][0];
+	s += (u64)a.a1 * c.enc[k][1];
+	s += (u64)((i64)a.a2 * (i32)c.enc[k][2]);
+	return (u32)(s >> 32) - __umulhi((u32)s * c.pinv[k], p) + 2 * p;
 }
 
 // ---------------------------------------------------------------- digits
-// Unsigned digits of the low pck*lbase bits of f, then f >>= pck*lbase
-// (ocl/kernel.cl:1478-1537).
-template <int L, int PCK>
-__device__ __forceinline__ void extract_shift(Big<L> & f, int lb, u32 (&d)[PCK])
+// A coefficient is pck digits of lbase bits; the carry rule (unsigned digits,
+// the top one balanced; ocl/kernel.cl:1478-1537) only depends on the
+// coefficient as one digit of W = pck lbase bits, W = 32 ws + bs.  W is the
+// same in every thread, so the limb moves are uniform branches.
+struct Width
 {
-	const u32 bm = (1u << lb) - 1;
-	const u64 low = big_low64<L>(f);
-	if (PCK == 1)
-	{
-		d[0] = (u32)low & bm;
-		f = big_sar<L>(f, lb);
-	}
-	else
-	{
-		const u64 r01 = low & (((u64)1 << (2 * lb)) - 1);
-		d[0] = (u32)r01 & bm;
-		d[1] = (u32)(r01 >> lb);
-		f = big_sar<L>(f, 2 * lb);
-		if (PCK == 4)
-		{
-			const u64 r23 = big_low64<L>(f) & (((u64)1 << (2 * lb)) - 1);
-			d[2 % PCK] = (u32)r23 & bm;
-			d[3 % PCK] = (u32)(r23 >> lb);
-			f = big_sar<L>(f, 2 * lb);
-		}
-	}
+	int ws, bs;
+	u32 mask;                            // low bs bits
+};
+__device__ __forceinline__ Width make_width(int w)
+{
+	return Width{ w >> 5, w & 31, (1u << (w & 31)) - 1 };
 }
 
-// f + (d_0 + d_1 base + ... ) with unsigned digits
-template <int L, int PCK>
-__device__ __forceinline__ Big<L> add_digits(const Big<L> & f, int lb, const u32 (&d)[PCK])
-{
-	Big<L> t = big_zero<L>();
-	if (PCK == 1) { t.l[0] = d[0]; }
-	else
-	{
-		const u64 r01 = (u64)d[0] | ((u64)d[1] << lb);
-		if (PCK == 2) { t.l[0] = (u32)r01; t.l[1] = (u32)(r01 >> 32); }
-		else
-		{
-			const u64 r23 = (u64)d[2 % PCK] | ((u64)d[3 % PCK] << lb);
-			// value = r01 + r23 * 2^(2 lb), 2 lb <= 62
-			const int s = 2 * lb;
-			const u64 lo = r01 | (r23 << s);
-			const u64 hi = r23 >> (64 - s);
-			t.l[0] = (u32)lo; t.l[1] = (u32)(lo >> 32);
-			if (L > 2) t.l[2 % L] = (u32)hi;
-			if (L > 3) t.l[3 % L] = (u32)(hi >> 32);
-		}
-	}
-	return big_add<L>(f, t);
-}
-
-// Exact value of a balanced coefficient (unsigned digits e_0 .. e_{PCK-2},
-// signed top digit, base 2^lb) as three two's-complement limbs.
+// Limbs that hold W bits: lbase <= 31, pck lbase <= 80.
 template <int PCK>
-__device__ __forceinline__ void digits_exact(int lb, i32 top, const u32 (&e)[PCK], u32 & d0, u32 & d1, u32 & d2)
+struct DigitLimbs { static constexpr int N = (PCK == 1) ? 1 : (PCK == 2) ? 2 : 3; };
+
+// d = the low W bits of f (unsigned), f >>= W (arithmetic).
+template <int L, int ND>
+__device__ __forceinline__ void split_digit(Big<L> & f, const Width & w, u32 (&d)[ND])
 {
-	__int128 v = (__int128)top;
+	const u32 fill = (u32)((i32)f.l[L - 1] >> 31);
+	u32 t[L + 1];
 #pragma unroll
-	for (int l = PCK - 2; l >= 0; --l) v = (v << lb) + (__int128)e[l];
-	const unsigned __int128 u = (unsigned __int128)v;
-	d0 = (u32)u; d1 = (u32)(u >> 32); d2 = (u32)(u >> 64);
+	for (int i = 0; i < L; ++i) t[i] = f.l[i];
+	t[L] = fill;
+#pragma unroll
+	for (int i = 0; i < ND; ++i) d[i] = (i < w.ws) ? t[i % L] : (i == w.ws) ? t[i % L] & w.mask : 0u;
+	if (ND > 1 && w.ws >= 1)
+	{
+#pragma unroll
+		for (int i = 0; i < L; ++i) t[i] = t[i + 1];
+	}
+	if (ND > 2 && w.ws >= 2)
+	{
+#pragma unroll
+		for (int i = 0; i < L; ++i) t[i] = t[i + 1];
+	}
+#pragma unroll
+	for (int i = 0; i < L; ++i) f.l[i] = __funnelshift_r(t[i], t[i + 1], w.bs);
+}
+
+// f + d (d unsigned)
+template <int L, int ND>
+__device__ __forceinline__ Big<L> add_digit(const Big<L> & f, const u32 (&d)[ND])
+{
+	Big<L> t;
+#pragma unroll
+	for (int i = 0; i < L; ++i) t.l[i] = (i < ND) ? d[i % ND] : 0u;
+	return big_add<L>(f, t);
 }
 
 // ---------------------------------------------------------------- reference primes

@@ -89,6 +89,22 @@ struct TZp
 	u32 pow(u32 x, u64 e) const { u32 r = 1; while (e) { if (e & 1) r = mul(r, x); x = mul(x, x); e >>= 1; } return r; }
 	u32 inv(u32 x) const { return pow(x, p - 2); }
 	u32 shoup(u32 w) const { return (u32)(((u64)w << 32) / p); }
+	bool is_square(u32 x) const { return pow(x, (p - 1) / 2) == 1; }
+	// a square root of the square x (Tonelli-Shanks; p - 1 = odd 2^23 at least)
+	u32 sqrt(u32 x) const
+	{
+		u32 q = p - 1; int m = 0;
+		while ((q & 1) == 0) { q >>= 1; ++m; }
+		u32 g = 2; while (is_square(g)) ++g;
+		u32 c = pow(g, q), t = pow(x, q), r = pow(x, (q + 1) / 2);
+		while (t != 1)
+		{
+			int i = 0; for (u32 y = t; y != 1; y = mul(y, y)) ++i;
+			u32 b = c; for (int j = 0; j < m - i - 1; ++j) b = mul(b, b);
+			m = i; c = mul(b, b); t = mul(t, c); r = mul(r, b);
+		}
+		return r;
+	}
 };
 
 size_t bitrev(size_t i, size_t n)
@@ -313,23 +329,36 @@ struct ab_transform
 		mpz_clears(N, factor, nullptr);
 	}
 
+	// The weights of encode_res for prime k and image factor s: s 2^(30 j), times
+	// 2^32 for its Montgomery reduction.
+	static void encode_weights(TConst & tc, int k, u32 s)
+	{
+		const TZp z(TPRIMES[k]);
+		u32 x = z.mul(s, (u32)(((u64)1 << 32) % z.p));
+		for (int j = 0; j < 3; ++j) { tc.enc[k][j] = x; x = z.mul(x, (u32)(((u64)1 << 30) % z.p)); }
+	}
+
 	// Constants of the transform primes (TConst) and of the reference primes
 	// (RefConst) for the class (K, pck, ln) and digit size lbase.
 	static void build_consts(const ab_params & prm, const Geometry & geo, TConst & tc, RefConst & rc)
 	{
-		const int K = prm.K, KP = K + 1, L = K;
+		const int K = prm.K, KP = K + 1;
 		const size_t n = (size_t)1 << prm.ln;
 		std::memset(&tc, 0, sizeof(tc));
 		tc.K = K; tc.KP = KP; tc.pck = prm.pck; tc.lbase = prm.lbase; tc.ln = prm.ln;
 		tc.n = (u32)n;
 		apply_geometry(tc, geo);
-		mpz_t M, Mk, t, mod; mpz_inits(M, Mk, t, mod, nullptr);
+		mpz_t M, Mk, S, t, mod; mpz_inits(M, Mk, S, t, mod, nullptr);
 		mpz_set_ui(M, 1);
 		for (int k = 0; k < KP; ++k) mpz_mul_ui(M, M, TPRIMES[k]);
-		mpz_set_ui(mod, 1); mpz_mul_2exp(mod, mod, (mp_bitcnt_t)32 * L);
-		auto limbs = [&](const mpz_t v, u32 * out) {
-			mpz_fdiv_r(t, v, mod);
-			for (int j = 0; j < L; ++j) { out[j] = (u32)mpz_get_ui(t); mpz_fdiv_q_2exp(t, t, 32); }
+		mpz_set_ui(mod, 1); mpz_mul_2exp(mod, mod, (mp_bitcnt_t)32 * K);
+		// radix 2^30, the top entry 32 bits and what lies above them in `high`
+		auto columns = [&](const mpz_t v, u32 * out, u32 & high) {
+			mpz_set(t, v);
+			for (int j = 0; j < K - 1; ++j) { out[j] = (u32)mpz_get_ui(t) & ((1u << 30) - 1); mpz_fdiv_q_2exp(t, t, 30); }
+			out[K - 1] = (u32)mpz_get_ui(t);
+			mpz_fdiv_q_2exp(t, t, 32);
+			high = (u32)mpz_get_ui(t);
 		};
 		for (int k = 0; k < KP; ++k)
 		{
@@ -338,23 +367,38 @@ struct ab_transform
 			tc.p[k] = p;
 			u32 pinv = 1; for (int i = 0; i < 6; ++i) pinv *= 2 - p * pinv;
 			tc.pinv[k] = pinv;
-			tc.one_s[k] = z.shoup(1);
-			tc.c32[k] = (u32)(((u64)1 << 32) % p); tc.c32s[k] = z.shoup(tc.c32[k]);
-			tc.c64[k] = z.mul(tc.c32[k], tc.c32[k]); tc.c64s[k] = z.shoup(tc.c64[k]);
-			const u32 p95 = z.mul(tc.c64[k], (u32)(((u64)1 << 31) % p));
-			tc.k95[k] = (p - p95) % p;
 			mpz_divexact_ui(Mk, M, p);
-			const u32 mk_mod_p = (u32)mpz_fdiv_ui(Mk, p);
 			// (2/n) 2^32 (M/p)^-1: undoes the n/2 of the inverse levels and the
-			// 2^-32 of the Montgomery pointwise product, and weights the CRT
-			tc.crt[k] = z.mul(z.mul(z.inv((u32)((n / 2) % p)), tc.c32[k]), z.inv(mk_mod_p));
-			tc.crts[k] = z.shoup(tc.crt[k]);
-			tc.fl[k] = (u32)(((u64)1 << 60) / p);
-			limbs(Mk, tc.mk[k]);
+			// 2^-32 of the Montgomery pointwise product, and weights the CRT.
+			// Both factors of a product carry s_k with s_k^2 = that / e_k, so the
+			// inverse output needs no product of its own (crt).
+			const u32 cw = z.mul(z.mul(z.inv((u32)((n / 2) % p)), (u32)(((u64)1 << 32) % p)), z.inv((u32)mpz_fdiv_ui(Mk, p)));
+			u32 e = 1;
+			while (!z.is_square(z.mul(cw, z.inv(e)))) ++e;
+			encode_weights(tc, k, z.sqrt(z.mul(cw, z.inv(e))));
+			mpz_mul_ui(Mk, Mk, e);
+			columns(Mk, tc.mk[k], tc.mkh[k]);
+			// the top column of the CRT sum must fit 64 bits, and its operands 32
+			// (a 33rd bit only where crt<4> adds it)
+			if (tc.mkh[k] != 0 && !(K == 4 && k == 3)) throw ab_error(AB_E_ARG, "CRT weight beyond 32 bits");
+			mpz_mul_ui(Mk, Mk, 2 * p);
+			mpz_add(S, S, Mk);
 		}
+		mpz_fdiv_q_2exp(t, S, (mp_bitcnt_t)30 * (K - 1));
+		if (mpz_sizeinbase(t, 2) > 64) throw ab_error(AB_E_ARG, "CRT sum beyond 64 bits");
+		// 1 / M as 2^tsh 2^(32 + 30 (K - 1)) / M in [2^30, 2^32) / 2^32
+		int sh = 0;
+		do
+		{
+			++sh;
+			mpz_set_ui(t, 1); mpz_mul_2exp(t, t, (mp_bitcnt_t)(64 + 30 * (K - 1) + sh));
+			mpz_fdiv_q(t, t, M);
+		} while (mpz_sizeinbase(t, 2) < 31);
+		tc.tinv = (u32)mpz_get_ui(t); tc.tsh = (u32)sh;
 		mpz_neg(t, M);
-		limbs(t, tc.negm);
-		mpz_clears(M, Mk, t, mod, nullptr);
+		mpz_fdiv_r(t, t, mod);
+		columns(t, tc.negm, tc.negmh);
+		mpz_clears(M, Mk, S, t, mod, nullptr);
 
 		std::memset(&rc, 0, sizeof(rc));
 		rc.K = K;
@@ -1292,8 +1336,16 @@ int ab_diag_forward(ab_transform * h, int domain, const uint32_t * in, uint32_t 
 		using T = ab_transform;
 		h->upload(T::XW, in);
 		if (!h->import_words(T::TMP)) throw ab_error(AB_E_ARG, "input is not a normal-form register");
-		if (domain) h->full_forward(h->b(T::TMP), h->b(T::AQ1), nullptr);
-		else h->full_forward(h->b(T::TMP), nullptr, h->b(T::AQ1));
+		// plain residues: the engine's own images carry a factor per prime
+		const TConst scaled = h->tc;
+		for (int k = 0; k < h->KP; ++k) T::encode_weights(h->tc, k, 1u);
+		try
+		{
+			if (domain) h->full_forward(h->b(T::TMP), h->b(T::AQ1), nullptr);
+			else h->full_forward(h->b(T::TMP), nullptr, h->b(T::AQ1));
+		}
+		catch (...) { h->tc = scaled; throw; }
+		h->tc = scaled;
 		h->download(T::AQ1, out, (size_t)h->KP * h->n);
 		h->prefwd = false;
 	});
@@ -1876,7 +1928,7 @@ struct ab_mixed
 				for (int i = 0; i < nc; ++i)
 				{
 					const ab_batch & x = *b[i];
-					f.nbx[i] = x.geo.RC / (u32)x.geo.C;
+					f.nbx[i] = x.geo.NC;
 					f.njobs[i] = (u32)lists[i][q].nj;
 					f.sel[i] = x.geo.LA * 8 + x.cls.K;
 					f.jobs[i] = lists[i][q].cj;

@@ -14,8 +14,8 @@
 // and they do not depend on the primes or the order of the butterflies.
 //
 // This file splits the n coefficients 2-D (row*R + col): the column pass owns
-// the first LA levels (all H rows of 32 adjacent columns, all KP primes, in
-// shared memory) and the row pass owns the last LB levels (one row of one
+// the first LA levels (all H rows of up to 28 adjacent columns, all KP primes,
+// in shared memory) and the row pass owns the last LB levels (one row of one
 // prime per CTA, 16 coefficients per thread in registers).
 #include <atomic>
 #include <utility>
@@ -398,32 +398,53 @@ __global__ void __launch_bounds__(RowCfg<LOG_R>::NT, RowCfg<LOG_R>::MINB) k_rowp
 }
 
 // ================================================================ column pass
-constexpr int CC = 32;  // own columns per CTA
-#ifndef AB_COL_THREADS
-#define AB_COL_THREADS 384
+// A CTA's tile is CW = 32 columns wide, one lane per column: E predecessor
+// columns, whose groups only give the carry into the CTA's first group, then
+// the CTA's own columns.  CTA 0 has E = 8 (the mod R / mod Q decision needs
+// the final value of the register's last coefficient, whose own predecessor
+// group is the 4 columns before it) and 24 own columns, the others E = 4 and
+// up to 28; a row of 32 columns is a single CTA without predecessors.  So every
+// butterfly task is a full warp of 32 adjacent columns, and a tile row is
+// 128 bytes of shared memory without padding.
+constexpr int CW = 32;
+__host__ __device__ constexpr u32 col_ctas(u32 RC) { return (RC <= 32) ? 1u : 1u + (RC - 24u + 27u) / 28u; }
+
+// Threads of a column-pass CTA: the carry phases have 8 groups of 4 columns
+// per row, the butterfly stages KP / 8 times 32 tasks per row, so the thread
+// count follows the number of rows.
+#ifndef AB_COL_TPR
+#define AB_COL_TPR 8
 #endif
-constexpr int COL_THREADS = AB_COL_THREADS;
-constexpr int TW = 40;  // tile row stride: own columns + up to 8 predecessor columns
+#ifndef AB_COL_REGT
+#define AB_COL_REGT 1024
+#endif
+constexpr int COL_THREADS = 384;                       // fused kernels: every split in one launch
+template <int LOG_H>
+struct ColCfg
+{
+	static constexpr int NT = ((AB_COL_TPR << LOG_H) < 64) ? 64 : (AB_COL_TPR << LOG_H);
+	static constexpr int MINB = (AB_COL_REGT / NT < 16) ? AB_COL_REGT / NT : 16;
+};
 
 // One radix-2^S step of the column transform (levels on row bits b..b+S-1)
-// for one column of one prime: the 2^S rows that differ in those bits.
+// for one column of one prime: the 2^S rows that differ in those bits, read
+// from src and written to dst (tile or global, row strides ss and ds).
 // Global level l (2^l polynomials) works on row bit LOG_H-1-l with twiddle
 // tw[2^l + j], j = row >> (LOG_H - l) (forward: w; inverse: -w^-1).
 template <int S, bool INV>
-__device__ __forceinline__ void col_step(u32 * __restrict__ colp, int LOG_H, int b, u32 o, const uint2 * __restrict__ tw,
-	u32 p, u32 p2)
+__device__ __forceinline__ void col_step(const u32 * src, u32 ss, u32 * dst, u32 ds, int LOG_H, int b, u32 o,
+	const uint2 * __restrict__ tw, u32 p, u32 p2)
 {
 	u32 v[1 << S];
 	const u32 row0 = (o & ((1u << b) - 1)) | ((o >> b) << (b + S));
-	u32 * const base = colp + row0 * TW;
-	const u32 D = (u32)TW << b;
+	const u32 * const sp = src + row0 * ss;
 #pragma unroll
-	for (int g = 0; g < (1 << S); ++g) v[g] = base[g * D];
+	for (int g = 0; g < (1 << S); ++g) v[g] = sp[((u32)g << b) * ss];
 	const u32 ohi = o >> b;
 #pragma unroll
-	for (int ss = 0; ss < S; ++ss)
+	for (int t = 0; t < S; ++t)
 	{
-		const int s = INV ? ss : (S - 1 - ss);
+		const int s = INV ? t : (S - 1 - t);
 		const int lvl = LOG_H - 1 - (b + s);
 		const uint2 * __restrict__ twl = tw + ((1u << lvl) + (ohi << (S - 1 - s)));
 #pragma unroll
@@ -439,140 +460,142 @@ __device__ __forceinline__ void col_step(u32 * __restrict__ colp, int LOG_H, int
 			}
 		}
 	}
+	u32 * const dp = dst + row0 * ds;
 #pragma unroll
-	for (int g = 0; g < (1 << S); ++g) base[g * D] = v[g];
+	for (int g = 0; g < (1 << S); ++g) dp[((u32)g << b) * ds] = v[g];
 }
 
-// One task of a column stage: column u of prime k, row group o.
-template <int LOG_H, bool INV>
-__device__ __forceinline__ void col_task(u32 * tile, int u, int o, int k, int S, int b, const uint2 * twk, const TConst & c)
+// The LOG_H column levels in at most two stages: the bottom SB row bits and
+// the other ST ones.
+template <int LOG_H>
+struct ColStages
 {
-	u32 * colp = tile + (k << LOG_H) * TW + u;
-	const uint2 * tw = twk + (k << LOG_H);
-	const u32 p = c.p[k];
-	if (S == 3) col_step<3, INV>(colp, LOG_H, b, (u32)o, tw, p, 2 * p);
-	else if (S == 2) col_step<2, INV>(colp, LOG_H, b, (u32)o, tw, p, 2 * p);
-	else col_step<1, INV>(colp, LOG_H, b, (u32)o, tw, p, 2 * p);
-}
+	static constexpr int ST = (LOG_H > 3) ? LOG_H / 2 : 0, SB = LOG_H - ST;
+};
 
-// All LOG_H levels of the CC own columns [E, E + CC) and, with pred, the E
-// predecessor columns [0, E) of every prime, in place in the tile; stages of
-// 3 levels (the remainder first in the forward order).  Task indices split
-// by shifts only (E is 0, 4 or 8).
-template <int LOG_H, int KP, bool INV>
-__device__ __forceinline__ void col_transform(u32 * tile, int E, bool pred, const uint2 * twk, const TConst & c)
+// Inverse levels of every tile column, from global memory (x: plane 0, row 0)
+// into the tile.
+template <int LOG_H, int KP>
+__device__ __forceinline__ void col_inverse(const u32 * __restrict__ x, u32 n, u32 R, u32 gc, bool live, u32 * tile, const uint2 * twk, const TConst & c)
 {
-	constexpr int SR = (LOG_H % 3 == 0) ? 3 : LOG_H % 3;       // top stage (row bits LOG_H-SR..LOG_H-1)
-	constexpr int NST = 1 + (LOG_H - SR) / 3;
-	static_assert(CC == 32, "32 own columns per CTA");
-	const int tid = (int)threadIdx.x, NT = (int)blockDim.x;
-	const int le = (E == 8) ? 3 : 2;                           // log2 E when E > 0
-#pragma unroll 1
-	for (int st = 0; st < NST; ++st)
+	constexpr int SB = ColStages<LOG_H>::SB, ST = ColStages<LOG_H>::ST, PS = CW << LOG_H;
+	const int tid = (int)threadIdx.x, NT = (int)blockDim.x, u = tid & 31;
+	for (int task = tid; task < (KP << (LOG_H - SB + 5)); task += NT)
 	{
-		// forward: top stage first; inverse: bottom stage first
-		const int idx = INV ? (NST - 1 - st) : st;
-		const bool top = (idx == 0);
-		const int b = top ? (LOG_H - SR) : (LOG_H - SR - 3 * idx);
-		const int S = top ? SR : 3;
-		const int lo = LOG_H - S;                                // log2 of the row groups
-		for (int task = tid; task < (KP << (lo + 5)); task += NT)
-			col_task<LOG_H, INV>(tile, E + (task & 31), (task >> 5) & ((1 << lo) - 1), task >> (lo + 5), S, b, twk, c);
-		if (pred && E > 0)
-			for (int task = tid; task < (KP << (lo + le)); task += NT)
-				col_task<LOG_H, INV>(tile, task & (E - 1), (task >> le) & ((1 << lo) - 1), task >> (lo + le), S, b, twk, c);
+		const int o = (task >> 5) & ((1 << (LOG_H - SB)) - 1), k = task >> (LOG_H - SB + 5);
+		const u32 p = c.p[k];
+		if (live) col_step<SB, true>(x + (size_t)k * n + gc, R, tile + k * PS + u, CW, LOG_H, 0, (u32)o, twk + (k << LOG_H), p, 2 * p);
+	}
+	__syncthreads();
+	if constexpr (ST > 0)
+	{
+		for (int task = tid; task < (KP << (LOG_H - ST + 5)); task += NT)
+		{
+			const int o = (task >> 5) & ((1 << (LOG_H - ST)) - 1), k = task >> (LOG_H - ST + 5);
+			const u32 p = c.p[k];
+			col_step<ST, true>(tile + k * PS + u, CW, tile + k * PS + u, CW, LOG_H, SB, (u32)o, twk + (k << LOG_H), p, 2 * p);
+		}
 		__syncthreads();
 	}
 }
 
-// Adds delta to the exact value of one coefficient (three limb planes, plane
-// stride PS words).
-__device__ __forceinline__ void exact_add(u32 * t, int PS, __int128 delta)
+// Forward levels of the own columns, from the tile into global memory.
+template <int LOG_H, int KP>
+__device__ __forceinline__ void col_forward(u32 * tile, u32 * __restrict__ x, u32 n, u32 R, u32 gc, bool own, const uint2 * twk, const TConst & c)
 {
-	const unsigned __int128 u = (unsigned __int128)t[0] | ((unsigned __int128)t[PS] << 32) | ((unsigned __int128)t[2 * PS] << 64);
-	__int128 v = (__int128)(u << 32) >> 32;             // sign-extend the 96-bit value
-	v += delta;
-	const unsigned __int128 w = (unsigned __int128)v;
-	t[0] = (u32)w; t[PS] = (u32)(w >> 32); t[2 * PS] = (u32)(w >> 64);
+	constexpr int SB = ColStages<LOG_H>::SB, ST = ColStages<LOG_H>::ST, PS = CW << LOG_H;
+	const int tid = (int)threadIdx.x, NT = (int)blockDim.x, u = tid & 31;
+	if constexpr (ST > 0)
+	{
+		for (int task = tid; task < (KP << (LOG_H - ST + 5)); task += NT)
+		{
+			const int o = (task >> 5) & ((1 << (LOG_H - ST)) - 1), k = task >> (LOG_H - ST + 5);
+			const u32 p = c.p[k];
+			col_step<ST, false>(tile + k * PS + u, CW, tile + k * PS + u, CW, LOG_H, SB, (u32)o, twk + (k << LOG_H), p, 2 * p);
+		}
+		__syncthreads();
+	}
+	for (int task = tid; task < (KP << (LOG_H - SB + 5)); task += NT)
+	{
+		const int o = (task >> 5) & ((1 << (LOG_H - SB)) - 1), k = task >> (LOG_H - SB + 5);
+		const u32 p = c.p[k];
+		if (own) col_step<SB, false>(tile + k * PS + u, CW, x + (size_t)k * n + gc, R, LOG_H, 0, (u32)o, twk + (k << LOG_H), p, 2 * p);
+	}
 }
 
-// Residues of the exact values of 4 coefficients (limb words l[0..2], each 4
-// coefficients) in the KP planes of the tile at tp (plane stride PS words).
-template <int KP>
-__device__ __forceinline__ void encode4(const TConst & c, const uint4 (&l)[AB_NW], u32 * tp, int PS)
+// Adds d to an exact value (three limbs).
+__device__ __forceinline__ void exact_add(u32 (&x)[AB_NW], __int128 d)
 {
-	const u32 d0[4] = { l[0].x, l[0].y, l[0].z, l[0].w };
-	const u32 d1[4] = { l[1].x, l[1].y, l[1].z, l[1].w };
-	const u32 d2[4] = { l[2].x ^ 0x80000000u, l[2].y ^ 0x80000000u, l[2].z ^ 0x80000000u, l[2].w ^ 0x80000000u };
-#pragma unroll
-	for (int k = 0; k < KP; ++k)
-	{
-		uint4 r;
-		r.x = encode_res(c, k, d0[0], d1[0], d2[0]);
-		r.y = encode_res(c, k, d0[1], d1[1], d2[1]);
-		r.z = encode_res(c, k, d0[2], d1[2], d2[2]);
-		r.w = encode_res(c, k, d0[3], d1[3], d2[3]);
-		*reinterpret_cast<uint4 *>(tp + k * PS) = r;
-	}
+	const unsigned __int128 v = ((unsigned __int128)x[0] | ((unsigned __int128)x[1] << 32) | ((unsigned __int128)x[2] << 64)) +
+	                            (unsigned __int128)d;
+	x[0] = (u32)v; x[1] = (u32)(v >> 32); x[2] = (u32)(v >> 64);
 }
 
 // Second carry phase for one group of 4 coefficients (kernel.cl:1582-1613):
-// f = carry-in, d = the group's unsigned digits; returns each coefficient's
-// exact value (balanced top digit, the last coefficient absorbing the rest)
-// as three limbs and the top sub-digit of the last coefficient.
+// f = carry-in, d = the group's unsigned W-bit digits.  The first three become
+// balanced, v in [-2^(W-1), 2^(W-1)) with the carry (f + d + 2^(W-1)) >> W;
+// the last one absorbs the rest.  x: exact values (three limbs each).  After
+// the first step the carry is below 2^55, so three limbs hold every sum.
 template <int L, int PCK>
-__device__ __forceinline__ i32 carry_phase2(int lb, Big<L> f, const u32 (&d)[4][PCK], u32 (&x)[AB_NW][4])
+__device__ __forceinline__ void carry_phase2(const Width & w, const u32 (&half)[AB_NW], const Big<L> & f, const u32 (&d)[4][DigitLimbs<PCK>::N],
+	u32 (&x)[4][AB_NW])
 {
-	const i32 base = (i32)(1u << lb);
+	constexpr int ND = DigitLimbs<PCK>::N;
+	u32 hd[ND];
 #pragma unroll
-	for (int j = 0; j < 3; ++j)
+	for (int i = 0; i < ND; ++i) hd[i] = half[i];
+	Big<AB_NW> g;
+	auto balanced = [&](const u32 (&e)[ND], u32 (&v)[AB_NW]) {
+		Big<AB_NW> a, h;
+#pragma unroll
+		for (int i = 0; i < AB_NW; ++i) { a.l[i] = (i < ND) ? e[i % ND] : 0u; h.l[i] = half[i]; }
+		a = big_sub<AB_NW>(a, h);
+#pragma unroll
+		for (int i = 0; i < AB_NW; ++i) v[i] = a.l[i];
+	};
 	{
-		f = add_digits<L, PCK>(f, lb, d[j]);
-		u32 e[PCK];
-		extract_shift<L, PCK>(f, lb, e);
-		i32 top = (i32)e[PCK - 1];
-		if (top >= base / 2) { top -= base; f = big_add_u32<L>(f, 1u); }
-		digits_exact<PCK>(lb, top, e, x[0][j], x[1][j], x[2][j]);
+		Big<L> t = add_digit<L, ND>(add_digit<L, ND>(f, d[0]), hd);
+		const u32 s = (u32)((i32)t.l[L - 1] >> 31);
+		u32 e[ND];
+		split_digit<L, ND>(t, w, e);
+		balanced(e, x[0]);
+#pragma unroll
+		for (int i = 0; i < AB_NW; ++i) g.l[i] = (i < L) ? t.l[i % L] : s;
 	}
-	f = add_digits<L, PCK>(f, lb, d[3]);
-	const u32 bm = (u32)base - 1;
-	u32 e[PCK];
-	i32 top;
-	if (PCK == 1)
+#pragma unroll
+	for (int j = 1; j < 3; ++j)
 	{
-		top = (i32)(i64)big_low64<L>(f);
+		g = add_digit<AB_NW, ND>(add_digit<AB_NW, ND>(g, d[j]), hd);
+		u32 e[ND];
+		split_digit<AB_NW, ND>(g, w, e);
+		balanced(e, x[j]);
 	}
-	else if (PCK == 2)
-	{
-		const i64 r01 = (i64)big_low64<L>(f);
-		e[0] = (u32)r01 & bm;
-		top = (i32)(r01 >> lb);
-	}
-	else
-	{
-		const u64 r01 = big_low64<L>(f) & (((u64)1 << (2 * lb)) - 1);
-		e[0] = (u32)r01 & bm;
-		e[1 % PCK] = (u32)(r01 >> lb);
-		const Big<L> f23 = big_sar<L>(f, 2 * lb);
-		const i64 r23 = (i64)big_low64<L>(f23);
-		e[2 % PCK] = (u32)r23 & bm;
-		top = (i32)(r23 >> lb);
-	}
-	digits_exact<PCK>(lb, top, e, x[0][3], x[1][3], x[2][3]);
-	return top;
+	g = add_digit<AB_NW, ND>(g, d[3]);
+#pragma unroll
+	for (int i = 0; i < AB_NW; ++i) x[3][i] = g.l[i];
 }
 
-// The column pass of column group b of nb (32 columns each) of candidate
-// cand, by all threads of the CTA; sm: colpass_smem bytes of shared memory.
+// The column pass of column group b of nb of candidate cand, by all threads
+// of the CTA (a multiple of 32); sm: colpass_smem bytes of shared memory.
+//
+// Bound by the integer multiplier (butterflies 4 units each, CRT about 75 and
+// encoding 54 units per coefficient of 6 primes) when the grid fills the GPU,
+// by the chain of phases when it does not.  So a coefficient is handled as one
+// digit of W = pck lbase bits instead of pck digits (no 128-bit shifts by a
+// runtime amount), the residues are the CRT coordinates themselves (crt), the
+// exact values go from the carry to their residues in registers, and the first
+// and last butterfly stages read and write global memory directly.
 template <int LOG_H, int K, int PCK>
 __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 cand, int b, int nb, u32 * sm, int & decision)
 {
 	constexpr int KP = K + 1, L = K;             // transform primes, limbs of the carry
 	constexpr int H = 1 << LOG_H;
-	constexpr int PS = H * TW;                   // tile plane stride
-	u32 * const tile = sm;                       // [KP][H][TW]
-	u32 * const cw = tile + KP * PS;             // [H][TW/4][L] carry-out words
-	uint2 * const twc = reinterpret_cast<uint2 *>(cw + H * (TW / 4) * L);   // [3][KP][H] column twiddles
+	constexpr int PS = H * CW;                   // tile plane stride
+	constexpr int ND = DigitLimbs<PCK>::N;
+	u32 * const tile = sm;                       // [KP][H][CW]
+	u32 * const cw = tile + KP * PS;             // [H][8][L] carry-out words
+	u32 * const edge = cw + H * 8 * L;           // [2][4][AB_NW]: the groups that the mod R / mod Q step adjusts
+	uint2 * const twc = reinterpret_cast<uint2 *>(edge + 24);   // [3][KP][H] column twiddles
 
 	const u32 amul = (J.mult != nullptr) ? J.mult[cand] : J.a;
 	if (amul == 0u) return;                       // inactive batch slot
@@ -585,21 +608,18 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 		if (J.out_fwd[1]) J.out_fwd[1] += ot;
 		if (J.out_snap) J.out_snap = (J.snap_flag[cand] != 0u) ? J.out_snap + on : nullptr;
 	}
-	const int lb = (J.cand != nullptr) ? J.cand[cand].lbase : c.lbase;
+	const int wbits = PCK * ((J.cand != nullptr) ? J.cand[cand].lbase : c.lbase);
 	const u32 R = c.R, n = c.n;
-	const u32 c0 = (u32)b * CC;
 	const bool single = (nb == 1);
-	// predecessor columns: the 4 left of the CTA (the last 4 of the previous row
-	// for CTA 0); CTA 0 also takes the 4 before those when the mod R / mod Q
-	// decision needs the final top coefficient
-	const int E = (!J.transformed || single) ? 0 : ((b == 0 && J.lower != LOWER_NONE) ? 8 : 4);
-	const int WU = CC + E, ng = WU / 4;
+	const int E = single ? 0 : (b == 0) ? 8 : 4;
+	const u32 c0 = (b == 0) ? 0u : 28u * (u32)b - 4u;                  // first own column
+	const int WU = min(CW, E + (int)(R - c0)), ng = WU / 4;            // live columns and groups of a row
 	const int tid = (int)threadIdx.x, NT = (int)blockDim.x;
+	// global column of tile column u (CTA 0's predecessors end the previous row)
+	auto gcol = [&](int u) -> u32 { return c0 + (u32)(u - E) + ((b == 0 && u < E) ? R : 0u); };
+	const int lane = tid & 31;
 
-	auto gcol = [&](int u) -> u32 { return (u < E) ? ((b == 0) ? R - (u32)E + (u32)u : c0 - (u32)E + (u32)u) : c0 + (u32)(u - E); };
-
-	// ---- the column twiddles (constant tables), then the tile (NTT form: KP
-	// planes; normal form: the three limb planes), which the previous pass wrote
+	// ---- the column twiddles (constant tables)
 	for (int idx = tid; idx < KP * H; idx += NT)
 	{
 		const int k = idx / H, i = idx % H;
@@ -608,65 +628,65 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 		if (J.out_fwd[0] != nullptr) twc[KP * H + idx] = J.w_out[0][k * COLTW + i];
 		if (J.out_fwd[1] != nullptr) twc[2 * KP * H + idx] = J.w_out[1][k * COLTW + i];
 	}
-	griddep_wait();
-	griddep_launch();
-	const int np_in = J.transformed ? KP : AB_NW;
-	for (int idx = tid; idx < (np_in << (LOG_H + 3)); idx += NT)
-	{
-		const int u4 = idx & 7, row = (idx >> 3) & (H - 1), k = idx >> (LOG_H + 3);
-		const uint4 val = __ldg(reinterpret_cast<const uint4 *>(J.in + (size_t)k * n + (size_t)row * R + c0 + 4 * u4));
-		*reinterpret_cast<uint4 *>(tile + k * PS + row * TW + E + 4 * u4) = val;
-	}
-	if (E > 0)
-	{
-		const int le4 = (E == 8) ? 1 : 0;                          // log2 of the predecessor groups
-		for (int idx = tid; idx < (np_in << (LOG_H + le4)); idx += NT)
-		{
-			const int u4 = idx & (E / 4 - 1), row = (idx >> le4) & (H - 1), k = idx >> (LOG_H + le4);
-			const uint4 val = __ldg(reinterpret_cast<const uint4 *>(J.in + (size_t)k * n + (size_t)row * R + gcol(4 * u4)));
-			*reinterpret_cast<uint4 *>(tile + k * PS + row * TW + 4 * u4) = val;
-		}
-	}
 	if (tid == 0) decision = 0;
 	__syncthreads();
+	griddep_wait();
+	griddep_launch();
+
+	// a group's exact values: normal form out, residues into the tile
+	const bool fwd = (J.out_fwd[0] != nullptr) || (J.out_fwd[1] != nullptr);
+	auto encode = [&](int row, int u4, const u32 (&x)[4][AB_NW]) {
+		Pieces a[4];
+#pragma unroll
+		for (int j = 0; j < 4; ++j) a[j] = split30(x[j][0], x[j][1], x[j][2]);
+#pragma unroll
+		for (int k = 0; k < KP; ++k)
+			*reinterpret_cast<uint4 *>(tile + k * PS + row * CW + 4 * u4) =
+				make_uint4(encode_res(c, k, a[0]), encode_res(c, k, a[1]), encode_res(c, k, a[2]), encode_res(c, k, a[3]));
+	};
+	auto finalize = [&](int row, int u4, const u32 (&x)[4][AB_NW]) {
+		const size_t o = (size_t)row * R + gcol(4 * u4);
+#pragma unroll
+		for (int l = 0; l < AB_NW; ++l)
+		{
+			const uint4 val = make_uint4(x[0][l], x[1][l], x[2][l], x[3][l]);
+			if (J.out_norm) *reinterpret_cast<uint4 *>(J.out_norm + (size_t)l * n + o) = val;
+			if (J.out_snap) *reinterpret_cast<uint4 *>(J.out_snap + (size_t)l * n + o) = val;
+		}
+		if (fwd) encode(row, u4, x);
+	};
+	auto load_norm = [&](const u32 * src, int row, int u4, u32 (&x)[4][AB_NW]) {
+#pragma unroll
+		for (int l = 0; l < AB_NW; ++l)
+		{
+			const uint4 t = *reinterpret_cast<const uint4 *>(src + (size_t)l * n + (size_t)row * R + gcol(4 * u4));
+			x[0][l] = t.x; x[1][l] = t.y; x[2][l] = t.z; x[3][l] = t.w;
+		}
+	};
 
 	if (J.transformed)
 	{
-		// ---- inverse column levels (all WU columns, KP primes)
-		col_transform<LOG_H, KP, true>(tile, E, true, twc, c);
+		// ---- inverse column levels
+		col_inverse<LOG_H, KP>(J.in, n, R, gcol(lane), lane < WU, tile, twc, c);
 
+		const Width w = make_width(wbits);
 		// ---- carry phase 1: per group, exact values (CRT), x a, - sub,
 		// unsigned digits + carry-out
-		const int npg = (E == 8) ? H + 1 : (E == 4) ? H : 0;    // predecessor groups carried (for E = 8 only row H-1's first)
-		for (int idx = tid; idx < H * (CC / 4) + npg; idx += NT)
+		for (int idx = tid; idx < H * 8; idx += NT)
 		{
-			int row, u4;
-			if (idx < H * (CC / 4)) { row = idx >> 3; u4 = E / 4 + (idx & 7); }
-			else
-			{
-				const int q = idx - H * (CC / 4);
-				if (E == 4) { row = q; u4 = 0; }
-				else { row = (q < H) ? q : H - 1; u4 = (q < H) ? 1 : 0; }
-			}
+			const int row = idx >> 3, u4 = idx & 7;
+			if (u4 >= ng) continue;
 			u32 xv[KP][4];
 #pragma unroll
 			for (int k = 0; k < KP; ++k)
 			{
-				const uint4 t = *reinterpret_cast<const uint4 *>(tile + k * PS + row * TW + 4 * u4);
+				const uint4 t = *reinterpret_cast<const uint4 *>(tile + k * PS + row * CW + 4 * u4);
 				xv[k][0] = t.x; xv[k][1] = t.y; xv[k][2] = t.z; xv[k][3] = t.w;
 			}
-			u32 sv[AB_NW][4];
-			if (J.sub != nullptr)
-			{
-#pragma unroll
-				for (int l = 0; l < AB_NW; ++l)
-				{
-					const uint4 t = __ldg(reinterpret_cast<const uint4 *>(J.sub + (size_t)l * n + (size_t)row * R + gcol(4 * u4)));
-					sv[l][0] = t.x; sv[l][1] = t.y; sv[l][2] = t.z; sv[l][3] = t.w;
-				}
-			}
+			u32 sv[4][AB_NW];
+			if (J.sub != nullptr) load_norm(J.sub, row, u4, sv);
 			Big<L> f = big_zero<L>();
-			u32 dg[4][PCK];
+			u32 dg[4][ND];
 #pragma unroll
 			for (int j = 0; j < 4; ++j)
 			{
@@ -675,133 +695,139 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 				for (int k = 0; k < KP; ++k) rr[k] = xv[k][j];
 				Big<L> V = crt<L>(c, rr);
 				if (amul != 1u) V = big_mul_u32<L>(V, amul);
-				if (J.sub != nullptr) V = big_sub<L>(V, big_from_exact<L>(sv[0][j], sv[1][j], sv[2][j]));
+				if (J.sub != nullptr) V = big_sub<L>(V, big_from_exact<L>(sv[j][0], sv[j][1], sv[j][2]));
 				f = big_add<L>(f, V);
-				extract_shift<L, PCK>(f, lb, dg[j]);
+				split_digit<L, ND>(f, w, dg[j]);
 			}
 #pragma unroll
-			for (int l = 0; l < PCK; ++l)
-				*reinterpret_cast<uint4 *>(tile + l * PS + row * TW + 4 * u4) = make_uint4(dg[0][l], dg[1][l], dg[2][l], dg[3][l]);
+			for (int l = 0; l < ND; ++l)
+				*reinterpret_cast<uint4 *>(tile + l * PS + row * CW + 4 * u4) = make_uint4(dg[0][l], dg[1][l], dg[2][l], dg[3][l]);
 #pragma unroll
-			for (int l = 0; l < L; ++l) cw[(row * (TW / 4) + u4) * L + l] = f.l[l];
+			for (int l = 0; l < L; ++l) cw[idx * L + l] = f.l[l];
 		}
 		__syncthreads();
 
 		// ---- carry phase 2: add the previous group's carry-out, balanced
-		// digits, exact values
-		const int own_groups = CC / 4;
-		for (int idx = tid; idx < H * own_groups + 1; idx += NT)
+		// values; then the outputs of the group.  Each thread reads and writes
+		// only its own group of the tile.
+		const int hb = wbits - 1;
+		const u32 half[AB_NW] = { (hb >> 5) == 0 ? 1u << (hb & 31) : 0u, (hb >> 5) == 1 ? 1u << (hb & 31) : 0u, (hb >> 5) == 2 ? 1u << (hb & 31) : 0u };
+		const bool adjust = (J.lower != LOWER_NONE);
+		for (int idx = tid; idx < H * 8; idx += NT)
 		{
-			int row, u4;
-			bool store = true;
-			if (idx == H * own_groups)
-			{
-				// CTA 0 re-derives the last coefficient of the register from its
-				// predecessor columns, for the mod R / mod Q decision
-				if (E != 8) continue;
-				row = H - 1; u4 = 1; store = false;
-			}
-			else
-			{
-				row = idx / own_groups; u4 = E / 4 + idx % own_groups;
-			}
+			const int row = idx >> 3, u4 = idx & 7;
+			if (u4 >= ng) continue;
+			// CTA 0 re-derives the last coefficient of the register from its
+			// predecessor columns, for the mod R / mod Q decision
+			const bool top0 = adjust && E == 8 && row == H - 1 && u4 == 1;
+			if (4 * u4 < E && !top0) continue;
 			int prow = row, pu4 = u4 - 1;
 			bool neg = false;
-			if (store && b == 0 && u4 == E / 4)
+			if (b == 0 && 4 * u4 == E)
 			{
 				// first group of a row: its predecessor ends the previous row
-				pu4 = (E == 0) ? (ng - 1) : (E / 4 - 1);
+				if (E == 0) pu4 = ng - 1;
 				if (row > 0) prow = row - 1;
 				else { prow = H - 1; neg = (J.nega != 0); }
 			}
 			Big<L> f;
 #pragma unroll
-			for (int l = 0; l < L; ++l) f.l[l] = cw[(prow * (TW / 4) + pu4) * L + l];
+			for (int l = 0; l < L; ++l) f.l[l] = cw[(prow * 8 + pu4) * L + l];
 			if (neg) f = big_neg<L>(f);
-			u32 dg[4][PCK];
+			u32 dg[4][ND];
 #pragma unroll
-			for (int l = 0; l < PCK; ++l)
+			for (int l = 0; l < ND; ++l)
 			{
-				const uint4 t = *reinterpret_cast<const uint4 *>(tile + l * PS + row * TW + 4 * u4);
+				const uint4 t = *reinterpret_cast<const uint4 *>(tile + l * PS + row * CW + 4 * u4);
 				dg[0][l] = t.x; dg[1][l] = t.y; dg[2][l] = t.z; dg[3][l] = t.w;
 			}
-			u32 ex[AB_NW][4];
-			const i32 top = carry_phase2<L, PCK>(lb, f, dg, ex);
-			if (store)
+			u32 ex[4][AB_NW];
+			carry_phase2<L, PCK>(w, half, f, dg, ex);
+			const bool first = (b == 0) && row == 0 && 4 * u4 == E;
+			const bool last = (b == nb - 1) && row == H - 1 && u4 == ng - 1;
+			if (adjust && (first || last || top0))
 			{
+				if (last || top0)
+				{
+					// the last coefficient is 2^W or more
+					Big<AB_NW> t;
 #pragma unroll
-				for (int l = 0; l < AB_NW; ++l)
-					*reinterpret_cast<uint4 *>(tile + l * PS + row * TW + 4 * u4) = make_uint4(ex[l][0], ex[l][1], ex[l][2], ex[l][3]);
+					for (int l = 0; l < AB_NW; ++l) t.l[l] = ex[3][l];
+					u32 e[ND];
+					split_digit<AB_NW, ND>(t, w, e);
+					if ((i32)t.l[2] >= 0 && (t.l[0] | t.l[1] | t.l[2]) != 0u) decision = 1;
+				}
+				if (!top0)
+				{
+#pragma unroll
+					for (int j = 0; j < 4; ++j)
+#pragma unroll
+						for (int l = 0; l < AB_NW; ++l) edge[(last ? 12 : 0) + 3 * j + l] = ex[j][l];
+				}
 			}
-			const bool is_last = (row == H - 1) && (u4 == ng - 1) && (b == nb - 1);
-			if ((is_last || !store) && top >= (i32)(1u << lb)) decision = 1;
+			else finalize(row, u4, ex);
 		}
-		__syncthreads();
 
 		// ---- mod R (+2) / mod Q on the top and bottom coefficients (kernel.cl:1653-1683)
-		if (J.lower != LOWER_NONE && tid == 0)
+		if (adjust && (b == 0 || b == nb - 1))
 		{
-			if (decision && b == nb - 1) exact_add(tile + (H - 1) * TW + WU - 1, PS, -((__int128)1 << (c.pck * lb)));
-			if (b == 0)
+			__syncthreads();
+			if (tid < 2 && ((tid == 0) ? b == 0 : b == nb - 1))
 			{
-				int d = 0;
-				if (decision) d += (J.lower == LOWER_Q) ? -1 : 1;
-				if (J.lower == LOWER_R_ADD2) d += 2;
-				if (d != 0) exact_add(tile + E, PS, (__int128)d);
+				u32 ex[4][AB_NW];
+#pragma unroll
+				for (int j = 0; j < 4; ++j)
+#pragma unroll
+					for (int l = 0; l < AB_NW; ++l) ex[j][l] = edge[12 * tid + 3 * j + l];
+				if (tid == 0)
+				{
+					int d = 0;
+					if (decision) d += (J.lower == LOWER_Q) ? -1 : 1;
+					if (J.lower == LOWER_R_ADD2) d += 2;
+					exact_add(ex[0], (__int128)d);
+					finalize(0, E / 4, ex);
+				}
+				else
+				{
+					if (decision) exact_add(ex[3], -((__int128)1 << wbits));
+					finalize(H - 1, ng - 1, ex);
+				}
 			}
 		}
-		__syncthreads();
 	}
-
 	griddep_launch_late();
-	// ---- outputs: normal form, then the first LA forward levels of the next
-	// product in one or two domains (the residues are encoded from the exact
-	// values in the tile, or for the second domain from the normal form in
-	// global memory)
-	if (J.out_norm != nullptr || J.out_snap != nullptr)
-	{
-		for (int idx = tid; idx < AB_NW * H * (CC / 4); idx += NT)
-		{
-			const int u4 = idx % (CC / 4), row = (idx / (CC / 4)) % H, l = idx / ((CC / 4) * H);
-			const uint4 val = *reinterpret_cast<const uint4 *>(tile + l * PS + row * TW + E + 4 * u4);
-			const size_t o = (size_t)l * n + (size_t)row * R + c0 + 4 * u4;
-			if (J.out_norm) *reinterpret_cast<uint4 *>(J.out_norm + o) = val;
-			if (J.out_snap) *reinterpret_cast<uint4 *>(J.out_snap + o) = val;
-		}
-	}
-	bool first = true;
+
+	// ---- the first LA forward levels of the result in one or two domains: the
+	// residues of a transformed source are in the tile; those of a normal-form
+	// source, and of the second domain, come from the normal form in global memory
+	bool in_tile = (J.transformed != 0);
+	const bool own = (lane >= E && lane < WU);
 #pragma unroll 1
 	for (int dom = 0; dom < 2; ++dom)
 	{
 		u32 * const out = (dom == 0) ? J.out_fwd[0] : J.out_fwd[1];
 		if (out == nullptr) continue;
-		__syncthreads();
-		const u32 * src = first ? nullptr : (J.transformed ? J.out_norm : J.in);
-		for (int idx = tid; idx < H * (CC / 4); idx += NT)
+		if (!in_tile)
 		{
-			const int u4 = idx % (CC / 4), row = idx / (CC / 4);
-			u32 * const tp = tile + row * TW + E + 4 * u4;
-			uint4 l[AB_NW];
-#pragma unroll
-			for (int i = 0; i < AB_NW; ++i)
-				l[i] = (src == nullptr) ? *reinterpret_cast<const uint4 *>(tp + i * PS)
-				                        : *reinterpret_cast<const uint4 *>(src + (size_t)i * n + (size_t)row * R + c0 + 4 * u4);
-			encode4<KP>(c, l, tp, PS);
+			__syncthreads();
+			const u32 * src = J.transformed ? J.out_norm : J.in;
+			for (int idx = tid; idx < H * 8; idx += NT)
+			{
+				const int row = idx >> 3, u4 = idx & 7;
+				if (4 * u4 < E || u4 >= ng) continue;
+				u32 x[4][AB_NW];
+				load_norm(src, row, u4, x);
+				encode(row, u4, x);
+			}
 		}
 		__syncthreads();
-		col_transform<LOG_H, KP, false>(tile, E, false, twc + (1 + dom) * KP * H, c);
-		for (int idx = tid; idx < KP * H * (CC / 4); idx += NT)
-		{
-			const int u4 = idx % (CC / 4), row = (idx / (CC / 4)) % H, k = idx / ((CC / 4) * H);
-			*reinterpret_cast<uint4 *>(out + (size_t)k * n + (size_t)row * R + c0 + 4 * u4) =
-				*reinterpret_cast<const uint4 *>(tile + k * PS + row * TW + E + 4 * u4);
-		}
-		first = false;
+		col_forward<LOG_H, KP>(tile, out, n, R, gcol(lane), own, twc + (1 + dom) * KP * H, c);
+		in_tile = false;
 	}
 }
 
 template <int LOG_H, int K, int PCK>
-__global__ void __launch_bounds__(COL_THREADS, 2) k_colpass(const ColJobs jobs, const TConst c)
+__global__ void __launch_bounds__(ColCfg<LOG_H>::NT, ColCfg<LOG_H>::MINB) k_colpass(const ColJobs jobs, const TConst c)
 {
 	extern __shared__ __align__(16) u32 sm[];
 	__shared__ int decision;
@@ -1033,14 +1059,14 @@ bool make_geometry(int ln, int lb_override, Geometry & g)
 	const int LA = (L - LB < 6) ? L - LB : 6, G = L - LB - LA;
 	if (G > 3) return false;
 	g.ln = ln; g.LB = LB; g.LA = LA; g.G = G;
-	g.H = 1u << LA; g.R = 1u << (LB + 1); g.HR = g.H << G; g.RC = g.R << G; g.C = CC;
+	g.H = 1u << LA; g.R = 1u << (LB + 1); g.HR = g.H << G; g.RC = g.R << G; g.NC = col_ctas(g.RC);
 	return true;
 }
 
 size_t colpass_smem(const Geometry & g, int KP)
 {
 	const size_t L = (size_t)KP - 1;
-	return sizeof(u32) * ((size_t)KP * g.H * TW + (size_t)g.H * (TW / 4) * L) + sizeof(uint2) * 3 * (size_t)KP * g.H;
+	return sizeof(u32) * ((size_t)KP * g.H * CW + (size_t)g.H * 8 * L + 24) + sizeof(uint2) * 3 * (size_t)KP * g.H;
 }
 
 // The dynamic shared-memory limit of a kernel is a per-device setting: set it
@@ -1134,8 +1160,8 @@ static cudaError_t colpass_t(const Geometry & g, const TConst & c, const ColJobs
 	const cudaError_t e = allow_dynamic_smem(k_colpass<LOG_H, K, PCK>, smem, attr_done);
 	if (e != cudaSuccess) return e;
 	if (ncand == 0) return cudaSuccess;      // set-up only (before a stream capture)
-	const dim3 grid(g.RC / CC, (unsigned)njobs, (unsigned)ncand);
-	return launch_pdl(k_colpass<LOG_H, K, PCK>, grid, dim3(COL_THREADS), smem, s, jobs, c);
+	const dim3 grid(g.NC, (unsigned)njobs, (unsigned)ncand);
+	return launch_pdl(k_colpass<LOG_H, K, PCK>, grid, dim3(ColCfg<LOG_H>::NT), smem, s, jobs, c);
 }
 
 template <int K, int PCK>

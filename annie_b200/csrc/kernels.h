@@ -78,7 +78,7 @@ struct Geometry
 {
 	int ln, LA, LB, G;
 	u32 H, R, HR, RC;
-	int C;               // columns per column-pass CTA
+	u32 NC;              // CTAs of a column pass (per job and candidate)
 };
 
 // Chooses the split for a transform of length 2^ln (6 <= ln <= 22);
@@ -119,7 +119,7 @@ struct FusedColPass
 {
 	int nclass;
 	u32 begin[AB_FUSE_MAXC + 1];
-	u32 nbx[AB_FUSE_MAXC];        // RC / 32 column groups
+	u32 nbx[AB_FUSE_MAXC];        // column-pass CTAs
 	u32 njobs[AB_FUSE_MAXC];
 	int sel[AB_FUSE_MAXC];        // LA * 8 + K
 	ColJobs jobs[AB_FUSE_MAXC];
