@@ -107,23 +107,55 @@ __device__ __forceinline__ Big<L> big_zero()
 	return r;
 }
 
+// a + b + carry-in chain; the carry flag lives only inside one asm statement,
+// so each chain is one statement.
 template <int L>
 __device__ __forceinline__ Big<L> big_add(const Big<L> & a, const Big<L> & b)
 {
+	static_assert(L >= 2 && L <= 5, "2 to 5 limbs");
 	Big<L> r;
-	u64 c = 0;
-#pragma unroll
-	for (int i = 0; i < L; ++i) { c += (u64)a.l[i] + b.l[i]; r.l[i] = (u32)c; c >>= 32; }
+	if constexpr (L == 2)
+		asm("add.cc.u32 %0, %2, %4;\n\taddc.u32 %1, %3, %5;"
+		    : "=&r"(r.l[0]), "=r"(r.l[1]) : "r"(a.l[0]), "r"(a.l[1]), "r"(b.l[0]), "r"(b.l[1]));
+	else if constexpr (L == 3)
+		asm("add.cc.u32 %0, %3, %6;\n\taddc.cc.u32 %1, %4, %7;\n\taddc.u32 %2, %5, %8;"
+		    : "=&r"(r.l[0]), "=&r"(r.l[1]), "=r"(r.l[2])
+		    : "r"(a.l[0]), "r"(a.l[1]), "r"(a.l[2]), "r"(b.l[0]), "r"(b.l[1]), "r"(b.l[2]));
+	else if constexpr (L == 4)
+		asm("add.cc.u32 %0, %4, %8;\n\taddc.cc.u32 %1, %5, %9;\n\taddc.cc.u32 %2, %6, %10;\n\taddc.u32 %3, %7, %11;"
+		    : "=&r"(r.l[0]), "=&r"(r.l[1]), "=&r"(r.l[2]), "=r"(r.l[3])
+		    : "r"(a.l[0]), "r"(a.l[1]), "r"(a.l[2]), "r"(a.l[3]), "r"(b.l[0]), "r"(b.l[1]), "r"(b.l[2]), "r"(b.l[3]));
+	else
+		asm("add.cc.u32 %0, %5, %10;\n\taddc.cc.u32 %1, %6, %11;\n\taddc.cc.u32 %2, %7, %12;\n\taddc.cc.u32 %3, %8, %13;\n\t"
+		    "addc.u32 %4, %9, %14;"
+		    : "=&r"(r.l[0]), "=&r"(r.l[1]), "=&r"(r.l[2]), "=&r"(r.l[3]), "=r"(r.l[L - 1])
+		    : "r"(a.l[0]), "r"(a.l[1]), "r"(a.l[2]), "r"(a.l[3]), "r"(a.l[L - 1]),
+		      "r"(b.l[0]), "r"(b.l[1]), "r"(b.l[2]), "r"(b.l[3]), "r"(b.l[L - 1]));
 	return r;
 }
 
 template <int L>
 __device__ __forceinline__ Big<L> big_sub(const Big<L> & a, const Big<L> & b)
 {
+	static_assert(L >= 2 && L <= 5, "2 to 5 limbs");
 	Big<L> r;
-	u64 c = 1;
-#pragma unroll
-	for (int i = 0; i < L; ++i) { c += (u64)a.l[i] + (u64)(~b.l[i]); r.l[i] = (u32)c; c >>= 32; }
+	if constexpr (L == 2)
+		asm("sub.cc.u32 %0, %2, %4;\n\tsubc.u32 %1, %3, %5;"
+		    : "=&r"(r.l[0]), "=r"(r.l[1]) : "r"(a.l[0]), "r"(a.l[1]), "r"(b.l[0]), "r"(b.l[1]));
+	else if constexpr (L == 3)
+		asm("sub.cc.u32 %0, %3, %6;\n\tsubc.cc.u32 %1, %4, %7;\n\tsubc.u32 %2, %5, %8;"
+		    : "=&r"(r.l[0]), "=&r"(r.l[1]), "=r"(r.l[2])
+		    : "r"(a.l[0]), "r"(a.l[1]), "r"(a.l[2]), "r"(b.l[0]), "r"(b.l[1]), "r"(b.l[2]));
+	else if constexpr (L == 4)
+		asm("sub.cc.u32 %0, %4, %8;\n\tsubc.cc.u32 %1, %5, %9;\n\tsubc.cc.u32 %2, %6, %10;\n\tsubc.u32 %3, %7, %11;"
+		    : "=&r"(r.l[0]), "=&r"(r.l[1]), "=&r"(r.l[2]), "=r"(r.l[3])
+		    : "r"(a.l[0]), "r"(a.l[1]), "r"(a.l[2]), "r"(a.l[3]), "r"(b.l[0]), "r"(b.l[1]), "r"(b.l[2]), "r"(b.l[3]));
+	else
+		asm("sub.cc.u32 %0, %5, %10;\n\tsubc.cc.u32 %1, %6, %11;\n\tsubc.cc.u32 %2, %7, %12;\n\tsubc.cc.u32 %3, %8, %13;\n\t"
+		    "subc.u32 %4, %9, %14;"
+		    : "=&r"(r.l[0]), "=&r"(r.l[1]), "=&r"(r.l[2]), "=&r"(r.l[3]), "=r"(r.l[L - 1])
+		    : "r"(a.l[0]), "r"(a.l[1]), "r"(a.l[2]), "r"(a.l[3]), "r"(a.l[L - 1]),
+		      "r"(b.l[0]), "r"(b.l[1]), "r"(b.l[2]), "r"(b.l[3]), "r"(b.l[L - 1]));
 	return r;
 }
 
@@ -253,29 +285,35 @@ __device__ __forceinline__ Width make_width(int w)
 template <int PCK>
 struct DigitLimbs { static constexpr int N = (PCK == 1) ? 1 : (PCK == 2) ? 2 : 3; };
 
-// d = the low W bits of f (unsigned), f >>= W (arithmetic).
-template <int L, int ND>
+// d = the low W bits of f (unsigned), f >>= W (arithmetic).  FULL: W reaches
+// into the last of the ND limbs (ws = ND - 1), as the parameter rule's digit
+// sizes do for every class; other (forced) sizes take the general form.
+template <bool FULL, int L, int ND>
 __device__ __forceinline__ void split_digit(Big<L> & f, const Width & w, u32 (&d)[ND])
 {
 	const u32 fill = (u32)((i32)f.l[L - 1] >> 31);
-	u32 t[L + 1];
+	u32 t[L + ND];
 #pragma unroll
-	for (int i = 0; i < L; ++i) t[i] = f.l[i];
-	t[L] = fill;
-#pragma unroll
-	for (int i = 0; i < ND; ++i) d[i] = (i < w.ws) ? t[i % L] : (i == w.ws) ? t[i % L] & w.mask : 0u;
-	if (ND > 1 && w.ws >= 1)
+	for (int i = 0; i < L + ND; ++i) t[i] = (i < L) ? f.l[i % L] : fill;
+	if constexpr (FULL)
 	{
 #pragma unroll
-		for (int i = 0; i < L; ++i) t[i] = t[i + 1];
+		for (int i = 0; i < ND; ++i) d[i] = (i < ND - 1) ? t[i] : t[i] & w.mask;
+#pragma unroll
+		for (int i = 0; i < L; ++i) f.l[i] = (i + ND - 1 < L) ? __funnelshift_r(t[i + ND - 1], t[i + ND], w.bs) : fill;
 	}
-	if (ND > 2 && w.ws >= 2)
+	else
 	{
 #pragma unroll
-		for (int i = 0; i < L; ++i) t[i] = t[i + 1];
-	}
+		for (int i = 0; i < ND; ++i) d[i] = (i < w.ws) ? t[i] : (i == w.ws) ? t[i] & w.mask : 0u;
+		for (int m = 0; m < w.ws; ++m)
+		{
 #pragma unroll
-	for (int i = 0; i < L; ++i) f.l[i] = __funnelshift_r(t[i], t[i + 1], w.bs);
+			for (int i = 0; i < L; ++i) t[i] = t[i + 1];
+		}
+#pragma unroll
+		for (int i = 0; i < L; ++i) f.l[i] = __funnelshift_r(t[i], t[i + 1], w.bs);
+	}
 }
 
 // f + d (d unsigned)

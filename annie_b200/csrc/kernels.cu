@@ -18,6 +18,7 @@
 // in shared memory) and the row pass owns the last LB levels (one row of one
 // prime per CTA, 16 coefficients per thread in registers).
 #include <atomic>
+#include <type_traits>
 #include <utility>
 
 #include "kernels.h"
@@ -536,7 +537,7 @@ __device__ __forceinline__ void exact_add(u32 (&x)[AB_NW], __int128 d)
 // balanced, v in [-2^(W-1), 2^(W-1)) with the carry (f + d + 2^(W-1)) >> W;
 // the last one absorbs the rest.  x: exact values (three limbs each).  After
 // the first step the carry is below 2^55, so three limbs hold every sum.
-template <int L, int PCK>
+template <bool FULL, int L, int PCK>
 __device__ __forceinline__ void carry_phase2(const Width & w, const u32 (&half)[AB_NW], const Big<L> & f, const u32 (&d)[4][DigitLimbs<PCK>::N],
 	u32 (&x)[4][AB_NW])
 {
@@ -557,7 +558,7 @@ __device__ __forceinline__ void carry_phase2(const Width & w, const u32 (&half)[
 		Big<L> t = add_digit<L, ND>(add_digit<L, ND>(f, d[0]), hd);
 		const u32 s = (u32)((i32)t.l[L - 1] >> 31);
 		u32 e[ND];
-		split_digit<L, ND>(t, w, e);
+		split_digit<FULL, L, ND>(t, w, e);
 		balanced(e, x[0]);
 #pragma unroll
 		for (int i = 0; i < AB_NW; ++i) g.l[i] = (i < L) ? t.l[i % L] : s;
@@ -567,7 +568,7 @@ __device__ __forceinline__ void carry_phase2(const Width & w, const u32 (&half)[
 	{
 		g = add_digit<AB_NW, ND>(add_digit<AB_NW, ND>(g, d[j]), hd);
 		u32 e[ND];
-		split_digit<AB_NW, ND>(g, w, e);
+		split_digit<FULL, AB_NW, ND>(g, w, e);
 		balanced(e, x[j]);
 	}
 	g = add_digit<AB_NW, ND>(g, d[3]);
@@ -670,6 +671,7 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 		col_inverse<LOG_H, KP>(J.in, n, R, gcol(lane), lane < WU, tile, twc, c);
 
 		const Width w = make_width(wbits);
+		const bool full = (w.ws == ND - 1);
 		// ---- carry phase 1: per group, exact values (CRT), x a, - sub,
 		// unsigned digits + carry-out
 		for (int idx = tid; idx < H * 8; idx += NT)
@@ -687,18 +689,22 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 			if (J.sub != nullptr) load_norm(J.sub, row, u4, sv);
 			Big<L> f = big_zero<L>();
 			u32 dg[4][ND];
+			auto digits = [&](auto is_full) {
 #pragma unroll
-			for (int j = 0; j < 4; ++j)
-			{
-				u32 rr[KP];
+				for (int j = 0; j < 4; ++j)
+				{
+					u32 rr[KP];
 #pragma unroll
-				for (int k = 0; k < KP; ++k) rr[k] = xv[k][j];
-				Big<L> V = crt<L>(c, rr);
-				if (amul != 1u) V = big_mul_u32<L>(V, amul);
-				if (J.sub != nullptr) V = big_sub<L>(V, big_from_exact<L>(sv[j][0], sv[j][1], sv[j][2]));
-				f = big_add<L>(f, V);
-				split_digit<L, ND>(f, w, dg[j]);
-			}
+					for (int k = 0; k < KP; ++k) rr[k] = xv[k][j];
+					Big<L> V = crt<L>(c, rr);
+					if (amul != 1u) V = big_mul_u32<L>(V, amul);
+					if (J.sub != nullptr) V = big_sub<L>(V, big_from_exact<L>(sv[j][0], sv[j][1], sv[j][2]));
+					f = (j == 0) ? V : big_add<L>(f, V);
+					split_digit<decltype(is_full)::value, L, ND>(f, w, dg[j]);
+				}
+			};
+			if (full) digits(std::true_type{});
+			else digits(std::false_type{});
 #pragma unroll
 			for (int l = 0; l < ND; ++l)
 				*reinterpret_cast<uint4 *>(tile + l * PS + row * CW + 4 * u4) = make_uint4(dg[0][l], dg[1][l], dg[2][l], dg[3][l]);
@@ -742,7 +748,8 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 				dg[0][l] = t.x; dg[1][l] = t.y; dg[2][l] = t.z; dg[3][l] = t.w;
 			}
 			u32 ex[4][AB_NW];
-			carry_phase2<L, PCK>(w, half, f, dg, ex);
+			if (full) carry_phase2<true, L, PCK>(w, half, f, dg, ex);
+			else carry_phase2<false, L, PCK>(w, half, f, dg, ex);
 			const bool first = (b == 0) && row == 0 && 4 * u4 == E;
 			const bool last = (b == nb - 1) && row == H - 1 && u4 == ng - 1;
 			if (adjust && (first || last || top0))
@@ -754,7 +761,7 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 #pragma unroll
 					for (int l = 0; l < AB_NW; ++l) t.l[l] = ex[3][l];
 					u32 e[ND];
-					split_digit<AB_NW, ND>(t, w, e);
+					split_digit<false, AB_NW, ND>(t, w, e);
 					if ((i32)t.l[2] >= 0 && (t.l[0] | t.l[1] | t.l[2]) != 0u) decision = 1;
 				}
 				if (!top0)
