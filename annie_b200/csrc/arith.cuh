@@ -48,6 +48,29 @@ __device__ __forceinline__ u32 mont(u32 a, u32 b, u32 p, u32 pinv)
 	return hi - __umulhi(lo * pinv, p) + p;
 }
 
+// t 2^-32 mod p for a 64-bit t < f 2^32 p, in (0, (f + 1) p) (Montgomery,
+// pinv = p^-1 mod 2^32).
+__device__ __forceinline__ u32 redc(u64 t, u32 p, u32 pinv)
+{
+	return (u32)(t >> 32) - __umulhi((u32)t * pinv, p) + p;
+}
+
+// w 2^32 mod p from the Shoup pair (w, floor(w 2^32 / p)) of w
+__device__ __forceinline__ u32 mont_twiddle(uint2 w, u32 p) { return 0u - w.y * p; }
+
+// (x0 + x1 X)(y0 + y1 X) 2^-32 mod (X^2 - c), in place in (x0, x1); words in
+// [0, 2p) (in and out), cm = c 2^32 mod p.  Products are summed in 64 bits
+// before their one reduction (below 2^32 2p: x y < 4 p^2 and p < 2^30), three
+// reductions for the four products and the twiddle.  Without mul, y = x.
+__device__ __forceinline__ void poly_product(u32 & x0, u32 & x1, u32 y0, u32 y1, bool mul, u32 cm, u32 p, u32 p2, u32 pinv)
+{
+	const u32 t = redc((u64)x1 * y1, p, pinv);
+	const u32 r0 = redc((u64)x0 * y0 + (u64)t * cm, p, pinv);
+	const u32 r1 = mul ? redc((u64)x0 * y1 + (u64)x1 * y0, p, pinv) : redc((u64)(x0 + x0) * x1, p, pinv);
+	x0 = red2(r0, p2);
+	x1 = red2(r1, p2);
+}
+
 // Forward (decimation-in-time form) butterfly x0 +- w x1, inputs and outputs
 // in [0, 4p).
 __device__ __forceinline__ void fwd_bf(u32 & x0, u32 & x1, u32 w, u32 ws, u32 p, u32 p2)

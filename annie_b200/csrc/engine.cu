@@ -264,6 +264,7 @@ struct ab_transform
 	cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_fork = nullptr, ev_q = nullptr;
 	bool overlap = true;                 // run the Q chain on st2 (off for per-launch profiling)
 	bool split = false;                  // without overlap: still one launch per domain
+	bool resident = false;               // short length: runs of squarings in one launch (resident.cu)
 	ab_params prm{};
 	int KP = 0;                          // transform primes
 	size_t n = 0;
@@ -595,9 +596,21 @@ struct ab_transform
 		if (!prefwd) { ColJob j = cj_norm(b(REG0)); set_fwd(j, b(AQ0), b(AR0)); cols(j); q_pending = false; }
 	}
 
+	// `steps` squarings (multiplier a where bit s of bits is set, else 1) of the
+	// normal-form register x, or with y one product x y, in one launch
+	void run_resident(u32 * x, const u32 * y, int steps, uint64_t bits, u32 a)
+	{
+		ResJob j; std::memset(&j, 0, sizeof(j));
+		j.reg = x; j.y = y; j.nir = b(NIR); j.nq = b(NQ); j.wr = wf(false); j.wri = wv(false); j.wq = wf(true);
+		j.steps = steps; j.bits = bits; j.a = a;
+		CK(launch_resident(j, tc, st));
+		++launches;
+	}
+
 	// squareMMGW (transformGPU.h:556-568)
 	void square_mul(u32 a)
 	{
+		if (resident && !split) { run_resident(b(REG0), nullptr, 1, 1, a); prefwd = false; return; }
 		prefwd_reg0();
 		first_product(a, nullptr, nullptr, nullptr, q_pending);
 		reduce_tail(b(TQ), b(REG0), true, overlap);
@@ -669,6 +682,7 @@ struct ab_transform
 		if (!make_geometry(prm.ln, lb, g)) throw ab_error(AB_E_ARG, "geometry not available for this length");
 		CK(cudaStreamSynchronize(st));
 		use_geometry(g);
+		resident = false;                        // the caller wants the passes, with this split
 		prefwd = false;                          // AQ0/AR0 hold levels of the old split
 		if (gexec) { cudaGraphExecDestroy(gexec); gexec = nullptr; }
 	}
@@ -676,6 +690,12 @@ struct ab_transform
 	// mulMMGW (transformGPU.h:540-554)
 	void mul(int dst, int src)
 	{
+		if (resident)
+		{
+			run_resident(b(dst), b(src), 1, 0, 1);
+			if (dst == REG0) prefwd = false;
+			return;
+		}
 		full_forward(b(src), b(OPQ), b(OPR));
 		{ ColJob j = cj_norm(b(dst)); set_fwd(j, b(AQ0), b(AR0)); cols(j); }
 		prefwd = false;
@@ -833,8 +853,19 @@ struct ab_transform
 		host.assign((size_t)AB_NW * n, 0);
 		upload_twiddles();
 		setup_device(pp);
+		resident = resident_fits(tc);
 	}
 };
+
+// Slots of a batch up to which a chunk runs resident (resident.cu) and not as
+// passes.  Measured on B200, 64 squarings, us per step of the whole batch
+// (resident / passes with their best split): ln 9 (K = 3) 256 slots 36.1 / 58.6;
+// ln 10 (K = 5) 256 slots 87.9 / 107.8; ln 11 (K = 5) 32 slots 33.2 / 38.5, 64
+// slots 59.1 / 53.5; ln 12 (K = 5) 16 slots 32.0 / 36.8, 32 slots 59.7 / 47.9.
+static int resident_slots(int ln)
+{
+	return (ln <= 10) ? 1 << 30 : (ln == 11) ? 32 : (ln == 12) ? 16 : 0;
+}
 
 // ============================================================ batches
 // A size class (K, pck, ln) of `cap` candidates with stacked buffers: buffer
@@ -867,6 +898,7 @@ struct ab_batch
 	cudaGraphExec_t gexec = nullptr;
 	int g_steps = 0;
 	uint64_t g_kernels = 0;
+	bool resident = false;             // short length: a chunk is one launch (resident.cu)
 	int zl = 0;                        // slots the graph launches (grid.z): a power of two covering every live slot
 	uint64_t launches = 0;
 
@@ -1068,6 +1100,16 @@ int ab_square_mul_bits(ab_transform * h, const uint64_t * bits, size_t count, in
 		auto m_at = [&](size_t i) { return ((bits[i / 64] >> (i % 64)) & 1) ? (u32)a : 1u; };
 		size_t i = 0;
 		const size_t G = ab_transform::GRAPH_STEPS;
+		if (h->resident)
+		{
+			for (; i < count; i += 64)
+			{
+				const int steps = (int)std::min<size_t>(64, count - i);
+				h->run_resident(h->b(ab_transform::REG0), nullptr, steps, bits[i / 64], (u32)a);
+			}
+			h->prefwd = false;
+			return;
+		}
 		if (!h->view && h->prof_used >= h->prof.size())
 		{
 			u32 m[ab_transform::GRAPH_STEPS];
@@ -1298,6 +1340,13 @@ int ab_square_mul_noalloc(ab_transform * h, uint32_t * reg, int32_t a)
 		// scratch word is written before it is read within the call, so
 		// nothing needs clearing between calls.
 		CK(launch_import(h->rc, reg, x, (u32)n, flag, h->st));
+		if (h->resident)
+		{
+			h->run_resident(x, nullptr, 1, 1, (u32)a);
+			CK(launch_export(h->rc, x, reg, (u32)n, h->st));
+			h->launches += 2;
+			return;
+		}
 		ColJob j0 = h->cj_norm(x); h->set_fwd(j0, aq0, ar0); h->cols(j0);
 		RowJob rq = h->rj(aq0, ROW_SQUARE, true), rr = h->rj(ar0, ROW_SQUARE, false);
 		h->rows(rq, &rr);
@@ -1453,6 +1502,7 @@ int ab_batch_create(int device, const ab_params * cls, int capacity, int max_ste
 		RowJobs rjs{}; ColJobs cjs{};
 		CK(launch_rowpass(b->geo, b->tc, rjs, 1, b->st, 0));
 		CK(launch_colpass(b->geo, b->tc, cjs, 1, b->st, 0));
+		b->resident = resident_fits(b->tc);
 		CK(cudaStreamSynchronize(b->st));
 	});
 	if (rc != AB_OK) { delete b; return rc; }
@@ -1502,7 +1552,7 @@ void batch_prepare(int count, const uint64_t * const * Nl, const size_t * nlimbs
 // batch's shared buffers and stream.
 void batch_attach(ab_batch * b, ab_transform * v, int slot)
 {
-	v->device = b->device; v->st = b->st; v->overlap = false;
+	v->device = b->device; v->st = b->st; v->overlap = false; v->resident = b->resident;
 	v->KP = b->cls.K + 1;
 	v->d_flag = b->d_flag;
 	for (int i = 0; i < ab_transform::NSLOT; ++i) v->bufp[i] = b->base[i] + (size_t)slot * b->slot_words(i);
@@ -1710,6 +1760,20 @@ int ab_batch_steps(ab_batch * b, int steps, const uint32_t * mult, const uint8_t
 		CK(cudaMemcpyAsync(b->d_ctrl, hc, (size_t)3 * steps * cap * 4, cudaMemcpyHostToDevice, b->st));
 		CK(cudaEventRecord(b->ctrl_done[hi], b->st));
 		b->ctrl_i ^= 1;
+		if (b->resident && zl <= resident_slots(b->cls.ln))
+		{
+			using T = ab_transform;
+			ResJob j; std::memset(&j, 0, sizeof(j));
+			j.reg = b->base[T::REG0]; j.nir = b->base[T::NIR]; j.nq = b->base[T::NQ];
+			j.wr = b->wf(false); j.wri = b->wv(false); j.wq = b->wf(true);
+			j.steps = steps; j.mult = b->ctrl(0, 0); j.snap = b->ctrl(0, 2); j.out_snap = b->base[T::SNAP];
+			j.ctrl_stride = (size_t)3 * cap; j.stride_norm = b->w_norm; j.stride_ntt = b->w_ntt; j.cand = b->d_cand;
+			CK(launch_resident(j, b->tc, b->st, zl));
+			CK(cudaEventRecord(b->chunk_done, b->st));
+			++b->launches;
+			for (ab_transform * v : b->views) if (v) v->prefwd = false;
+			return;
+		}
 		if (b->gexec == nullptr || b->g_steps != steps || b->zl != zl)
 		{
 			if (b->gexec) { cudaGraphExecDestroy(b->gexec); b->gexec = nullptr; }
@@ -1742,8 +1806,9 @@ int ab_batch_set_geometry(ab_batch * b, int lb)
 		CK(cudaStreamSynchronize(b->st));
 		b->geo = g;
 		++b->geo_version;
+		b->resident = false;                     // the caller wants the passes, with this split
 		apply_geometry(b->tc, g);
-		for (ab_transform * v : b->views) if (v) { v->use_geometry(g); v->prefwd = false; }
+		for (ab_transform * v : b->views) if (v) { v->use_geometry(g); v->resident = false; v->prefwd = false; }
 		RowJobs rjs{}; ColJobs cjs{};
 		CK(launch_rowpass(b->geo, b->tc, rjs, 1, b->st, 0));
 		CK(launch_colpass(b->geo, b->tc, cjs, 1, b->st, 0));
@@ -1772,6 +1837,16 @@ int ab_batch_autotune(ab_batch * b, int src, int steps, int * row_levels)
 			auto it = g_tuned.find(key);
 			if (it != g_tuned.end()) best = it->second;
 		}
+		// the split only matters to the passes; choosing one keeps the resident
+		// runs of the slot counts that have them
+		const bool resident = b->resident;
+		struct Keep
+		{
+			ab_batch * b; bool resident;
+			~Keep() { b->resident = resident; for (ab_transform * v : b->views) if (v) v->resident = resident; }
+		} keep{ b, resident };
+		if (resident && b->cap <= resident_slots(b->cls.ln)) best = b->geo.LB;
+		else b->resident = false;
 		if (best == 0)
 		{
 			// copies of `src` fill the empty slots; only they step (src and the

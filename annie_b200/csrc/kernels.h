@@ -130,6 +130,32 @@ size_t fused_rowpass_smem(int log_r);
 cudaError_t launch_fused_rowpass(const FusedRowPass * d, const TConst * tcs, u32 ctas, size_t smem, cudaStream_t s);
 cudaError_t launch_fused_colpass(const FusedColPass * d, const TConst * tcs, u32 ctas, size_t smem, cudaStream_t s);
 
+// Runs of squarings of short transforms (lengths up to 2^12), one launch for
+// the whole run: a thread-block cluster per candidate (resident.cu).
+struct ResJob
+{
+	u32 * reg;                 // normal-form register, replaced by the result of the last step
+	const u32 * y;             // nullable: the steps multiply by this normal-form register instead of squaring
+	const u32 * nir, * nq;     // transforms of N^-1 (domain R) and N (domain Q)
+	const uint2 * wr, * wri, * wq;   // row tables
+	int steps;
+	// multiplier of step s: mult[s * ctrl_stride + candidate] (0 = the candidate
+	// rests), or with mult null: a where bit s of `bits` is set (at most 64
+	// steps), else 1
+	u64 bits;
+	u32 a;
+	const u32 * mult;
+	const u32 * snap;          // nullable: nonzero = the step's result also goes to out_snap
+	u32 * out_snap;
+	size_t ctrl_stride;
+	size_t stride_norm, stride_ntt;  // words between candidates (reg, y, out_snap; nir, nq)
+	const CandConst * cand;    // per-candidate digit size (nullable)
+};
+// Whether the class and length of c have a resident kernel that fits the
+// current device.
+bool resident_fits(const TConst & c);
+cudaError_t launch_resident(const ResJob & J, const TConst & c, cudaStream_t s, int ncand = 1);
+
 // Register words of the reference (K planes of residues mod its primes) from
 // the normal form, and back.  The import sets *bad when a coefficient's value
 // does not fit the 96-bit normal form (the words are not a normal-form

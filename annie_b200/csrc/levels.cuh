@@ -1,0 +1,213 @@
+// Butterfly levels of one transform (or one row of a longer one) of 2^LN words
+// held in shared memory, shared by the row pass (kernels.cu) and the resident
+// kernel (resident.cu).
+//
+// 8 words per thread: stages of 3 levels, the top one taking the remainder,
+// and a bottom step of two levels, the pointwise product and two inverse
+// levels.  A stage costs a shared-memory round trip and a barrier, about the
+// same as its three levels; 16 words per thread would save one stage of a
+// row, but halves the warps that hide each other's latency.
+#pragma once
+#include "kernels.h"
+
+namespace ab
+{
+
+// Layout in shared memory: 4 pad words per 32, so that the stages (8 words at
+// stride 1, 8, 64, 512 per thread) have no bank conflicts and groups of 4
+// words stay 16-byte aligned.
+__host__ __device__ constexpr u32 rpad(u32 e) { return e + ((e >> 5) << 2); }
+
+// Twiddles of the 2^LN words: the level with 2^t polynomials at w + (wb << t)
+// + j, as Shoup pairs; -w^-1 of the inverse levels at wi + (ib << t) + j, or
+// mirrored, wi + (ib << t) + 2^t - 1 - j (domain Q, where that is the forward
+// table of the mirrored row).  GLOBAL: tables in global memory, else shared.
+struct LevelTw
+{
+	const uint2 * w, * wi;
+	u32 wb, ib;
+	bool mirror;
+};
+
+// CNT adjacent pairs from p (aligned to them)
+template <int CNT, bool GLOBAL>
+__device__ __forceinline__ void load_pairs(const uint2 * p, uint2 (&v)[CNT])
+{
+	if constexpr (CNT == 1) v[0] = GLOBAL ? __ldg(p) : *p;
+	else
+	{
+#pragma unroll
+		for (int i = 0; i < CNT / 2; ++i)
+		{
+			const uint4 q = GLOBAL ? __ldg(reinterpret_cast<const uint4 *>(p) + i) : reinterpret_cast<const uint4 *>(p)[i];
+			v[2 * i] = make_uint2(q.x, q.y); v[2 * i + 1] = make_uint2(q.z, q.w);
+		}
+	}
+}
+
+// The twiddles j = x .. x + CNT - 1 of level t (CNT divides x).
+template <int CNT, bool INV, bool GLOBAL>
+__device__ __forceinline__ void level_tw(const LevelTw & tw, int t, u32 x, uint2 (&v)[CNT])
+{
+	if (!INV) load_pairs<CNT, GLOBAL>(tw.w + (tw.wb << t) + x, v);
+	else if (!tw.mirror) load_pairs<CNT, GLOBAL>(tw.wi + (tw.ib << t) + x, v);
+	else
+	{
+		uint2 r[CNT];
+		load_pairs<CNT, GLOBAL>(tw.wi + (tw.ib << t) + (1u << t) - x - CNT, r);
+#pragma unroll
+		for (int i = 0; i < CNT; ++i) v[i] = r[CNT - 1 - i];
+	}
+}
+
+// One level of a group's 2^S words: on group bit s, level t = LN - 1 - (B + s).
+template <int LN, int S, int B, bool INV, bool GLOBAL, int SB>
+__device__ __forceinline__ void level(u32 (&v)[1 << S], const LevelTw & tw, u32 ohi, u32 p, u32 p2)
+{
+	constexpr int CNT = 1 << (S - 1 - SB);
+	uint2 wv[CNT];
+	level_tw<CNT, INV, GLOBAL>(tw, LN - 1 - (B + SB), ohi << (S - 1 - SB), wv);
+#pragma unroll
+	for (int jh = 0; jh < CNT; ++jh)
+#pragma unroll
+		for (int gl = 0; gl < (1 << SB); ++gl)
+		{
+			const int g = (jh << (SB + 1)) + gl;
+			if (INV) inv_bf(v[g], v[g + (1 << SB)], wv[jh].x, wv[jh].y, p, p2);
+			else fwd_bf(v[g], v[g + (1 << SB)], wv[jh].x, wv[jh].y, p, p2);
+		}
+}
+
+// Levels on index bits B..B+S-1: forward from the top one, inverse from the
+// bottom one.  SRC / DST: the words lie in shared memory (padded) or, for the
+// outer end of a row, in global memory (plain).
+enum Where { IN_SHARED, IN_GLOBAL };
+template <int LN, int S, int B, bool INV, bool GLOBAL, Where SRC, Where DST>
+__device__ __forceinline__ void level_stage(const u32 * src, u32 * dst, const LevelTw & tw, u32 tid, u32 NT, u32 p, u32 p2)
+{
+	constexpr u32 N = 1u << LN;
+	for (u32 o = tid; o < (N >> S); o += NT)
+	{
+		u32 v[1 << S];
+		const u32 ohi = o >> B;
+		const u32 e0 = (o & ((1u << B) - 1)) | (ohi << (B + S)), a0 = rpad(e0);
+#pragma unroll
+		for (int g = 0; g < (1 << S); ++g) v[g] = (SRC == IN_GLOBAL) ? src[e0 + ((u32)g << B)] : src[a0 + rpad((u32)g << B)];
+		if constexpr (INV)
+		{
+			level<LN, S, B, true, GLOBAL, 0>(v, tw, ohi, p, p2);
+			if constexpr (S > 1) level<LN, S, B, true, GLOBAL, 1>(v, tw, ohi, p, p2);
+			if constexpr (S > 2) level<LN, S, B, true, GLOBAL, 2>(v, tw, ohi, p, p2);
+			if constexpr (S > 3) level<LN, S, B, true, GLOBAL, 3>(v, tw, ohi, p, p2);
+		}
+		else
+		{
+			if constexpr (S > 3) level<LN, S, B, false, GLOBAL, 3>(v, tw, ohi, p, p2);
+			if constexpr (S > 2) level<LN, S, B, false, GLOBAL, 2>(v, tw, ohi, p, p2);
+			if constexpr (S > 1) level<LN, S, B, false, GLOBAL, 1>(v, tw, ohi, p, p2);
+			level<LN, S, B, false, GLOBAL, 0>(v, tw, ohi, p, p2);
+		}
+#pragma unroll
+		for (int g = 0; g < (1 << S); ++g)
+		{
+			if (DST == IN_GLOBAL) dst[e0 + ((u32)g << B)] = v[g];
+			else dst[a0 + rpad((u32)g << B)] = v[g];
+		}
+	}
+}
+
+// Pointwise product of 4 adjacent degree-1 polynomials (v[2m], v[2m+1]) mod
+// (x^2 -+ c), words in [0, 2p); c0 for the first two, c1 for the others (even
+// polynomials -c, odd ones +c).  y: the other factor (mul), else a square.
+__device__ __forceinline__ void pointwise4(u32 (&v)[8], const u32 (&y)[8], bool mul, uint2 c0, uint2 c1, u32 p, u32 p2, u32 pinv)
+{
+#pragma unroll
+	for (int m = 0; m < 4; ++m)
+	{
+		const u32 cm = mont_twiddle((m < 2) ? c0 : c1, p);
+		poly_product(v[2 * m], v[2 * m + 1], mul ? y[2 * m] : v[2 * m], mul ? y[2 * m + 1] : v[2 * m + 1], mul,
+			((m & 1) == 0) ? cm : p - cm, p, p2, pinv);
+	}
+}
+
+enum BottomMode { BOTTOM_SQUARE = 0, BOTTOM_MUL = 1, BOTTOM_FORWARD = 2 };
+
+// The bottom of a transform, 8 adjacent words per thread: the last two forward
+// levels, the pointwise product, the first two inverse levels, in place; or
+// (BOTTOM_FORWARD) the last two levels only, the words in [0, 2p) to out.
+// op(o, a, b) gives the other factor's words 8 o .. 8 o + 7, out(o, a, b) takes
+// the image.
+template <int LN, bool GLOBAL, typename Op, typename Out>
+__device__ __forceinline__ void level_bottom(u32 * x, int mode, const LevelTw & tw, u32 tid, u32 NT, u32 p, u32 p2, u32 pinv, Op op, Out out)
+{
+	constexpr u32 N = 1u << LN;
+	for (u32 o = tid; o < N / 8; o += NT)
+	{
+		u32 v[8], y[8];
+		uint4 * const xp = reinterpret_cast<uint4 *>(x + rpad(8 * o));
+		uint4 a = make_uint4(0, 0, 0, 0), b = a;
+		if (mode == BOTTOM_MUL) op(o, a, b);
+		y[0] = a.x; y[1] = a.y; y[2] = a.z; y[3] = a.w; y[4] = b.x; y[5] = b.y; y[6] = b.z; y[7] = b.w;
+		a = xp[0]; b = xp[1];
+		v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+		uint2 w0[1], w1[2];
+		level_tw<1, false, GLOBAL>(tw, LN - 3, o, w0);
+		level_tw<2, false, GLOBAL>(tw, LN - 2, 2 * o, w1);
+#pragma unroll
+		for (int i = 0; i < 4; ++i) fwd_bf(v[i], v[i + 4], w0[0].x, w0[0].y, p, p2);
+#pragma unroll
+		for (int i = 0; i < 2; ++i)
+		{
+			fwd_bf(v[i], v[i + 2], w1[0].x, w1[0].y, p, p2);
+			fwd_bf(v[i + 4], v[i + 6], w1[1].x, w1[1].y, p, p2);
+		}
+#pragma unroll
+		for (int i = 0; i < 8; ++i) v[i] = red2(v[i], p2);
+		if (mode == BOTTOM_FORWARD)
+		{
+			out(o, make_uint4(v[0], v[1], v[2], v[3]), make_uint4(v[4], v[5], v[6], v[7]));
+			continue;
+		}
+		pointwise4(v, y, mode == BOTTOM_MUL, w1[0], w1[1], p, p2, pinv);
+		level_tw<2, true, GLOBAL>(tw, LN - 2, 2 * o, w1);
+		level_tw<1, true, GLOBAL>(tw, LN - 3, o, w0);
+#pragma unroll
+		for (int i = 0; i < 2; ++i)
+		{
+			inv_bf(v[i], v[i + 2], w1[0].x, w1[0].y, p, p2);
+			inv_bf(v[i + 4], v[i + 6], w1[1].x, w1[1].y, p, p2);
+		}
+#pragma unroll
+		for (int i = 0; i < 4; ++i) inv_bf(v[i], v[i + 4], w0[0].x, w0[0].y, p, p2);
+		xp[0] = make_uint4(v[0], v[1], v[2], v[3]);
+		xp[1] = make_uint4(v[4], v[5], v[6], v[7]);
+	}
+}
+
+// A whole transform step: the words at src (shared, padded, or global) through
+// all forward levels, the pointwise product and all inverse levels into dst,
+// working in x (shared).  src may be x, dst may be x.  The caller's barrier
+// makes src and the tables visible; on return the words of dst are written but
+// not yet ordered for other threads.
+template <int LN, bool GLOBAL, Where SRC, Where DST, typename Op, typename Out>
+__device__ __forceinline__ void level_transform(const u32 * src, u32 * x, u32 * dst, int mode, const LevelTw & tw, u32 tid, u32 NT,
+	u32 p, u32 pinv, Op op, Out out)
+{
+	const u32 p2 = 2 * p;
+	constexpr int REM = (LN - 3) % 3;
+	constexpr int TOP = (REM == 0) ? 3 : (REM == 1 && LN >= 13) ? 4 : REM, BT = LN - TOP;    // the top stage: bits BT..LN-1
+	level_stage<LN, TOP, BT, false, GLOBAL, SRC, IN_SHARED>(src, x, tw, tid, NT, p, p2);
+	__syncthreads();
+	if constexpr (BT >= 12) { level_stage<LN, 3, 9, false, GLOBAL, IN_SHARED, IN_SHARED>(x, x, tw, tid, NT, p, p2); __syncthreads(); }
+	if constexpr (BT >= 9) { level_stage<LN, 3, 6, false, GLOBAL, IN_SHARED, IN_SHARED>(x, x, tw, tid, NT, p, p2); __syncthreads(); }
+	if constexpr (BT >= 6) { level_stage<LN, 3, 3, false, GLOBAL, IN_SHARED, IN_SHARED>(x, x, tw, tid, NT, p, p2); __syncthreads(); }
+	level_bottom<LN, GLOBAL>(x, mode, tw, tid, NT, p, p2, pinv, op, out);
+	if (mode == BOTTOM_FORWARD) return;
+	__syncthreads();
+	if constexpr (BT >= 6) { level_stage<LN, 3, 3, true, GLOBAL, IN_SHARED, IN_SHARED>(x, x, tw, tid, NT, p, p2); __syncthreads(); }
+	if constexpr (BT >= 9) { level_stage<LN, 3, 6, true, GLOBAL, IN_SHARED, IN_SHARED>(x, x, tw, tid, NT, p, p2); __syncthreads(); }
+	if constexpr (BT >= 12) { level_stage<LN, 3, 9, true, GLOBAL, IN_SHARED, IN_SHARED>(x, x, tw, tid, NT, p, p2); __syncthreads(); }
+	level_stage<LN, TOP, BT, true, GLOBAL, IN_SHARED, DST>(x, dst, tw, tid, NT, p, p2);
+}
+
+} // namespace ab

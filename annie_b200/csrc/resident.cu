@@ -1,0 +1,408 @@
+// Short transforms (up to 2^12 words per prime), resident in shared memory.
+//
+// One thread-block cluster holds one candidate for a whole run of squarings:
+// CTA dom KP + k keeps the transform of prime k in domain dom (0 = R, 1 = Q)
+// in its shared memory, with the twiddles and the image of N^-1 (R) or N (Q).
+// A squaring is three products; each is a transform step inside every CTA
+// (forward levels, pointwise product, inverse levels) and a carry step over
+// coefficients, in which every CTA gathers the residues of its range from the
+// others (distributed shared memory), carries, and writes the new residues
+// into the CTAs of the next product.  A hardware cluster barrier separates the
+// steps: six per squaring, where the row and column passes need six dependent
+// kernel launches and the L2 between them.  Those short launches cost 3 to
+// 5 us each whatever the length; the cluster's steps cost what their longest
+// dependency chain costs.
+//
+// The arithmetic is that of the passes (kernels.cu): the same primes, twiddle
+// positions, products, CRT and carry rule, so the registers are the same.
+#include <atomic>
+#include <type_traits>
+
+#include "kernels.h"
+#include "carry.cuh"
+#include "levels.cuh"
+
+namespace ab
+{
+
+namespace
+{
+
+__device__ __forceinline__ u32 cluster_rank()
+{
+	u32 r;
+	asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+	return r;
+}
+
+// All threads of the cluster; orders shared-memory accesses of all its CTAs.
+__device__ __forceinline__ void cluster_sync()
+{
+	__syncwarp();
+	asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Address of this CTA's shared variable at p, in CTA `rank` of the cluster.
+__device__ __forceinline__ u32 remote(const void * p, u32 rank)
+{
+	u32 r;
+	asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((u32)__cvta_generic_to_shared(p)), "r"(rank));
+	return r;
+}
+__device__ __forceinline__ u32 ld_remote(u32 a)
+{
+	u32 v;
+	asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+	return v;
+}
+__device__ __forceinline__ void st_remote(u32 a, u32 v)
+{
+	asm volatile("st.shared::cluster.u32 [%0], %1;" :: "r"(a), "r"(v) : "memory");
+}
+
+#ifndef AB_RES_REGT
+#define AB_RES_REGT 1024
+#endif
+template <int LN, int K>
+struct ResCfg
+{
+	static constexpr int KP = K + 1, C = 2 * KP;               // CTAs of a cluster
+	static constexpr u32 N = 1u << LN, G = N / 4;              // words, groups of 4 coefficients
+	static constexpr u32 Q = (G + C - 1) / C;                  // groups of a CTA in the carry steps
+	// threads of one domain's carry: a lane per coefficient, two predecessor groups
+	static constexpr u32 NC = ((Q + 2) * 4 + 31) / 32 * 32;
+	static constexpr bool BOTH = 2 * NC <= 512;                // both domains of the first product at once
+	static constexpr u32 NT0 = (N / 8 > NC) ? N / 8 : NC;
+	static constexpr u32 NT = (BOTH && 2 * NC > NT0) ? 2 * NC : (NT0 < 64) ? 64 : (NT0 + 31) / 32 * 32;
+	// shared memory, words: two work buffers, two operand images, twiddles (two
+	// tables of N/2 pairs), T_Q, carries of both domains
+	static constexpr u32 W = rpad(N);
+	static constexpr u32 TQ = Q * 4 * AB_NW, CWN = (Q + 2) * K;
+	static constexpr size_t SMEM = sizeof(u32) * (2 * W + 2 * N + 2 * N + TQ + 2 * CWN);
+	// CTAs per SM that the kernel is compiled for
+	static constexpr u32 BY_T = AB_RES_REGT / NT, BY_S = (u32)((size_t)227 * 1024 / (SMEM + 1024));
+	static constexpr u32 MINB = (BY_T < BY_S ? BY_T : BY_S) < 1 ? 1 : (BY_T < BY_S ? BY_T : BY_S);
+};
+
+// One transform step of a CTA: the residues in xb, forward, product with the
+// image op, inverse into xa; or (BOTTOM_FORWARD) the image into op.  op: two
+// planes of N/8 uint4 (a thread's 8 words, without bank conflicts).
+template <int LN>
+__device__ __forceinline__ void res_transform(const u32 * xb, u32 * xa, u32 * op, int mode, const LevelTw & tw, u32 p, u32 pinv)
+{
+	uint4 * const q = reinterpret_cast<uint4 *>(op);
+	constexpr u32 N8 = (1u << LN) / 8;
+	level_transform<LN, false, IN_SHARED, IN_SHARED>(xb, xa, xa, mode, tw, threadIdx.x, blockDim.x, p, pinv,
+		[&](u32 o, uint4 & a, uint4 & b) { a = q[o]; b = q[N8 + o]; },
+		[&](u32 o, uint4 a, uint4 b) { q[o] = a; q[N8 + o] = b; });
+}
+
+// The carry of one product, a lane per coefficient and 4 lanes per group
+// (t: thread of the domain, below NC): the group's predecessor groups come
+// first (two in CTA 0, which re-derives the register's last coefficient for
+// the mod R / mod Q decision; one in the others).  Returns the coefficient's
+// exact value in x, and whether the lane owns it.
+template <int LN, int K, int PCK, bool FULL>
+__device__ __forceinline__ bool res_carry(const TConst & c, u32 rank, u32 t, u32 src, bool nega, u32 amul, const u32 * tq, int lower,
+	const Width & w, int wbits, const u32 * xa, u32 * cw, int * decision, u32 (&x)[AB_NW], u32 & e)
+{
+	using Cfg = ResCfg<LN, K>;
+	constexpr int KP = Cfg::KP, L = K, ND = DigitLimbs<PCK>::N;
+	constexpr u32 G = Cfg::G, Q = Cfg::Q, N = Cfg::N;
+	const u32 g0 = rank * Q, cnt = (g0 >= G) ? 0u : (G - g0 < Q) ? G - g0 : Q;
+	const u32 E = (cnt == 0) ? 0u : (rank == 0) ? 2u : 1u;
+	const u32 li = t >> 2, j = t & 3;
+	const bool active = li < E + cnt;
+	u32 g = g0 + li - E;                          // group (CTA 0's predecessors end the register)
+	if (rank == 0 && li < E) g += G;
+	e = active ? 4 * g + j : 0u;
+	Big<L> f = big_zero<L>();
+	if (active)
+	{
+		u32 y[KP];
+		const u32 o = (u32)sizeof(u32) * rpad(e);
+#pragma unroll
+		for (int k = 0; k < KP; ++k) y[k] = ld_remote(remote(xa, src + k) + o);
+		u32 s[AB_NW];
+		if (tq != nullptr)
+		{
+			const u32 own = g / Q;
+			const u32 a = remote(tq, own) + (u32)sizeof(u32) * (4 * (g - own * Q) + j);
+#pragma unroll
+			for (int l = 0; l < AB_NW; ++l) s[l] = ld_remote(a + l * (u32)sizeof(u32) * 4 * Q);
+		}
+		f = crt<L>(c, y);
+		if (amul != 1u) f = big_mul_u32<L>(f, amul);
+		if (tq != nullptr) f = big_sub<L>(f, big_from_exact<L>(s[0], s[1], s[2]));
+	}
+	// phase 1: the group's digits and carry-out
+	u32 d[ND];
+	lane_digits<FULL, L, ND>(f, w, j, d);
+	if (active && j == 3)
+	{
+#pragma unroll
+		for (int l = 0; l < L; ++l) cw[li * L + l] = f.l[l];
+	}
+	__syncthreads();
+	// phase 2: the previous group's carry-out, balanced digits; the last
+	// coefficient of a group absorbs the rest
+	const bool top0 = (lower != LOWER_NONE) && rank == 0 && li == 1;
+	const bool mine = active && li >= E;
+	Big<L> cin = big_zero<L>();
+	if (j == 0 && (mine || top0))
+	{
+#pragma unroll
+		for (int l = 0; l < L; ++l) cin.l[l] = cw[(li - 1) * L + l];
+		if (g == 0 && nega) cin = big_neg<L>(cin);
+	}
+	lane_balance<FULL, L, ND>(cin, d, w, half_of(wbits), j, x);
+	if (lower != LOWER_NONE)
+	{
+		// mod R (+2) / mod Q on the top and bottom coefficients (kernel.cl:1653-1683):
+		// whether the last coefficient is 2^W or more
+		if ((mine || top0) && e == N - 1) *decision = reaches_width(x, w) ? 1 : 0;
+		__syncthreads();
+		if (mine && (e == 0 || e == N - 1))
+		{
+			Big<AB_NW> a, b;
+#pragma unroll
+			for (int i = 0; i < AB_NW; ++i) a.l[i] = x[i];
+			if (e == 0)
+			{
+				int dv = 0;
+				if (*decision) dv += (lower == LOWER_Q) ? -1 : 1;
+				if (lower == LOWER_R_ADD2) dv += 2;
+				b.l[0] = (u32)dv; b.l[1] = b.l[2] = (u32)(dv >> 31);
+				a = big_add<AB_NW>(a, b);
+			}
+			else if (*decision)
+			{
+#pragma unroll
+				for (int i = 0; i < AB_NW; ++i) b.l[i] = (i == (wbits >> 5)) ? 1u << (wbits & 31) : 0u;
+				a = big_sub<AB_NW>(a, b);
+			}
+#pragma unroll
+			for (int i = 0; i < AB_NW; ++i) x[i] = a.l[i];
+		}
+	}
+	return mine;
+}
+
+template <int LN, int K, int PCK>
+__global__ void __launch_bounds__(ResCfg<LN, K>::NT, ResCfg<LN, K>::MINB) k_resident(const ResJob J, const TConst c)
+{
+	using Cfg = ResCfg<LN, K>;
+	constexpr int KP = Cfg::KP;
+	constexpr u32 N = Cfg::N, W = Cfg::W, NC = Cfg::NC;
+	extern __shared__ __align__(16) u32 sm[];
+	__shared__ int decision;
+	u32 * const xa = sm, * const xb = xa + W;               // transform step: xb -> xa
+	u32 * const op = xb + W, * const op2 = op + N;          // image of N^-1 / N; of the second factor
+	uint2 * const w = reinterpret_cast<uint2 *>(op2 + N);
+	uint2 * const wi = w + N / 2;
+	u32 * const tq = reinterpret_cast<u32 *>(wi + N / 2);   // T_Q of this CTA's coefficients, three planes of 4 Q words
+	u32 * const cwr = tq + Cfg::TQ, * const cwq = cwr + Cfg::CWN;
+
+	const u32 rank = cluster_rank(), cand = blockIdx.y;
+	const u32 dom = rank / KP, k = rank - dom * KP;
+	const u32 tid = threadIdx.x, NT = Cfg::NT;
+	const u32 p = c.p[k], pinv = c.pinv[k];
+	// the last step that the slot takes part in; an idle slot's cluster leaves
+	__shared__ int last;
+	if (tid == 0) last = (J.mult != nullptr) ? -1 : J.steps - 1;
+	__syncthreads();
+	if (J.mult != nullptr)
+	{
+		for (int s = (int)tid; s < J.steps; s += (int)NT)
+			if (J.mult[(size_t)s * J.ctrl_stride + cand] != 0u) atomicMax(&last, s);
+		__syncthreads();
+		if (last < 0) return;
+	}
+
+	const size_t on = (size_t)cand * J.stride_norm, ot = (size_t)cand * J.stride_ntt;
+	u32 * const reg = J.reg + on;
+	const uint2 * const gw = (dom == 0 ? J.wr : J.wq) + (size_t)k * (N / 2);
+	for (u32 i = tid; i < N / 2; i += NT)
+	{
+		w[i] = __ldg(gw + i);
+		if (dom == 0) wi[i] = __ldg(J.wri + (size_t)k * (N / 2) + i);
+	}
+	const LevelTw tw{ w, (dom == 0) ? wi : w, 1u, 1u, dom != 0 };
+	{
+		const uint4 * img = reinterpret_cast<const uint4 *>((dom == 0 ? J.nir : J.nq) + ot + (size_t)k * N);
+		uint4 * o4 = reinterpret_cast<uint4 *>(op);
+		for (u32 i = tid; i < N / 4; i += NT) o4[(i & 1) * (N / 8) + (i >> 1)] = __ldg(img + i);
+	}
+	auto encode_all = [&](const u32 * src) {
+		for (u32 i = tid; i < N; i += NT) xb[rpad(i)] = encode_res(c, (int)k, split30(src[i], src[N + i], src[2 * N + i]));
+	};
+	if (J.y != nullptr)
+	{
+		encode_all(J.y + on);
+		__syncthreads();
+		res_transform<LN>(xb, xa, op2, BOTTOM_FORWARD, tw, p, pinv);
+		__syncthreads();
+	}
+	encode_all(reg);
+	__syncthreads();
+
+	const int wbits = PCK * ((J.cand != nullptr) ? J.cand[cand].lbase : c.lbase);
+	const Width wd = make_width(wbits);
+	const bool full = (wd.ws == DigitLimbs<PCK>::N - 1);
+	auto carry = [&](u32 t, u32 src, bool nega, u32 amul, const u32 * sub, int lower, u32 * cw, u32 (&x)[AB_NW], u32 & e) {
+		return full ? res_carry<LN, K, PCK, true>(c, rank, t, src, nega, amul, sub, lower, wd, wbits, xa, cw, &decision, x, e)
+		            : res_carry<LN, K, PCK, false>(c, rank, t, src, nega, amul, sub, lower, wd, wbits, xa, cw, &decision, x, e);
+	};
+	// residues of a coefficient into the CTAs of domain d
+	auto scatter = [&](const u32 (&x)[AB_NW], u32 e, bool r_dom, bool q_dom) {
+		const Pieces a = split30(x[0], x[1], x[2]);
+		const u32 o = (u32)sizeof(u32) * rpad(e);
+#pragma unroll
+		for (int q = 0; q < KP; ++q)
+		{
+			const u32 v = encode_res(c, q, a);
+			if (r_dom) st_remote(remote(xb, (u32)q) + o, v);
+			if (q_dom) st_remote(remote(xb, (u32)(KP + q)) + o, v);
+		}
+	};
+	auto keep_tq = [&](const u32 (&x)[AB_NW], u32 e) {
+		const u32 i = e - 4 * rank * Cfg::Q;
+#pragma unroll
+		for (int l = 0; l < AB_NW; ++l) tq[l * 4 * Cfg::Q + i] = x[l];
+	};
+
+#pragma unroll 1
+	for (int s = 0; s < J.steps; ++s)
+	{
+		const u32 amul = (J.mult != nullptr) ? J.mult[(size_t)s * J.ctrl_stride + cand] : ((J.bits >> s) & 1) ? J.a : 1u;
+		if (amul == 0u) continue;                 // the slot rests in this step
+		u32 x[AB_NW], e;
+		// T_R = a x y mod R, T_Q = a x y mod Q
+		res_transform<LN>(xb, xa, op2, (J.y != nullptr) ? BOTTOM_MUL : BOTTOM_SQUARE, tw, p, pinv);
+		cluster_sync();
+		if constexpr (Cfg::BOTH)
+		{
+			// the second half of the threads takes domain Q
+			const bool q = tid >= NC && tid < 2 * NC;
+			const u32 t = q ? tid - NC : tid;
+			const bool mine = carry((tid < 2 * NC) ? t : 4u * N, q ? (u32)KP : 0u, q, amul, nullptr, LOWER_NONE, q ? cwq : cwr, x, e);
+			if (mine && q) keep_tq(x, e);
+			else if (mine) scatter(x, e, true, false);
+		}
+		else
+		{
+			if (carry(tid, 0u, false, amul, nullptr, LOWER_NONE, cwr, x, e)) scatter(x, e, true, false);
+			if (carry(tid, (u32)KP, true, amul, nullptr, LOWER_NONE, cwq, x, e)) keep_tq(x, e);
+		}
+		cluster_sync();
+		// m' = T_R N^-1 mod R, + 2
+		if (dom == 0) res_transform<LN>(xb, xa, op, BOTTOM_MUL, tw, p, pinv);
+		cluster_sync();
+		if (carry(tid, 0u, false, 1u, nullptr, LOWER_R_ADD2, cwr, x, e)) scatter(x, e, false, true);
+		cluster_sync();
+		// m' N - T_Q mod Q
+		if (dom == 1) res_transform<LN>(xb, xa, op, BOTTOM_MUL, tw, p, pinv);
+		cluster_sync();
+		const bool snap = (J.snap != nullptr) && J.snap[(size_t)s * J.ctrl_stride + cand] != 0u;
+		if (carry(tid, (u32)KP, true, 1u, tq, LOWER_Q, cwr, x, e))
+		{
+			scatter(x, e, true, true);
+#pragma unroll
+			for (u32 l = 0; l < AB_NW; ++l)
+			{
+				if (s == last) reg[l * N + e] = x[l];
+				if (snap) J.out_snap[on + l * N + e] = x[l];
+			}
+		}
+		cluster_sync();
+	}
+}
+
+template <int LN, int K, int PCK>
+cudaError_t resident_t(const ResJob & J, const TConst & c, cudaStream_t s, int ncand, bool * fits)
+{
+	using Cfg = ResCfg<LN, K>;
+	static_assert(Cfg::NC <= 1024 && Cfg::NT <= 1024, "a lane per coefficient");
+	// per device: the kernel's attributes, and whether a cluster of it fits
+	static std::atomic<unsigned long long> done{0}, ok{0};
+	int dev = 0;
+	cudaError_t e = cudaGetDevice(&dev);
+	if (e != cudaSuccess) return e;
+	const unsigned long long bit = 1ull << (dev & 63);
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = dim3(Cfg::C, (unsigned)ncand);
+	cfg.blockDim = dim3(Cfg::NT);
+	cfg.dynamicSmemBytes = Cfg::SMEM;
+	cfg.stream = s;
+	cudaLaunchAttribute attr[1];
+	attr[0].id = cudaLaunchAttributeClusterDimension;
+	attr[0].val.clusterDim.x = Cfg::C;
+	attr[0].val.clusterDim.y = 1;
+	attr[0].val.clusterDim.z = 1;
+	cfg.attrs = attr;
+	cfg.numAttrs = 1;
+	if (!(done.load(std::memory_order_acquire) & bit))
+	{
+		e = cudaFuncSetAttribute(k_resident<LN, K, PCK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM);
+		if (e != cudaSuccess) return e;
+		if (Cfg::C > 8) e = cudaFuncSetAttribute(k_resident<LN, K, PCK>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+		if (e != cudaSuccess) return e;
+		cfg.gridDim = dim3(Cfg::C, 1);
+		int clusters = 0;
+		e = cudaOccupancyMaxActiveClusters(&clusters, k_resident<LN, K, PCK>, &cfg);
+		if (e != cudaSuccess) { cudaGetLastError(); clusters = 0; }
+		if (clusters > 0) ok.fetch_or(bit, std::memory_order_acq_rel);
+		done.fetch_or(bit, std::memory_order_acq_rel);
+		cfg.gridDim = dim3(Cfg::C, (unsigned)ncand);
+	}
+	const bool can = (ok.load(std::memory_order_acquire) & bit) != 0;
+	if (fits) *fits = can;
+	if (ncand == 0) return cudaSuccess;       // query and set-up only
+	if (!can) return cudaErrorNotSupported;
+	return cudaLaunchKernelEx(&cfg, k_resident<LN, K, PCK>, J, c);
+}
+
+template <int K, int PCK>
+cudaError_t resident_k(const ResJob & J, const TConst & c, cudaStream_t s, int ncand, bool * fits)
+{
+	switch (c.ln)
+	{
+	case 6: return resident_t<6, K, PCK>(J, c, s, ncand, fits);
+	case 7: return resident_t<7, K, PCK>(J, c, s, ncand, fits);
+	case 8: return resident_t<8, K, PCK>(J, c, s, ncand, fits);
+	case 9: return resident_t<9, K, PCK>(J, c, s, ncand, fits);
+	case 10: return resident_t<10, K, PCK>(J, c, s, ncand, fits);
+	case 11: return resident_t<11, K, PCK>(J, c, s, ncand, fits);
+	case 12: return resident_t<12, K, PCK>(J, c, s, ncand, fits);
+	default: if (fits) *fits = false; return (ncand == 0) ? cudaSuccess : cudaErrorNotSupported;
+	}
+}
+
+cudaError_t resident_any(const ResJob & J, const TConst & c, cudaStream_t s, int ncand, bool * fits)
+{
+	switch (c.K)
+	{
+	case 2: return resident_k<2, 1>(J, c, s, ncand, fits);
+	case 3: return resident_k<3, 2>(J, c, s, ncand, fits);
+	case 4: return resident_k<4, 2>(J, c, s, ncand, fits);
+	case 5: return resident_k<5, 4>(J, c, s, ncand, fits);
+	default: if (fits) *fits = false; return (ncand == 0) ? cudaSuccess : cudaErrorNotSupported;
+	}
+}
+
+} // namespace
+
+bool resident_fits(const TConst & c)
+{
+	bool fits = false;
+	const ResJob none{};
+	return resident_any(none, c, nullptr, 0, &fits) == cudaSuccess && fits;
+}
+
+cudaError_t launch_resident(const ResJob & J, const TConst & c, cudaStream_t s, int ncand)
+{
+	if (ncand == 0) return cudaSuccess;
+	return resident_any(J, c, s, ncand, nullptr);
+}
+
+} // namespace ab
