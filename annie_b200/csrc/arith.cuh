@@ -39,15 +39,6 @@ __device__ __forceinline__ u32 shoup(u32 x, u32 w, u32 ws, u32 p)
 	return x * w - q * p;
 }
 
-// a b 2^-32 mod p in (0, 2p) for a, b < 2p (Montgomery, pinv = p^-1 mod 2^32):
-// a b - m p with m = (a b) pinv mod 2^32 is a multiple of 2^32, and
-// a b / 2^32 < p, m p / 2^32 < p.
-__device__ __forceinline__ u32 mont(u32 a, u32 b, u32 p, u32 pinv)
-{
-	const u32 lo = a * b, hi = __umulhi(a, b);
-	return hi - __umulhi(lo * pinv, p) + p;
-}
-
 // t 2^-32 mod p for a 64-bit t < f 2^32 p, in (0, (f + 1) p) (Montgomery,
 // pinv = p^-1 mod 2^32).
 __device__ __forceinline__ u32 redc(u64 t, u32 p, u32 pinv)

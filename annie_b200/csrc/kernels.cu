@@ -99,19 +99,35 @@ __device__ __forceinline__ void rp_radix(u32 (&v)[RP_EPT], u32 tid, u32 T, int b
 			const int s = INV ? ss : (S - 1 - ss);
 			const int t = LB - b - s;
 			const u32 i0 = (Hr << t) + (ohi << (S - 1 - s));
+			// CNT = 2^(S-1-s) adjacent pairs, aligned to them: 16-byte loads
+			uint2 wv[1 << (S - 1)];
+			const int CNT = 1 << (S - 1 - s);
+			const bool mirror = INV && tw.wi == nullptr;
+			const uint2 * const wp = !INV ? tw.w + i0 : !mirror ? tw.wi + i0 : tw.w + (3u * (tw.H << t) - i0 - (u32)CNT);
+			if (CNT == 1) wv[0] = __ldg(wp);
+			else
+			{
+#pragma unroll
+				for (int i = 0; i < CNT / 2; ++i)
+				{
+					const uint4 q = __ldg(reinterpret_cast<const uint4 *>(wp) + i);
+					wv[2 * i] = make_uint2(q.x, q.y); wv[2 * i + 1] = make_uint2(q.z, q.w);
+				}
+				if (mirror)
+				{
+#pragma unroll
+					for (int i = 0; i < CNT / 2; ++i) { const uint2 q = wv[i]; wv[i] = wv[CNT - 1 - i]; wv[CNT - 1 - i] = q; }
+				}
+			}
 #pragma unroll
 			for (int jh = 0; jh < (1 << (S - 1 - s)); ++jh)
 			{
-				uint2 wv;
-				if (!INV) wv = __ldg(tw.w + i0 + jh);
-				else if (tw.wi != nullptr) wv = __ldg(tw.wi + i0 + jh);
-				else wv = __ldg(tw.w + (3u * (tw.H << t) - 1u - (i0 + jh)));
 #pragma unroll
 				for (int gl = 0; gl < (1 << s); ++gl)
 				{
 					const int g = x * (1 << S) + (jh << (s + 1)) + gl;
-					if (INV) inv_bf(v[g], v[g + (1 << s)], wv.x, wv.y, p, p2);
-					else fwd_bf(v[g], v[g + (1 << s)], wv.x, wv.y, p, p2);
+					if (INV) inv_bf(v[g], v[g + (1 << s)], wv[jh].x, wv[jh].y, p, p2);
+					else fwd_bf(v[g], v[g + (1 << s)], wv[jh].x, wv[jh].y, p, p2);
 				}
 			}
 		}
@@ -184,8 +200,8 @@ __device__ __forceinline__ void rp_store_global(const u32 (&v)[RP_EPT], u32 * __
 // lane 2m holds the x0 of the thread pair's 16 polynomials, lane 2m+1 the x1.
 // Each lane computes 8 whole products (even lane: slots 0..7, odd: 8..15).
 // Inputs: [0, 4p) from the forward levels, the other operand in [0, 2p);
-// every product is a Montgomery product (a factor 2^-32 that the carry's CRT
-// weights remove); outputs in [0, 2p) for the inverse levels.
+// a factor 2^-32, which the image factors remove (crt); outputs in [0, 2p) for
+// the inverse levels.
 // w1: the 8 twiddles of the thread pair's last forward level (just read by
 // the forward stage, so an L1 hit), which are the polynomials' c.
 __device__ __forceinline__ void rp_pointwise(u32 (&v)[RP_EPT], const u32 * __restrict__ xp, bool is_mul, u32 tid, u32 NT,
@@ -195,32 +211,21 @@ __device__ __forceinline__ void rp_pointwise(u32 (&v)[RP_EPT], const u32 * __res
 	// 32*(tid>>1) + (tid&1) + 2g); NT: physical threads of the CTA (warp mask)
 	const bool odd = (tid & 1) != 0;
 	const unsigned mask = (NT >= 32) ? 0xffffffffu : ((1u << NT) - 1);
-	const u32 * __restrict__ xq = is_mul ? xp + (tid & 1) + ((tid >> 1) << 5) : nullptr;
+	// the other factor's words of the lane's 8 polynomials are adjacent
+	const uint4 * const xq = reinterpret_cast<const uint4 *>(xp) + (tid << 2);
+	uint4 op = make_uint4(0, 0, 0, 0);
 #pragma unroll
 	for (int i = 0; i < 8; ++i)
 	{
+		if (is_mul && (i & 1) == 0) op = __ldg(xq + (i >> 1));
 		const u32 r = __shfl_xor_sync(mask, odd ? v[i] : v[8 + i], 1);
 		const u32 x0 = red2(odd ? r : v[i], p2), x1 = red2(odd ? v[8 + i] : r, p2);
 		const int slot = odd ? 8 + i : i;   // polynomial slot; parity = sign
 		const uint2 cwp = __ldg(w1 + (odd ? 4 + (i >> 1) : (i >> 1)));
-		const u32 cw = cwp.x, cs = cwp.y;
-		u32 y0, y1, t;
-		if (is_mul)
-		{
-			const u32 pa = __ldg(xq + 2 * i), pb = __ldg(xq + 2 * (8 + i));
-			const u32 rp2 = __shfl_xor_sync(mask, odd ? pa : pb, 1);
-			const u32 p0 = odd ? rp2 : pa, p1 = odd ? pb : rp2;
-			t = shoup(mont(x1, p1, p, pinv), cw, cs, p);
-			y1 = red2(mont(x0, p1, p, pinv) + mont(x1, p0, p, pinv), p2);
-			y0 = mont(x0, p0, p, pinv);
-		}
-		else
-		{
-			t = shoup(mont(x1, x1, p, pinv), cw, cs, p);
-			y1 = mont(red2(x0 + x0, p2), x1, p, pinv);
-			y0 = mont(x0, x0, p, pinv);
-		}
-		y0 = red2(((slot & 1) == 0) ? y0 + t : y0 - t + p2, p2);
+		const u32 cm = mont_twiddle(cwp, p);
+		u32 y0 = x0, y1 = x1;
+		poly_product(y0, y1, !is_mul ? x0 : ((i & 1) == 0) ? op.x : op.z, !is_mul ? x1 : ((i & 1) == 0) ? op.y : op.w, is_mul,
+			((slot & 1) == 0) ? cm : p - cm, p, p2, pinv);
 		const u32 r2 = __shfl_xor_sync(mask, odd ? y0 : y1, 1);
 		if (odd) { v[8 + i] = y1; v[i] = r2; }
 		else { v[i] = y0; v[8 + i] = r2; }
@@ -254,6 +259,31 @@ struct RowCfg
 	static constexpr int MINB = (AB_ROW_MINB * AB_ROW_THREADS > 2048) ? 2048 / AB_ROW_THREADS : AB_ROW_MINB;
 	static constexpr size_t SMEM = sizeof(u32) * ((1u << LOG_R) + (1u << LOG_R) / 16);   // padded row
 };
+
+// Starts the load of a line that is read later (to L1; the value is dropped).
+__device__ __forceinline__ void touch(const void * p)
+{
+	u32 v;
+	asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
+}
+
+// What the last stage of a row reads from global memory, per warp of virtual
+// threads vt0 .. vt0 + 31 (512 words): 15 lines of forward twiddles, 15 of
+// inverse ones (levels LB-4 .. LB-1: 128 << i bytes at level LB-4+i), and 16
+// of the other factor.  Touched ahead of the barrier before that stage, so
+// that its 8 dependent levels find their twiddles in L1.
+__device__ __forceinline__ void rp_touch(u32 vt0, u32 lane, int LB, const RowTw & tw, u32 Hr, const u32 * xp)
+{
+	const u32 j = lane & 15;
+	if (j < 15)
+	{
+		// line j: level i = 0, 1, 2, 3 has lines 2^i - 1 .. 2^(i+1) - 2
+		const u32 i = 31u - (u32)__clz((int)(j + 1)), t = (u32)LB - 4u + i;
+		const u32 i0 = (Hr << t) + (vt0 << i >> 1) + (((j + 1) - (1u << i)) << 4);   // 16 pairs a line
+		touch(lane < 16 ? tw.w + i0 : tw.wi != nullptr ? tw.wi + i0 : tw.w + (3u * (tw.H << t) - 16u - i0));
+	}
+	if (xp != nullptr && lane < 16) touch(xp + (vt0 << 4) + (lane << 5));
+}
 
 // The row pass of row bx (prime k = bx / HR, row r) of candidate cand, by P
 // threads (tid < P) sharing the padded row buffer sm.  When P exceeds the
@@ -335,6 +365,8 @@ __device__ __forceinline__ void rowpass_body(const RowJob & J, const TConst & c,
 				rp_store_smem<4>(v, sm, vt, T, b);
 			}
 		}
+		const bool ahead = (T >= 32) && J.mode != ROW_FWD_ONLY;
+		if (ahead && tid < T) rp_touch(tid & ~31u, tid & 31, LB, tw, Hr, xp);
 		__syncthreads();
 
 		// ---- last stage (bits 4..1), pointwise, inverse last stage
@@ -343,6 +375,7 @@ __device__ __forceinline__ void rowpass_body(const RowJob & J, const TConst & c,
 		{
 			const u32 vt = tid + rr * NT;
 			if (IDLE && vt >= T) continue;
+			if (ahead && vt + NT < T) rp_touch((vt + NT) & ~31u, tid & 31, LB, tw, Hr, xp);
 			rp_load_smem<4>(v, sm, vt, T, 1);
 			rp_radix<4, false>(v, vt, T, 1, LB, tw, Hr, p, p2);
 			if (J.mode == ROW_FWD_ONLY)
