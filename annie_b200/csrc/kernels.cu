@@ -22,6 +22,7 @@
 #include <utility>
 
 #include "kernels.h"
+#include "carry.cuh"
 
 namespace ab
 {
@@ -453,10 +454,10 @@ __host__ __device__ constexpr u32 col_ctas(u32 RC) { return (RC <= 32) ? 1u : 1u
 #define AB_COL_REGT 1024
 #endif
 constexpr int COL_THREADS = 384;                       // fused kernels: every split in one launch
-template <int LOG_H>
+template <int LOG_H, bool WIDE>
 struct ColCfg
 {
-	static constexpr int NT = ((AB_COL_TPR << LOG_H) < 64) ? 64 : (AB_COL_TPR << LOG_H);
+	static constexpr int NT = WIDE ? 32 << LOG_H : ((AB_COL_TPR << LOG_H) < 64) ? 64 : (AB_COL_TPR << LOG_H);
 	static constexpr int MINB = (AB_COL_REGT / NT < 16) ? AB_COL_REGT / NT : 16;
 };
 
@@ -571,19 +572,19 @@ __device__ __forceinline__ void exact_add(u32 (&x)[AB_NW], __int128 d)
 // the last one absorbs the rest.  x: exact values (three limbs each).  After
 // the first step the carry is below 2^55, so three limbs hold every sum.
 template <bool FULL, int L, int PCK>
-__device__ __forceinline__ void carry_phase2(const Width & w, const u32 (&half)[AB_NW], const Big<L> & f, const u32 (&d)[4][DigitLimbs<PCK>::N],
+__device__ __forceinline__ void carry_phase2(const Width & w, const Big<AB_NW> & half, const Big<L> & f, const u32 (&d)[4][DigitLimbs<PCK>::N],
 	u32 (&x)[4][AB_NW])
 {
 	constexpr int ND = DigitLimbs<PCK>::N;
 	u32 hd[ND];
 #pragma unroll
-	for (int i = 0; i < ND; ++i) hd[i] = half[i];
+	for (int i = 0; i < ND; ++i) hd[i] = half.l[i];
 	Big<AB_NW> g;
 	auto balanced = [&](const u32 (&e)[ND], u32 (&v)[AB_NW]) {
-		Big<AB_NW> a, h;
+		Big<AB_NW> a;
 #pragma unroll
-		for (int i = 0; i < AB_NW; ++i) { a.l[i] = (i < ND) ? e[i % ND] : 0u; h.l[i] = half[i]; }
-		a = big_sub<AB_NW>(a, h);
+		for (int i = 0; i < AB_NW; ++i) a.l[i] = (i < ND) ? e[i % ND] : 0u;
+		a = big_sub<AB_NW>(a, half);
 #pragma unroll
 		for (int i = 0; i < AB_NW; ++i) v[i] = a.l[i];
 	};
@@ -619,7 +620,10 @@ __device__ __forceinline__ void carry_phase2(const Width & w, const u32 (&half)[
 // runtime amount), the residues are the CRT coordinates themselves (crt), the
 // exact values go from the carry to their residues in registers, and the first
 // and last butterfly stages read and write global memory directly.
-template <int LOG_H, int K, int PCK>
+//
+// WIDE: a thread per tile word (32 H threads) and the carry by 4 lanes per
+// group (carry.cuh), for launches that do not fill the GPU.
+template <int LOG_H, int K, int PCK, bool WIDE>
 __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 cand, int b, int nb, u32 * sm, int & decision)
 {
 	constexpr int KP = K + 1, L = K;             // transform primes, limbs of the carry
@@ -678,6 +682,12 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 			*reinterpret_cast<uint4 *>(tile + k * PS + row * CW + 4 * u4) =
 				make_uint4(encode_res(c, k, a[0]), encode_res(c, k, a[1]), encode_res(c, k, a[2]), encode_res(c, k, a[3]));
 	};
+	// the same for the thread's own word of a WIDE tile
+	auto encode1 = [&](const u32 (&x)[AB_NW]) {
+		const Pieces a = split30(x[0], x[1], x[2]);
+#pragma unroll
+		for (int k = 0; k < KP; ++k) tile[k * PS + tid] = encode_res(c, k, a);
+	};
 	auto finalize = [&](int row, int u4, const u32 (&x)[4][AB_NW]) {
 		const size_t o = (size_t)row * R + gcol(4 * u4);
 #pragma unroll
@@ -705,6 +715,89 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 
 		const Width w = make_width(wbits);
 		const bool full = (w.ws == ND - 1);
+		const bool adjust = (J.lower != LOWER_NONE);
+		const bool edges = adjust && (b == 0 || b == nb - 1);
+	if constexpr (WIDE)
+	{
+		// a thread per tile word: row tid / 32, column lane
+		const int row = tid >> 5, u4 = lane >> 2;
+		const u32 j = (u32)lane & 3u;
+		const size_t o = (size_t)row * R + gcol(lane);
+		Big<L> f = big_zero<L>();
+		if (lane < WU)
+		{
+			u32 y[KP];
+#pragma unroll
+			for (int k = 0; k < KP; ++k) y[k] = tile[k * PS + tid];
+			u32 sv[AB_NW] = {};
+			if (J.sub != nullptr)
+			{
+#pragma unroll
+				for (int l = 0; l < AB_NW; ++l) sv[l] = J.sub[(size_t)l * n + o];
+			}
+			f = crt<L>(c, y);
+			if (amul != 1u) f = big_mul_u32<L>(f, amul);
+			if (J.sub != nullptr) f = big_sub<L>(f, big_from_exact<L>(sv[0], sv[1], sv[2]));
+		}
+		u32 d[ND], x[AB_NW];
+		if (full) lane_digits<true, L, ND>(f, w, j, d);
+		else lane_digits<false, L, ND>(f, w, j, d);
+		if (lane < WU && j == 3)
+		{
+#pragma unroll
+			for (int l = 0; l < L; ++l) cw[(tid >> 2) * L + l] = f.l[l];
+		}
+		__syncthreads();
+		const bool mine = (lane >= E && lane < WU);
+		const bool top0 = adjust && E == 8 && row == H - 1 && u4 == 1;
+		Big<L> cin = big_zero<L>();
+		if (j == 0 && (mine || top0))
+		{
+			int prow = row, pu4 = u4 - 1;
+			bool neg = false;
+			if (b == 0 && lane == E)
+			{
+				// first group of a row: its predecessor ends the previous row
+				if (E == 0) pu4 = ng - 1;
+				if (row > 0) prow = row - 1;
+				else { prow = H - 1; neg = (J.nega != 0); }
+			}
+#pragma unroll
+			for (int l = 0; l < L; ++l) cin.l[l] = cw[(prow * 8 + pu4) * L + l];
+			if (neg) cin = big_neg<L>(cin);
+		}
+		if (full) lane_balance<true, L, ND>(cin, d, w, half_of(wbits), j, x);
+		else lane_balance<false, L, ND>(cin, d, w, half_of(wbits), j, x);
+		if (edges)
+		{
+			// mod R (+2) / mod Q on the top and bottom coefficients (kernel.cl:1653-1683);
+			// CTA 0 re-derives the last coefficient of the register from its
+			// predecessor columns
+			const bool last = (b == nb - 1) && row == H - 1 && lane == WU - 1;
+			if ((last || (top0 && j == 3)) && reaches_width(x, w)) decision = 1;
+			__syncthreads();
+			if (last && decision) exact_add(x, -((__int128)1 << wbits));
+			if (b == 0 && row == 0 && lane == E)
+			{
+				int dv = 0;
+				if (decision) dv += (J.lower == LOWER_Q) ? -1 : 1;
+				if (J.lower == LOWER_R_ADD2) dv += 2;
+				exact_add(x, (__int128)dv);
+			}
+		}
+		if (mine)
+		{
+#pragma unroll
+			for (int l = 0; l < AB_NW; ++l)
+			{
+				if (J.out_norm) J.out_norm[(size_t)l * n + o] = x[l];
+				if (J.out_snap) J.out_snap[(size_t)l * n + o] = x[l];
+			}
+			if (fwd) encode1(x);
+		}
+	}
+	else
+	{
 		// ---- carry phase 1: per group, exact values (CRT), x a, - sub,
 		// unsigned digits + carry-out
 		for (int idx = tid; idx < H * 8; idx += NT)
@@ -749,9 +842,7 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 		// ---- carry phase 2: add the previous group's carry-out, balanced
 		// values; then the outputs of the group.  Each thread reads and writes
 		// only its own group of the tile.
-		const int hb = wbits - 1;
-		const u32 half[AB_NW] = { (hb >> 5) == 0 ? 1u << (hb & 31) : 0u, (hb >> 5) == 1 ? 1u << (hb & 31) : 0u, (hb >> 5) == 2 ? 1u << (hb & 31) : 0u };
-		const bool adjust = (J.lower != LOWER_NONE);
+		const Big<AB_NW> half = half_of(wbits);
 		for (int idx = tid; idx < H * 8; idx += NT)
 		{
 			const int row = idx >> 3, u4 = idx & 7;
@@ -787,16 +878,7 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 			const bool last = (b == nb - 1) && row == H - 1 && u4 == ng - 1;
 			if (adjust && (first || last || top0))
 			{
-				if (last || top0)
-				{
-					// the last coefficient is 2^W or more
-					Big<AB_NW> t;
-#pragma unroll
-					for (int l = 0; l < AB_NW; ++l) t.l[l] = ex[3][l];
-					u32 e[ND];
-					split_digit<false, AB_NW, ND>(t, w, e);
-					if ((i32)t.l[2] >= 0 && (t.l[0] | t.l[1] | t.l[2]) != 0u) decision = 1;
-				}
+				if ((last || top0) && reaches_width(ex[3], w)) decision = 1;
 				if (!top0)
 				{
 #pragma unroll
@@ -809,7 +891,7 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 		}
 
 		// ---- mod R (+2) / mod Q on the top and bottom coefficients (kernel.cl:1653-1683)
-		if (adjust && (b == 0 || b == nb - 1))
+		if (edges)
 		{
 			__syncthreads();
 			if (tid < 2 && ((tid == 0) ? b == 0 : b == nb - 1))
@@ -835,6 +917,7 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 			}
 		}
 	}
+	}
 	griddep_launch_late();
 
 	// ---- the first LA forward levels of the result in one or two domains: the
@@ -851,6 +934,16 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 		{
 			__syncthreads();
 			const u32 * src = J.transformed ? J.out_norm : J.in;
+			if constexpr (WIDE)
+			{
+				if (own)
+				{
+					const size_t o = (size_t)(tid >> 5) * R + gcol(lane);
+					const u32 x[AB_NW] = { src[o], src[(size_t)n + o], src[2 * (size_t)n + o] };
+					encode1(x);
+				}
+			}
+			else
 			for (int idx = tid; idx < H * 8; idx += NT)
 			{
 				const int row = idx >> 3, u4 = idx & 7;
@@ -866,12 +959,12 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 	}
 }
 
-template <int LOG_H, int K, int PCK>
-__global__ void __launch_bounds__(ColCfg<LOG_H>::NT, ColCfg<LOG_H>::MINB) k_colpass(const ColJobs jobs, const TConst c)
+template <int LOG_H, int K, int PCK, bool WIDE>
+__global__ void __launch_bounds__(ColCfg<LOG_H, WIDE>::NT, ColCfg<LOG_H, WIDE>::MINB) k_colpass(const ColJobs jobs, const TConst c)
 {
 	extern __shared__ __align__(16) u32 sm[];
 	__shared__ int decision;
-	colpass_body<LOG_H, K, PCK>((blockIdx.y == 0) ? jobs.j[0] : jobs.j[1], c, blockIdx.z, (int)blockIdx.x, (int)gridDim.x, sm, decision);
+	colpass_body<LOG_H, K, PCK, WIDE>((blockIdx.y == 0) ? jobs.j[0] : jobs.j[1], c, blockIdx.z, (int)blockIdx.x, (int)gridDim.x, sm, decision);
 }
 
 // ================================================================ mixed-size passes
@@ -933,7 +1026,7 @@ __global__ void __launch_bounds__(AB_FUSED_ROW_THREADS, 4) k_fused_rowpass(const
 }
 
 #define AB_FUSED_COL(LH, KK, PP) \
-	case LH * 8 + KK: colpass_body<LH, KK, PP>(J, cs, f.cand, (int)f.bx, (int)d->nbx[f.ci], sm, decision); break;
+	case LH * 8 + KK: colpass_body<LH, KK, PP, false>(J, cs, f.cand, (int)f.bx, (int)d->nbx[f.ci], sm, decision); break;
 #define AB_FUSED_COL_K(LH) AB_FUSED_COL(LH, 2, 1) AB_FUSED_COL(LH, 3, 2) AB_FUSED_COL(LH, 4, 2) AB_FUSED_COL(LH, 5, 4)
 
 __global__ void __launch_bounds__(COL_THREADS, 2) k_fused_colpass(const FusedColPass * __restrict__ d, const TConst * __restrict__ tcs)
@@ -1192,16 +1285,34 @@ cudaError_t launch_midpass(const Geometry & g, const TConst & c, const RowJobs &
 	}
 }
 
-template <int LOG_H, int K, int PCK>
-static cudaError_t colpass_t(const Geometry & g, const TConst & c, const ColJobs & jobs, int njobs, cudaStream_t s, int ncand)
+template <int LOG_H, int K, int PCK, bool WIDE>
+static cudaError_t colpass_w(const Geometry & g, const TConst & c, const ColJobs & jobs, int njobs, cudaStream_t s, int ncand)
 {
 	const size_t smem = colpass_smem(g, K + 1);
 	static std::atomic<unsigned long long> attr_done{0};
-	const cudaError_t e = allow_dynamic_smem(k_colpass<LOG_H, K, PCK>, smem, attr_done);
+	const cudaError_t e = allow_dynamic_smem(k_colpass<LOG_H, K, PCK, WIDE>, smem, attr_done);
 	if (e != cudaSuccess) return e;
 	if (ncand == 0) return cudaSuccess;      // set-up only (before a stream capture)
 	const dim3 grid(g.NC, (unsigned)njobs, (unsigned)ncand);
-	return launch_pdl(k_colpass<LOG_H, K, PCK>, grid, dim3(ColCfg<LOG_H>::NT), smem, s, jobs, c);
+	return launch_pdl(k_colpass<LOG_H, K, PCK, WIDE>, grid, dim3(ColCfg<LOG_H, WIDE>::NT), smem, s, jobs, c);
+}
+
+#ifndef AB_COL_WIDE_CTAS
+#define AB_COL_WIDE_CTAS 296
+#endif
+template <int LOG_H, int K, int PCK>
+static cudaError_t colpass_t(const Geometry & g, const TConst & c, const ColJobs & jobs, int njobs, cudaStream_t s, int ncand)
+{
+	if constexpr (LOG_H <= 4)
+	{
+		if (ncand == 0)
+		{
+			const cudaError_t e = colpass_w<LOG_H, K, PCK, true>(g, c, jobs, njobs, s, 0);
+			if (e != cudaSuccess) return e;
+		}
+		else if (g.NC * (u32)njobs * (u32)ncand <= AB_COL_WIDE_CTAS) return colpass_w<LOG_H, K, PCK, true>(g, c, jobs, njobs, s, ncand);
+	}
+	return colpass_w<LOG_H, K, PCK, false>(g, c, jobs, njobs, s, ncand);
 }
 
 template <int K, int PCK>
