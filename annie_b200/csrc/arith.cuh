@@ -99,10 +99,23 @@ struct TConst
 	int LA, LB, G;                       // column levels, row levels, mid levels (lengths above 2^20)
 };
 
-// Digit size of one candidate (candidates of a batch share K and the length).
+// N as a sparse polynomial: its nonzero coefficients, when there are at most
+// AB_SPARSE of them (k 2^m + 1 has two or three: 1, and k across one or two
+// coefficients).
+#define AB_SPARSE 3
+struct SparseN
+{
+	u32 nt;                              // 0: N is dense
+	u32 idx[AB_SPARSE];
+	u32 coef[AB_SPARSE][AB_NW];
+};
+
+// Digit size and modulus of one candidate (candidates of a batch share K and
+// the length).
 struct CandConst
 {
 	int lbase;
+	SparseN sp;
 };
 
 // ---------------------------------------------------------------- big ints
@@ -254,6 +267,35 @@ __device__ __forceinline__ Big<L> crt(const TConst & c, const u32 (&y)[L + 1])
 	for (int i = 0; i < L - 1; ++i) V.l[i] = __funnelshift_r((u32)col[i] << 2, (u32)col[i + 1], 2 + 2 * i);
 	V.l[L - 1] = (u32)(col[L - 1] >> (2 * (L - 1)));
 	return V;
+}
+
+// Coefficient e of N(x) m(x) mod x^n + 1, mod 2^(32 L), for a sparse N;
+// get(i, d0, d1, d2) reads the exact value m_i.
+template <int L, typename Get>
+__device__ __forceinline__ Big<L> sparse_product(const SparseN & s, u32 e, u32 n, Get get)
+{
+	Big<L> v = big_zero<L>();
+	const u32 nt = s.nt;
+	for (u32 t = 0; t < nt; ++t)
+	{
+		const u32 i = s.idx[t];
+		u32 d0, d1, d2;
+		get((e - i) & (n - 1), d0, d1, d2);
+		Big<L> m = big_from_exact<L>(d0, d1, d2);
+		if (e < i) m = big_neg<L>(m);
+#pragma unroll
+		for (int j = 0; j < AB_NW && j < L; ++j)
+		{
+			const u32 q = s.coef[t][j];
+			if (q == 0u) continue;           // the same in every thread
+			const Big<L> x = (q == 1u) ? m : big_mul_u32<L>(m, q);
+			Big<L> y;
+#pragma unroll
+			for (int l = 0; l < L; ++l) y.l[l] = (l < j) ? 0u : x.l[(l - j + L) % L];
+			v = big_add<L>(v, y);
+		}
+	}
+	return v;
 }
 
 // The 30-bit pieces of an exact value (three limbs, |v| < 2^91): v = a0 +

@@ -264,6 +264,8 @@ struct ab_transform
 	cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_fork = nullptr, ev_q = nullptr;
 	bool overlap = true;                 // run the Q chain on st2 (off for per-launch profiling)
 	bool split = false;                  // without overlap: still one launch per domain
+	CandConst cand{};                    // digit size and sparse N, as on the device at d_cand
+	const CandConst * d_cand = nullptr;
 	bool resident = false;               // short length: runs of squarings in one launch (resident.cu)
 	ab_params prm{};
 	int KP = 0;                          // transform primes
@@ -519,6 +521,13 @@ struct ab_transform
 		j.in = in; j.transformed = 1; j.wi_in = wc(q, true); j.a = a; j.nega = q ? 1 : 0; j.sub = sub; j.lower = lower;
 		return j;
 	}
+	// carry of m N - sub mod Q for the normal form m and a sparse N
+	ColJob cj_sparse(const u32 * m, const u32 * sub) const
+	{
+		ColJob j; std::memset(&j, 0, sizeof(j));
+		j.in = m; j.transformed = SRC_SPARSE; j.a = 1; j.nega = 1; j.sub = sub; j.lower = LOWER_Q; j.cand = d_cand;
+		return j;
+	}
 	void set_fwd(ColJob & j, u32 * q_out, u32 * r_out) const
 	{
 		j.out_fwd[0] = q_out; j.w_out[0] = q_out ? wc(true, false) : nullptr;
@@ -542,10 +551,22 @@ struct ab_transform
 	void reduce_tail(const u32 * tq, u32 * out, bool want_prefwd, bool join_q = false)
 	{
 		rows(rj(b(AR1), ROW_MUL, false, b(NIR)));
-		ColJob j1 = cj_tr(b(AR1), false, 1, nullptr, LOWER_R_ADD2); set_fwd(j1, b(AQ1), nullptr); cols(j1);
-		rows(rj(b(AQ1), ROW_MUL, true, b(NQ)));
+		ColJob j1 = cj_tr(b(AR1), false, 1, nullptr, LOWER_R_ADD2), j2;
+		if (cand.sp.nt != 0)
+		{
+			// m' N from m' itself: no transform of m', no product of images
+			u32 * const m = (tq == b(TQ)) ? b(TMP) : b(TQ);
+			j1.out_norm = m; cols(j1);
+			j2 = cj_sparse(m, tq);
+		}
+		else
+		{
+			set_fwd(j1, b(AQ1), nullptr); cols(j1);
+			rows(rj(b(AQ1), ROW_MUL, true, b(NQ)));
+			j2 = cj_tr(b(AQ1), true, 1, tq, LOWER_Q);
+		}
 		if (join_q) CK(cudaStreamWaitEvent(st, ev_q, 0));
-		ColJob j2 = cj_tr(b(AQ1), true, 1, tq, LOWER_Q); j2.out_norm = out;
+		j2.out_norm = out;
 		const bool q_chain = overlap || split;   // the Q chain has launches of its own
 		if (want_prefwd) set_fwd(j2, q_chain ? nullptr : b(AQ0), b(AR0));
 		cols(j2);
@@ -602,7 +623,7 @@ struct ab_transform
 	{
 		ResJob j; std::memset(&j, 0, sizeof(j));
 		j.reg = x; j.y = y; j.nir = b(NIR); j.nq = b(NQ); j.wr = wf(false); j.wri = wv(false); j.wq = wf(true);
-		j.steps = steps; j.bits = bits; j.a = a;
+		j.steps = steps; j.bits = bits; j.a = a; j.cand = d_cand;
 		CK(launch_resident(j, tc, st));
 		++launches;
 	}
@@ -780,6 +801,8 @@ struct ab_transform
 		const size_t words = (size_t)AB_NW * n;
 		pp.wN.resize(words); pp.wNinv.resize(words); pp.wOne.resize(words);
 		encode(N, pp.wN.data());
+		cand.lbase = prm.lbase;
+		find_sparse(pp.wN);
 		encode(Ninv, pp.wNinv.data());
 		// MMGW form of 1 is R/2 mod N (transformGPU.h:743-747)
 		mpz_mod(Ninv, R, N);
@@ -787,6 +810,21 @@ struct ab_transform
 		mpz_fdiv_q_2exp(Ninv, Ninv, 1);
 		encode(Ninv, pp.wOne.data());
 		mpz_clears(R, Ninv, nullptr);
+	}
+
+	// N's nonzero coefficients, if there are few
+	void find_sparse(const std::vector<u32> & w)
+	{
+		SparseN & s = cand.sp;
+		s = SparseN{};
+		for (size_t i = 0; i < n; ++i)
+		{
+			if ((w[i] | w[n + i] | w[2 * n + i]) == 0) continue;
+			if (s.nt == AB_SPARSE) { s = SparseN{}; return; }
+			s.idx[s.nt] = (u32)i;
+			for (int l = 0; l < AB_NW; ++l) s.coef[s.nt][l] = w[(size_t)l * n + i];
+			++s.nt;
+		}
 	}
 
 	// device part: forward transforms of N (domain Q) and N^-1 (domain R), and 1
@@ -848,6 +886,9 @@ struct ab_transform
 		CK(cudaMalloc(&dmem, total * 4));
 		CK(cudaMemsetAsync(dmem, 0, total * 4, st));
 		d_flag = dmem;
+		static_assert(sizeof(CandConst) <= 48 * sizeof(u32), "beside the flag word");
+		CK(cudaMemcpyAsync(dmem + 16, &cand, sizeof(cand), cudaMemcpyHostToDevice, st));
+		d_cand = reinterpret_cast<const CandConst *>(dmem + 16);
 		for (int i = 0; i < NBUF; ++i) bufp[i] = dmem + offs[i];
 
 		host.assign((size_t)AB_NW * n, 0);
@@ -897,6 +938,7 @@ struct ab_batch
 	std::vector<ab_transform *> views;
 	cudaGraphExec_t gexec = nullptr;
 	int g_steps = 0;
+	bool g_sparse = false;             // gexec takes every N as sparse
 	uint64_t g_kernels = 0;
 	bool resident = false;             // short length: a chunk is one launch (resident.cu)
 	int zl = 0;                        // slots the graph launches (grid.z): a power of two covering every live slot
@@ -966,8 +1008,15 @@ struct ab_batch
 		j.out_fwd[1] = r_out; j.w_out[1] = r_out ? wc(false, false) : nullptr;
 	}
 
+	// whether the N of every slot that can step is sparse
+	bool all_sparse() const
+	{
+		for (const ab_transform * v : views) if (v != nullptr && !v->failed && v->cand.sp.nt == 0) return false;
+		return true;
+	}
+
 	// squareMMGW (transformGPU.h:556-568) for every slot, `steps` times
-	void record_steps(int steps)
+	void record_steps(int steps, bool sparse = false)
 	{
 		using T = ab_transform;
 		u32 * const aq0 = base[T::AQ0], * const ar0 = base[T::AR0], * const aq1 = base[T::AQ1], * const ar1 = base[T::AR1];
@@ -985,10 +1034,22 @@ struct ab_batch
 			ColJob jr = cj(ar0, true, false, mult, nullptr, LOWER_NONE); set_fwd(jr, nullptr, ar1);
 			cols(jq, &jr);
 			rows(rj(ar1, ROW_MUL, false, base[T::NIR], act));
-			ColJob j1 = cj(ar1, true, false, act, nullptr, LOWER_R_ADD2); set_fwd(j1, aq1, nullptr);
-			cols(j1);
-			rows(rj(aq1, ROW_MUL, true, base[T::NQ], act));
-			ColJob j2 = cj(aq1, true, true, act, base[T::TQ], LOWER_Q);
+			ColJob j1 = cj(ar1, true, false, act, nullptr, LOWER_R_ADD2), j2;
+			if (sparse)
+			{
+				// m' N from m' itself (every slot's N is sparse)
+				j1.out_norm = base[T::TMP];
+				cols(j1);
+				j2 = cj(base[T::TMP], false, true, act, base[T::TQ], LOWER_Q);
+				j2.transformed = SRC_SPARSE; j2.nega = 1;
+			}
+			else
+			{
+				set_fwd(j1, aq1, nullptr);
+				cols(j1);
+				rows(rj(aq1, ROW_MUL, true, base[T::NQ], act));
+				j2 = cj(aq1, true, true, act, base[T::TQ], LOWER_Q);
+			}
 			j2.out_norm = base[T::REG0];
 			set_fwd(j2, aq0, ar0);
 			j2.out_snap = base[T::SNAP]; j2.snap_flag = snap;
@@ -1354,9 +1415,19 @@ int ab_square_mul_noalloc(ab_transform * h, uint32_t * reg, int32_t a)
 		ColJob jr = h->cj_tr(ar0, false, (u32)a, nullptr, LOWER_NONE); h->set_fwd(jr, nullptr, ar1);
 		h->cols(jq, &jr);
 		h->rows(h->rj(ar1, ROW_MUL, false, h->b(T::NIR)));
-		ColJob j1 = h->cj_tr(ar1, false, 1, nullptr, LOWER_R_ADD2); h->set_fwd(j1, aq1, nullptr); h->cols(j1);
-		h->rows(h->rj(aq1, ROW_MUL, true, h->b(T::NQ)));
-		ColJob j2 = h->cj_tr(aq1, true, 1, tq, LOWER_Q); j2.out_norm = x; h->cols(j2);
+		ColJob j1 = h->cj_tr(ar1, false, 1, nullptr, LOWER_R_ADD2), j2;
+		if (h->cand.sp.nt != 0)
+		{
+			j1.out_norm = aq1; h->cols(j1);
+			j2 = h->cj_sparse(aq1, tq);
+		}
+		else
+		{
+			h->set_fwd(j1, aq1, nullptr); h->cols(j1);
+			h->rows(h->rj(aq1, ROW_MUL, true, h->b(T::NQ)));
+			j2 = h->cj_tr(aq1, true, 1, tq, LOWER_Q);
+		}
+		j2.out_norm = x; h->cols(j2);
 		CK(launch_export(h->rc, x, reg, (u32)n, h->st));
 		h->launches += 2;
 	});
@@ -1555,6 +1626,7 @@ void batch_attach(ab_batch * b, ab_transform * v, int slot)
 	v->device = b->device; v->st = b->st; v->overlap = false; v->resident = b->resident;
 	v->KP = b->cls.K + 1;
 	v->d_flag = b->d_flag;
+	v->d_cand = b->d_cand + slot;
 	for (int i = 0; i < ab_transform::NSLOT; ++i) v->bufp[i] = b->base[i] + (size_t)slot * b->slot_words(i);
 	for (int i = ab_transform::NSLOT; i < ab_transform::NBUF; ++i) v->bufp[i] = b->base[i];
 	v->host.assign(b->w_norm, 0);
@@ -1576,7 +1648,7 @@ void batch_install(ab_batch * b, int slot, std::unique_ptr<ab_transform> & vp, c
 	{
 		v->setup_device(pp);
 		CandConst & c = b->h_cand[slot];
-		c.lbase = v->prm.lbase;
+		c = v->cand;
 		CK(cudaMemcpyAsync(b->d_cand + slot, &c, sizeof(CandConst), cudaMemcpyHostToDevice, b->st));
 		CK(cudaStreamSynchronize(b->st));
 	}
@@ -1700,7 +1772,7 @@ int ab_batch_clone(ab_batch * b, int dst, int src)
 		ab_transform * v = new ab_transform();
 		v->view = true;
 		mpz_set(v->N, s->N); mpz_set(v->factor, s->factor);
-		v->prm = s->prm; v->n = s->n; v->geo = s->geo; v->tc = s->tc; v->rc = s->rc; v->failed = s->failed;
+		v->prm = s->prm; v->n = s->n; v->cand = s->cand; v->geo = s->geo; v->tc = s->tc; v->rc = s->rc; v->failed = s->failed;
 		batch_attach(b, v, dst);
 		v->noalloc = s->noalloc;
 		for (int i = 0; i < ab_transform::NSLOT; ++i)
@@ -1774,20 +1846,22 @@ int ab_batch_steps(ab_batch * b, int steps, const uint32_t * mult, const uint8_t
 			for (ab_transform * v : b->views) if (v) v->prefwd = false;
 			return;
 		}
-		if (b->gexec == nullptr || b->g_steps != steps || b->zl != zl)
+		const bool sparse = b->all_sparse();
+		if (b->gexec == nullptr || b->g_steps != steps || b->zl != zl || b->g_sparse != sparse)
 		{
 			if (b->gexec) { cudaGraphExecDestroy(b->gexec); b->gexec = nullptr; }
 			b->zl = zl;
 			cudaGraph_t g = nullptr;
 			b->recorded = 0;
 			CK(cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal));
-			try { b->record_steps(steps); }
+			try { b->record_steps(steps, sparse); }
 			catch (...) { cudaStreamEndCapture(b->st, &g); if (g) cudaGraphDestroy(g); throw; }
 			CK(cudaStreamEndCapture(b->st, &g));
 			const cudaError_t e = cudaGraphInstantiate(&b->gexec, g, 0);
 			cudaGraphDestroy(g);
 			CK(e);
 			b->g_steps = steps;
+			b->g_sparse = sparse;
 			b->g_kernels = b->recorded;
 		}
 		CK(cudaGraphLaunch(b->gexec, b->st));

@@ -622,8 +622,9 @@ __device__ __forceinline__ void carry_phase2(const Width & w, const Big<AB_NW> &
 // and last butterfly stages read and write global memory directly.
 //
 // WIDE: a thread per tile word (32 H threads) and the carry by 4 lanes per
-// group (carry.cuh), for launches that do not fill the GPU.
-template <int LOG_H, int K, int PCK, bool WIDE>
+// group (carry.cuh), for launches that do not fill the GPU.  SPARSE: the source
+// is SRC_SPARSE (both jobs of the launch).
+template <int LOG_H, int K, int PCK, bool WIDE, bool SPARSE>
 __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 cand, int b, int nb, u32 * sm, int & decision)
 {
 	constexpr int KP = K + 1, L = K;             // transform primes, limbs of the carry
@@ -639,7 +640,7 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 	if (amul == 0u) return;                       // inactive batch slot
 	{
 		const size_t on = (size_t)cand * J.stride_norm, ot = (size_t)cand * J.stride_ntt;
-		J.in += J.transformed ? ot : on;
+		J.in += (!SPARSE && J.transformed == SRC_NTT) ? ot : on;
 		if (J.sub) J.sub += on;
 		if (J.out_norm) J.out_norm += on;
 		if (J.out_fwd[0]) J.out_fwd[0] += ot;
@@ -662,7 +663,7 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 	{
 		const int k = idx / H, i = idx % H;
 		if (i == 0) continue;
-		if (J.transformed) twc[idx] = J.wi_in[k * COLTW + i];
+		if (!SPARSE && J.transformed == SRC_NTT) twc[idx] = J.wi_in[k * COLTW + i];
 		if (J.out_fwd[0] != nullptr) twc[KP * H + idx] = J.w_out[0][k * COLTW + i];
 		if (J.out_fwd[1] != nullptr) twc[2 * KP * H + idx] = J.w_out[1][k * COLTW + i];
 	}
@@ -708,10 +709,11 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 		}
 	};
 
-	if (J.transformed)
+	if (SPARSE || J.transformed == SRC_NTT)
 	{
 		// ---- inverse column levels
-		col_inverse<LOG_H, KP>(J.in, n, R, gcol(lane), lane < WU, tile, twc, c);
+		auto get_m = [&](u32 i, u32 & d0, u32 & d1, u32 & d2) { d0 = J.in[i]; d1 = J.in[n + i]; d2 = J.in[2 * (size_t)n + i]; };
+		if constexpr (!SPARSE) col_inverse<LOG_H, KP>(J.in, n, R, gcol(lane), lane < WU, tile, twc, c);
 
 		const Width w = make_width(wbits);
 		const bool full = (w.ws == ND - 1);
@@ -726,16 +728,20 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 		Big<L> f = big_zero<L>();
 		if (lane < WU)
 		{
-			u32 y[KP];
-#pragma unroll
-			for (int k = 0; k < KP; ++k) y[k] = tile[k * PS + tid];
 			u32 sv[AB_NW] = {};
 			if (J.sub != nullptr)
 			{
 #pragma unroll
 				for (int l = 0; l < AB_NW; ++l) sv[l] = J.sub[(size_t)l * n + o];
 			}
-			f = crt<L>(c, y);
+			if constexpr (SPARSE) f = sparse_product<L>(J.cand[cand].sp, (u32)o, n, get_m);
+			else
+			{
+				u32 y[KP];
+#pragma unroll
+				for (int k = 0; k < KP; ++k) y[k] = tile[k * PS + tid];
+				f = crt<L>(c, y);
+			}
 			if (amul != 1u) f = big_mul_u32<L>(f, amul);
 			if (J.sub != nullptr) f = big_sub<L>(f, big_from_exact<L>(sv[0], sv[1], sv[2]));
 		}
@@ -805,6 +811,7 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 			const int row = idx >> 3, u4 = idx & 7;
 			if (u4 >= ng) continue;
 			u32 xv[KP][4];
+			if constexpr (!SPARSE)
 #pragma unroll
 			for (int k = 0; k < KP; ++k)
 			{
@@ -819,10 +826,15 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 #pragma unroll
 				for (int j = 0; j < 4; ++j)
 				{
-					u32 rr[KP];
+					Big<L> V;
+					if constexpr (SPARSE) V = sparse_product<L>(J.cand[cand].sp, (u32)row * R + gcol(4 * u4) + (u32)j, n, get_m);
+					else
+					{
+						u32 rr[KP];
 #pragma unroll
-					for (int k = 0; k < KP; ++k) rr[k] = xv[k][j];
-					Big<L> V = crt<L>(c, rr);
+						for (int k = 0; k < KP; ++k) rr[k] = xv[k][j];
+						V = crt<L>(c, rr);
+					}
 					if (amul != 1u) V = big_mul_u32<L>(V, amul);
 					if (J.sub != nullptr) V = big_sub<L>(V, big_from_exact<L>(sv[j][0], sv[j][1], sv[j][2]));
 					f = (j == 0) ? V : big_add<L>(f, V);
@@ -923,7 +935,8 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 	// ---- the first LA forward levels of the result in one or two domains: the
 	// residues of a transformed source are in the tile; those of a normal-form
 	// source, and of the second domain, come from the normal form in global memory
-	bool in_tile = (J.transformed != 0);
+	const bool carried = SPARSE || (J.transformed == SRC_NTT);
+	bool in_tile = carried;
 	const bool own = (lane >= E && lane < WU);
 #pragma unroll 1
 	for (int dom = 0; dom < 2; ++dom)
@@ -933,7 +946,7 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 		if (!in_tile)
 		{
 			__syncthreads();
-			const u32 * src = J.transformed ? J.out_norm : J.in;
+			const u32 * src = carried ? J.out_norm : J.in;
 			if constexpr (WIDE)
 			{
 				if (own)
@@ -959,12 +972,12 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 	}
 }
 
-template <int LOG_H, int K, int PCK, bool WIDE>
+template <int LOG_H, int K, int PCK, bool WIDE, bool SPARSE>
 __global__ void __launch_bounds__(ColCfg<LOG_H, WIDE>::NT, ColCfg<LOG_H, WIDE>::MINB) k_colpass(const ColJobs jobs, const TConst c)
 {
 	extern __shared__ __align__(16) u32 sm[];
 	__shared__ int decision;
-	colpass_body<LOG_H, K, PCK, WIDE>((blockIdx.y == 0) ? jobs.j[0] : jobs.j[1], c, blockIdx.z, (int)blockIdx.x, (int)gridDim.x, sm, decision);
+	colpass_body<LOG_H, K, PCK, WIDE, SPARSE>((blockIdx.y == 0) ? jobs.j[0] : jobs.j[1], c, blockIdx.z, (int)blockIdx.x, (int)gridDim.x, sm, decision);
 }
 
 // ================================================================ mixed-size passes
@@ -1026,7 +1039,7 @@ __global__ void __launch_bounds__(AB_FUSED_ROW_THREADS, 4) k_fused_rowpass(const
 }
 
 #define AB_FUSED_COL(LH, KK, PP) \
-	case LH * 8 + KK: colpass_body<LH, KK, PP, false>(J, cs, f.cand, (int)f.bx, (int)d->nbx[f.ci], sm, decision); break;
+	case LH * 8 + KK: colpass_body<LH, KK, PP, false, false>(J, cs, f.cand, (int)f.bx, (int)d->nbx[f.ci], sm, decision); break;
 #define AB_FUSED_COL_K(LH) AB_FUSED_COL(LH, 2, 1) AB_FUSED_COL(LH, 3, 2) AB_FUSED_COL(LH, 4, 2) AB_FUSED_COL(LH, 5, 4)
 
 __global__ void __launch_bounds__(COL_THREADS, 2) k_fused_colpass(const FusedColPass * __restrict__ d, const TConst * __restrict__ tcs)
@@ -1285,18 +1298,35 @@ cudaError_t launch_midpass(const Geometry & g, const TConst & c, const RowJobs &
 	}
 }
 
-template <int LOG_H, int K, int PCK, bool WIDE>
+template <int LOG_H, int K, int PCK, bool WIDE, bool SPARSE>
 static cudaError_t colpass_w(const Geometry & g, const TConst & c, const ColJobs & jobs, int njobs, cudaStream_t s, int ncand)
 {
 	const size_t smem = colpass_smem(g, K + 1);
 	static std::atomic<unsigned long long> attr_done{0};
-	const cudaError_t e = allow_dynamic_smem(k_colpass<LOG_H, K, PCK, WIDE>, smem, attr_done);
+	const cudaError_t e = allow_dynamic_smem(k_colpass<LOG_H, K, PCK, WIDE, SPARSE>, smem, attr_done);
 	if (e != cudaSuccess) return e;
 	if (ncand == 0) return cudaSuccess;      // set-up only (before a stream capture)
 	const dim3 grid(g.NC, (unsigned)njobs, (unsigned)ncand);
-	return launch_pdl(k_colpass<LOG_H, K, PCK, WIDE>, grid, dim3(ColCfg<LOG_H, WIDE>::NT), smem, s, jobs, c);
+	return launch_pdl(k_colpass<LOG_H, K, PCK, WIDE, SPARSE>, grid, dim3(ColCfg<LOG_H, WIDE>::NT), smem, s, jobs, c);
 }
 
+template <int LOG_H, int K, int PCK, bool WIDE>
+static cudaError_t colpass_s(const Geometry & g, const TConst & c, const ColJobs & jobs, int njobs, cudaStream_t s, int ncand)
+{
+	if (ncand == 0)
+	{
+		const cudaError_t e = colpass_w<LOG_H, K, PCK, WIDE, true>(g, c, jobs, njobs, s, 0);
+		return (e != cudaSuccess) ? e : colpass_w<LOG_H, K, PCK, WIDE, false>(g, c, jobs, njobs, s, 0);
+	}
+	return (jobs.j[0].transformed == SRC_SPARSE) ? colpass_w<LOG_H, K, PCK, WIDE, true>(g, c, jobs, njobs, s, ncand)
+	                                             : colpass_w<LOG_H, K, PCK, WIDE, false>(g, c, jobs, njobs, s, ncand);
+}
+
+// A thread per tile word (WIDE) up to 16 rows and AB_COL_WIDE_CTAS CTAs: where
+// the launch leaves SMs idle, the shorter chains win (us per squaring, grouped /
+// wide: 524k bits 28.6 / 23.1, 2M bits 34.2 / 31.1, 4M bits 41.7 / 38.4); with
+// 32 rows a CTA has 1,024 threads and costs more to start than it saves (6.6M
+// bits, 147 CTAs: 52.1 / 60.7).
 #ifndef AB_COL_WIDE_CTAS
 #define AB_COL_WIDE_CTAS 296
 #endif
@@ -1307,12 +1337,12 @@ static cudaError_t colpass_t(const Geometry & g, const TConst & c, const ColJobs
 	{
 		if (ncand == 0)
 		{
-			const cudaError_t e = colpass_w<LOG_H, K, PCK, true>(g, c, jobs, njobs, s, 0);
+			const cudaError_t e = colpass_s<LOG_H, K, PCK, true>(g, c, jobs, njobs, s, 0);
 			if (e != cudaSuccess) return e;
 		}
-		else if (g.NC * (u32)njobs * (u32)ncand <= AB_COL_WIDE_CTAS) return colpass_w<LOG_H, K, PCK, true>(g, c, jobs, njobs, s, ncand);
+		else if (g.NC * (u32)njobs * (u32)ncand <= AB_COL_WIDE_CTAS) return colpass_s<LOG_H, K, PCK, true>(g, c, jobs, njobs, s, ncand);
 	}
-	return colpass_w<LOG_H, K, PCK, false>(g, c, jobs, njobs, s, ncand);
+	return colpass_s<LOG_H, K, PCK, false>(g, c, jobs, njobs, s, ncand);
 }
 
 template <int K, int PCK>

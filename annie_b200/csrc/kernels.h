@@ -47,12 +47,15 @@ struct RowJob
 };
 struct RowJobs { RowJob j[2]; };
 
+enum ColSource { SRC_NORM = 0, SRC_NTT = 1, SRC_SPARSE = 2 };
+
 enum LowerMode { LOWER_NONE = 0, LOWER_R_ADD2 = 1, LOWER_Q = 2 };
 
 struct ColJob
 {
 	const u32 * in;      // source buffer
-	int transformed;     // 1: NTT-form source awaiting the inverse column levels + carry; 0: normal form
+	int transformed;     // SRC_NTT: NTT-form source awaiting the inverse column levels + carry; SRC_NORM: normal form;
+	                     // SRC_SPARSE: normal form m, carry of N m mod x^n + 1 for the candidate's sparse N
 	const uint2 * wi_in; // column table -w^-1 of the source domain (transformed source), COLTW pairs per prime
 	u32 a;               // carry: multiply by a
 	int nega;            // carry: wrap-around negated (mod x^n + 1)
@@ -64,7 +67,7 @@ struct ColJob
 	size_t stride_ntt;   // words between candidates of NTT-form buffers (in when transformed, out_fwd)
 	size_t stride_norm;  // words between candidates of normal-form buffers (in when not, sub, out_norm, out_snap)
 	const u32 * mult;    // per candidate: the carry multiplier a, 0 = inactive (nullable: use `a`)
-	const CandConst * cand;  // per-candidate digit size (nullable: that of TConst)
+	const CandConst * cand;  // per-candidate digit size and sparse N (nullable: the digit size of TConst)
 	u32 * out_snap;      // per candidate: also store the normal form here when snap_flag[z] != 0
 	const u32 * snap_flag;
 };
@@ -149,7 +152,7 @@ struct ResJob
 	u32 * out_snap;
 	size_t ctrl_stride;
 	size_t stride_norm, stride_ntt;  // words between candidates (reg, y, out_snap; nir, nq)
-	const CandConst * cand;    // per-candidate digit size (nullable)
+	const CandConst * cand;    // per candidate: digit size, and N when it is sparse
 };
 // Whether the class and length of c have a resident kernel that fits the
 // current device.

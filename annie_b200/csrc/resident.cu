@@ -75,10 +75,10 @@ struct ResCfg
 	static constexpr u32 NT0 = (N / 8 > NC) ? N / 8 : NC;
 	static constexpr u32 NT = (BOTH && 2 * NC > NT0) ? 2 * NC : (NT0 < 64) ? 64 : (NT0 + 31) / 32 * 32;
 	// shared memory, words: two work buffers, two operand images, twiddles (two
-	// tables of N/2 pairs), T_Q, carries of both domains
+	// tables of N/2 pairs), T_Q, m' (sparse N), carries of both domains
 	static constexpr u32 W = rpad(N);
 	static constexpr u32 TQ = Q * 4 * AB_NW, CWN = (Q + 2) * K;
-	static constexpr size_t SMEM = sizeof(u32) * (2 * W + 2 * N + 2 * N + TQ + 2 * CWN);
+	static constexpr size_t SMEM = sizeof(u32) * (2 * W + 2 * N + 2 * N + 2 * TQ + 2 * CWN);
 	// CTAs per SM that the kernel is compiled for
 	static constexpr u32 BY_T = AB_RES_REGT / NT, BY_S = (u32)((size_t)227 * 1024 / (SMEM + 1024));
 	static constexpr u32 MINB = (BY_T < BY_S ? BY_T : BY_S) < 1 ? 1 : (BY_T < BY_S ? BY_T : BY_S);
@@ -100,11 +100,12 @@ __device__ __forceinline__ void res_transform(const u32 * xb, u32 * xa, u32 * op
 // The carry of one product, a lane per coefficient and 4 lanes per group
 // (t: thread of the domain, below NC): the group's predecessor groups come
 // first (two in CTA 0, which re-derives the register's last coefficient for
-// the mod R / mod Q decision; one in the others).  Returns the coefficient's
+// the mod R / mod Q decision; one in the others).  With mq, the product is
+// that of the sparse N with the exact values there, else the residues in xa.  Returns the coefficient's
 // exact value in x, and whether the lane owns it.
 template <int LN, int K, int PCK, bool FULL>
 __device__ __forceinline__ bool res_carry(const TConst & c, u32 rank, u32 t, u32 src, bool nega, u32 amul, const u32 * tq, int lower,
-	const Width & w, int wbits, const u32 * xa, u32 * cw, int * decision, u32 (&x)[AB_NW], u32 & e)
+	const Width & w, int wbits, const u32 * xa, const SparseN * sp, const u32 * mq, u32 * cw, int * decision, u32 (&x)[AB_NW], u32 & e)
 {
 	using Cfg = ResCfg<LN, K>;
 	constexpr int KP = Cfg::KP, L = K, ND = DigitLimbs<PCK>::N;
@@ -119,19 +120,24 @@ __device__ __forceinline__ bool res_carry(const TConst & c, u32 rank, u32 t, u32
 	Big<L> f = big_zero<L>();
 	if (active)
 	{
-		u32 y[KP];
-		const u32 o = (u32)sizeof(u32) * rpad(e);
-#pragma unroll
-		for (int k = 0; k < KP; ++k) y[k] = ld_remote(remote(xa, src + k) + o);
-		u32 s[AB_NW];
-		if (tq != nullptr)
+		// an exact value of every CTA's range: planes of 4 Q words
+		auto get = [&](const u32 * planes, u32 i, u32 & d0, u32 & d1, u32 & d2) {
+			const u32 own = (i >> 2) / Q, a = remote(planes, own) + (u32)sizeof(u32) * (i - own * 4 * Q);
+			d0 = ld_remote(a);
+			d1 = ld_remote(a + (u32)sizeof(u32) * 4 * Q);
+			d2 = ld_remote(a + 2 * (u32)sizeof(u32) * 4 * Q);
+		};
+		u32 y[KP] = {};
+		if (mq == nullptr)
 		{
-			const u32 own = g / Q;
-			const u32 a = remote(tq, own) + (u32)sizeof(u32) * (4 * (g - own * Q) + j);
+			const u32 o = (u32)sizeof(u32) * rpad(e);
 #pragma unroll
-			for (int l = 0; l < AB_NW; ++l) s[l] = ld_remote(a + l * (u32)sizeof(u32) * 4 * Q);
+			for (int k = 0; k < KP; ++k) y[k] = ld_remote(remote(xa, src + k) + o);
 		}
-		f = crt<L>(c, y);
+		u32 s[AB_NW];
+		if (tq != nullptr) get(tq, e, s[0], s[1], s[2]);
+		if (mq != nullptr) f = sparse_product<L>(*sp, e, N, [&](u32 i, u32 & d0, u32 & d1, u32 & d2) { get(mq, i, d0, d1, d2); });
+		else f = crt<L>(c, y);
 		if (amul != 1u) f = big_mul_u32<L>(f, amul);
 		if (tq != nullptr) f = big_sub<L>(f, big_from_exact<L>(s[0], s[1], s[2]));
 	}
@@ -201,7 +207,8 @@ __global__ void __launch_bounds__(ResCfg<LN, K>::NT, ResCfg<LN, K>::MINB) k_resi
 	uint2 * const w = reinterpret_cast<uint2 *>(op2 + N);
 	uint2 * const wi = w + N / 2;
 	u32 * const tq = reinterpret_cast<u32 *>(wi + N / 2);   // T_Q of this CTA's coefficients, three planes of 4 Q words
-	u32 * const cwr = tq + Cfg::TQ, * const cwq = cwr + Cfg::CWN;
+	u32 * const mq = tq + Cfg::TQ;                          // m' likewise, when N is sparse
+	u32 * const cwr = mq + Cfg::TQ, * const cwq = cwr + Cfg::CWN;
 
 	const u32 rank = cluster_rank(), cand = blockIdx.y;
 	const u32 dom = rank / KP, k = rank - dom * KP;
@@ -246,12 +253,16 @@ __global__ void __launch_bounds__(ResCfg<LN, K>::NT, ResCfg<LN, K>::MINB) k_resi
 	encode_all(reg);
 	__syncthreads();
 
-	const int wbits = PCK * ((J.cand != nullptr) ? J.cand[cand].lbase : c.lbase);
+	__shared__ SparseN sp;
+	if (tid == 0) sp = J.cand[cand].sp;
+	__syncthreads();
+	const bool sparse = (sp.nt != 0u);
+	const int wbits = PCK * J.cand[cand].lbase;
 	const Width wd = make_width(wbits);
 	const bool full = (wd.ws == DigitLimbs<PCK>::N - 1);
-	auto carry = [&](u32 t, u32 src, bool nega, u32 amul, const u32 * sub, int lower, u32 * cw, u32 (&x)[AB_NW], u32 & e) {
-		return full ? res_carry<LN, K, PCK, true>(c, rank, t, src, nega, amul, sub, lower, wd, wbits, xa, cw, &decision, x, e)
-		            : res_carry<LN, K, PCK, false>(c, rank, t, src, nega, amul, sub, lower, wd, wbits, xa, cw, &decision, x, e);
+	auto carry = [&](u32 t, u32 src, bool nega, u32 amul, const u32 * sub, int lower, const u32 * m, u32 * cw, u32 (&x)[AB_NW], u32 & e) {
+		return full ? res_carry<LN, K, PCK, true>(c, rank, t, src, nega, amul, sub, lower, wd, wbits, xa, &sp, m, cw, &decision, x, e)
+		            : res_carry<LN, K, PCK, false>(c, rank, t, src, nega, amul, sub, lower, wd, wbits, xa, &sp, m, cw, &decision, x, e);
 	};
 	// residues of a coefficient into the CTAs of domain d
 	auto scatter = [&](const u32 (&x)[AB_NW], u32 e, bool r_dom, bool q_dom) {
@@ -265,10 +276,10 @@ __global__ void __launch_bounds__(ResCfg<LN, K>::NT, ResCfg<LN, K>::MINB) k_resi
 			if (q_dom) st_remote(remote(xb, (u32)(KP + q)) + o, v);
 		}
 	};
-	auto keep_tq = [&](const u32 (&x)[AB_NW], u32 e) {
+	auto keep = [&](u32 * planes, const u32 (&x)[AB_NW], u32 e) {
 		const u32 i = e - 4 * rank * Cfg::Q;
 #pragma unroll
-		for (int l = 0; l < AB_NW; ++l) tq[l * 4 * Cfg::Q + i] = x[l];
+		for (int l = 0; l < AB_NW; ++l) planes[l * 4 * Cfg::Q + i] = x[l];
 	};
 
 #pragma unroll 1
@@ -285,26 +296,33 @@ __global__ void __launch_bounds__(ResCfg<LN, K>::NT, ResCfg<LN, K>::MINB) k_resi
 			// the second half of the threads takes domain Q
 			const bool q = tid >= NC && tid < 2 * NC;
 			const u32 t = q ? tid - NC : tid;
-			const bool mine = carry((tid < 2 * NC) ? t : 4u * N, q ? (u32)KP : 0u, q, amul, nullptr, LOWER_NONE, q ? cwq : cwr, x, e);
-			if (mine && q) keep_tq(x, e);
+			const bool mine = carry((tid < 2 * NC) ? t : 4u * N, q ? (u32)KP : 0u, q, amul, nullptr, LOWER_NONE, nullptr, q ? cwq : cwr, x, e);
+			if (mine && q) keep(tq, x, e);
 			else if (mine) scatter(x, e, true, false);
 		}
 		else
 		{
-			if (carry(tid, 0u, false, amul, nullptr, LOWER_NONE, cwr, x, e)) scatter(x, e, true, false);
-			if (carry(tid, (u32)KP, true, amul, nullptr, LOWER_NONE, cwq, x, e)) keep_tq(x, e);
+			if (carry(tid, 0u, false, amul, nullptr, LOWER_NONE, nullptr, cwr, x, e)) scatter(x, e, true, false);
+			if (carry(tid, (u32)KP, true, amul, nullptr, LOWER_NONE, nullptr, cwq, x, e)) keep(tq, x, e);
 		}
 		cluster_sync();
 		// m' = T_R N^-1 mod R, + 2
 		if (dom == 0) res_transform<LN>(xb, xa, op, BOTTOM_MUL, tw, p, pinv);
 		cluster_sync();
-		if (carry(tid, 0u, false, 1u, nullptr, LOWER_R_ADD2, cwr, x, e)) scatter(x, e, false, true);
+		if (carry(tid, 0u, false, 1u, nullptr, LOWER_R_ADD2, nullptr, cwr, x, e))
+		{
+			if (sparse) keep(mq, x, e);
+			else scatter(x, e, false, true);
+		}
 		cluster_sync();
-		// m' N - T_Q mod Q
-		if (dom == 1) res_transform<LN>(xb, xa, op, BOTTOM_MUL, tw, p, pinv);
-		cluster_sync();
+		// m' N - T_Q mod Q: a sparse N needs no transform
+		if (!sparse)
+		{
+			if (dom == 1) res_transform<LN>(xb, xa, op, BOTTOM_MUL, tw, p, pinv);
+			cluster_sync();
+		}
 		const bool snap = (J.snap != nullptr) && J.snap[(size_t)s * J.ctrl_stride + cand] != 0u;
-		if (carry(tid, (u32)KP, true, 1u, tq, LOWER_Q, cwr, x, e))
+		if (carry(tid, (u32)KP, true, 1u, tq, LOWER_Q, sparse ? mq : nullptr, cwr, x, e))
 		{
 			scatter(x, e, true, true);
 #pragma unroll
