@@ -23,46 +23,10 @@
 
 #include "kernels.h"
 #include "carry.cuh"
+#include "pdl.cuh"
 
 namespace ab
 {
-
-// Programmatic dependent launch: the row, mid and column passes are launched
-// so that the next pass on the stream may be scheduled while the current one
-// is still running.  Until griddep_wait() a pass reads only what no earlier
-// pass of the stream writes (twiddles, its launch parameters, the per-slot
-// control words uploaded before a graph launch) and writes only shared
-// memory; griddep_wait() returns once the previous kernel of the stream has
-// completed and its writes are visible.  The next pass is scheduled as the
-// CTAs of the current one exit (AB_PDL_TRIGGER 0).  An explicit trigger right
-// after griddep_wait (1) or before the final stores (2) lets the next pass
-// hold SM resources while this one still runs; both measured slower on B200
-// (33.2 M bits: 221.7 and 233.3 us per squaring against 210.1; without PDL
-// 218.9).
-#ifndef AB_PDL
-#define AB_PDL 1
-#endif
-#ifndef AB_PDL_TRIGGER
-#define AB_PDL_TRIGGER 0
-#endif
-__device__ __forceinline__ void griddep_wait()
-{
-#if AB_PDL
-	asm volatile("griddepcontrol.wait;" ::: "memory");
-#endif
-}
-__device__ __forceinline__ void griddep_launch()
-{
-#if AB_PDL && AB_PDL_TRIGGER == 1
-	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-#endif
-}
-__device__ __forceinline__ void griddep_launch_late()
-{
-#if AB_PDL && AB_PDL_TRIGGER == 2
-	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-#endif
-}
 
 // ================================================================ row pass
 // A CTA transforms one row (R = 2^(LB+1) words) of one prime: levels
@@ -317,7 +281,6 @@ __device__ __forceinline__ void rowpass_body(const RowJob & J, const TConst & c,
 	// twiddles of the last forward level of virtual thread vt: the c of its polynomials
 	auto w1 = [&](u32 vt) { return tw.w + (Hr << (LB - 1)) + ((vt >> 1) << 3); };
 	griddep_wait();
-	griddep_launch();
 
 	if constexpr (NS == 0)
 	{
@@ -409,7 +372,6 @@ __device__ __forceinline__ void rowpass_body(const RowJob & J, const TConst & c,
 			}
 		}
 		__syncthreads();
-		griddep_launch_late();
 #pragma unroll 1
 		for (u32 rr = 0; rr < RND; ++rr)
 		{
@@ -670,7 +632,6 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 	if (tid == 0) decision = 0;
 	__syncthreads();
 	griddep_wait();
-	griddep_launch();
 
 	// a group's exact values: normal form out, residues into the tile
 	const bool fwd = (J.out_fwd[0] != nullptr) || (J.out_fwd[1] != nullptr);
@@ -930,7 +891,6 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 		}
 	}
 	}
-	griddep_launch_late();
 
 	// ---- the first LA forward levels of the result in one or two domains: the
 	// residues of a transformed source are in the tile; those of a normal-form
@@ -1160,7 +1120,6 @@ __global__ void __launch_bounds__(256) k_midpass(const RowJobs jobs, const TCons
 	const uint2 * __restrict__ w = J.w + (size_t)k * (c.n >> 1);
 	const uint2 * __restrict__ wi = (J.wi != nullptr) ? J.wi + (size_t)k * (c.n >> 1) : nullptr;
 	griddep_wait();
-	griddep_launch();
 	u32 v[M];
 #pragma unroll
 	for (int m = 0; m < M; ++m) v[m] = x[(size_t)m * R];
@@ -1241,7 +1200,7 @@ static cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t 
 	cfg.stream = s;
 	cudaLaunchAttribute attr[1];
 	attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-	attr[0].val.programmaticStreamSerializationAllowed = AB_PDL;
+	attr[0].val.programmaticStreamSerializationAllowed = 1;
 	cfg.attrs = attr;
 	cfg.numAttrs = 1;
 	return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);

@@ -138,7 +138,7 @@ cudaError_t launch_fused_colpass(const FusedColPass * d, const TConst * tcs, u32
 struct ResJob
 {
 	u32 * reg;                 // normal-form register, replaced by the result of the last step
-	const u32 * y;             // nullable: the steps multiply by this normal-form register instead of squaring
+	const u32 * y;             // nullable: the (one) step multiplies by this normal-form register instead of squaring
 	const u32 * nir, * nq;     // transforms of N^-1 (domain R) and N (domain Q)
 	const uint2 * wr, * wri, * wq;   // row tables
 	int steps;

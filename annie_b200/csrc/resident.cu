@@ -21,6 +21,7 @@
 #include "kernels.h"
 #include "carry.cuh"
 #include "levels.cuh"
+#include "pdl.cuh"
 
 namespace ab
 {
@@ -68,17 +69,20 @@ struct ResCfg
 {
 	static constexpr int KP = K + 1, C = 2 * KP;               // CTAs of a cluster
 	static constexpr u32 N = 1u << LN, G = N / 4;              // words, groups of 4 coefficients
-	static constexpr u32 Q = (G + C - 1) / C;                  // groups of a CTA in the carry steps
-	// threads of one domain's carry: a lane per coefficient, two predecessor groups
+	// groups of a CTA in the carry steps: of a Q CTA where those carry T_Q alone
+	static constexpr u32 Q = (G + C - 1) / C, Q2 = (G + KP - 1) / KP;
+	// threads: 8 words each in a transform step; in a carry step a lane per
+	// coefficient, with up to two predecessor groups
 	static constexpr u32 NC = ((Q + 2) * 4 + 31) / 32 * 32;
-	static constexpr bool BOTH = 2 * NC <= 512;                // both domains of the first product at once
-	static constexpr u32 NT0 = (N / 8 > NC) ? N / 8 : NC;
-	static constexpr u32 NT = (BOTH && 2 * NC > NT0) ? 2 * NC : (NT0 < 64) ? 64 : (NT0 + 31) / 32 * 32;
-	// shared memory, words: two work buffers, two operand images, twiddles (two
-	// tables of N/2 pairs), T_Q, m' (sparse N), carries of both domains
+	static constexpr u32 NT0 = (N / 8 > NC) ? N / 8 : NC, NT = (NT0 < 64) ? 64 : (NT0 + 31) / 32 * 32;
+	static constexpr u32 CH = NT / 4 - 1;                      // groups of T_Q carried at a time
+	// shared memory, words: two work buffers; the operand's image; the second
+	// factor's, or m' of a sparse N; the twiddles; the inverse twiddles (R), or
+	// T_Q (Q); carries
 	static constexpr u32 W = rpad(N);
-	static constexpr u32 TQ = Q * 4 * AB_NW, CWN = (Q + 2) * K;
-	static constexpr size_t SMEM = sizeof(u32) * (2 * W + 2 * N + 2 * N + 2 * TQ + 2 * CWN);
+	static constexpr u32 TQ = Q2 * 4 * AB_NW, MQ = Q * 4 * AB_NW, CWN = NT / 4 * K;
+	static constexpr size_t SMEM = sizeof(u32) * (2 * W + 3 * N + (N > TQ ? N : TQ) + CWN);
+	static_assert(MQ <= N, "m' in the second factor's place");
 	// CTAs per SM that the kernel is compiled for
 	static constexpr u32 BY_T = AB_RES_REGT / NT, BY_S = (u32)((size_t)227 * 1024 / (SMEM + 1024));
 	static constexpr u32 MINB = (BY_T < BY_S ? BY_T : BY_S) < 1 ? 1 : (BY_T < BY_S ? BY_T : BY_S);
@@ -97,36 +101,44 @@ __device__ __forceinline__ void res_transform(const u32 * xb, u32 * xa, u32 * op
 		[&](u32 o, uint4 a, uint4 b) { q[o] = a; q[N8 + o] = b; });
 }
 
-// The carry of one product, a lane per coefficient and 4 lanes per group
-// (t: thread of the domain, below NC): the group's predecessor groups come
-// first (two in CTA 0, which re-derives the register's last coefficient for
-// the mod R / mod Q decision; one in the others).  With mq, the product is
-// that of the sparse N with the exact values there, else the residues in xa.  Returns the coefficient's
-// exact value in x, and whether the lane owns it.
+// Groups g0 .. g0 + cnt - 1 of a carry step, and the E predecessor groups that
+// give the carry into them (the groups before 0 end the register).
+struct CarryRange
+{
+	u32 g0, cnt, E;
+};
+
+// An exact value that the CTAs from `first` on keep, QQ groups each, as three
+// planes of 4 QQ words.
+template <u32 QQ>
+__device__ __forceinline__ void get_exact(const u32 * planes, u32 first, u32 i, u32 & d0, u32 & d1, u32 & d2)
+{
+	const u32 own = (i >> 2) / QQ, a = remote(planes, first + own) + (u32)sizeof(u32) * (i - own * 4 * QQ);
+	d0 = ld_remote(a);
+	d1 = ld_remote(a + (u32)sizeof(u32) * 4 * QQ);
+	d2 = ld_remote(a + 2 * (u32)sizeof(u32) * 4 * QQ);
+}
+
+// The carry of one product over a range, a lane per coefficient and 4 lanes per
+// group, the predecessor groups first (CTA 0 has two when it re-derives the
+// register's last coefficient for the mod R / mod Q decision).  The product's
+// residues are in xa of the CTAs from src on; with mq, it is that of the sparse
+// N with the exact values there.  tq: subtract T_Q.  Returns the coefficient's
+// exact value in x and whether the lane owns it.
 template <int LN, int K, int PCK, bool FULL>
-__device__ __forceinline__ bool res_carry(const TConst & c, u32 rank, u32 t, u32 src, bool nega, u32 amul, const u32 * tq, int lower,
+__device__ __forceinline__ bool res_carry(const TConst & c, const CarryRange & rg, u32 src, bool nega, u32 amul, const u32 * tq, int lower,
 	const Width & w, int wbits, const u32 * xa, const SparseN * sp, const u32 * mq, u32 * cw, int * decision, u32 (&x)[AB_NW], u32 & e)
 {
 	using Cfg = ResCfg<LN, K>;
 	constexpr int KP = Cfg::KP, L = K, ND = DigitLimbs<PCK>::N;
-	constexpr u32 G = Cfg::G, Q = Cfg::Q, N = Cfg::N;
-	const u32 g0 = rank * Q, cnt = (g0 >= G) ? 0u : (G - g0 < Q) ? G - g0 : Q;
-	const u32 E = (cnt == 0) ? 0u : (rank == 0) ? 2u : 1u;
-	const u32 li = t >> 2, j = t & 3;
-	const bool active = li < E + cnt;
-	u32 g = g0 + li - E;                          // group (CTA 0's predecessors end the register)
-	if (rank == 0 && li < E) g += G;
+	constexpr u32 G = Cfg::G, N = Cfg::N;
+	const u32 E = rg.E, li = threadIdx.x >> 2, j = threadIdx.x & 3;
+	const bool active = li < E + rg.cnt;
+	const u32 g = rg.g0 + li - E + ((rg.g0 + li < E) ? G : 0u);
 	e = active ? 4 * g + j : 0u;
 	Big<L> f = big_zero<L>();
 	if (active)
 	{
-		// an exact value of every CTA's range: planes of 4 Q words
-		auto get = [&](const u32 * planes, u32 i, u32 & d0, u32 & d1, u32 & d2) {
-			const u32 own = (i >> 2) / Q, a = remote(planes, own) + (u32)sizeof(u32) * (i - own * 4 * Q);
-			d0 = ld_remote(a);
-			d1 = ld_remote(a + (u32)sizeof(u32) * 4 * Q);
-			d2 = ld_remote(a + 2 * (u32)sizeof(u32) * 4 * Q);
-		};
 		u32 y[KP] = {};
 		if (mq == nullptr)
 		{
@@ -135,8 +147,8 @@ __device__ __forceinline__ bool res_carry(const TConst & c, u32 rank, u32 t, u32
 			for (int k = 0; k < KP; ++k) y[k] = ld_remote(remote(xa, src + k) + o);
 		}
 		u32 s[AB_NW];
-		if (tq != nullptr) get(tq, e, s[0], s[1], s[2]);
-		if (mq != nullptr) f = sparse_product<L>(*sp, e, N, [&](u32 i, u32 & d0, u32 & d1, u32 & d2) { get(mq, i, d0, d1, d2); });
+		if (tq != nullptr) get_exact<Cfg::Q2>(tq, KP, e, s[0], s[1], s[2]);
+		if (mq != nullptr) f = sparse_product<L>(*sp, e, N, [&](u32 i, u32 & d0, u32 & d1, u32 & d2) { get_exact<Cfg::Q>(mq, 0, i, d0, d1, d2); });
 		else f = crt<L>(c, y);
 		if (amul != 1u) f = big_mul_u32<L>(f, amul);
 		if (tq != nullptr) f = big_sub<L>(f, big_from_exact<L>(s[0], s[1], s[2]));
@@ -152,7 +164,7 @@ __device__ __forceinline__ bool res_carry(const TConst & c, u32 rank, u32 t, u32
 	__syncthreads();
 	// phase 2: the previous group's carry-out, balanced digits; the last
 	// coefficient of a group absorbs the rest
-	const bool top0 = (lower != LOWER_NONE) && rank == 0 && li == 1;
+	const bool top0 = (lower != LOWER_NONE) && E == 2 && li == 1;
 	const bool mine = active && li >= E;
 	Big<L> cin = big_zero<L>();
 	if (j == 0 && (mine || top0))
@@ -194,38 +206,29 @@ __device__ __forceinline__ bool res_carry(const TConst & c, u32 rank, u32 t, u32
 	return mine;
 }
 
-template <int LN, int K, int PCK>
-__global__ void __launch_bounds__(ResCfg<LN, K>::NT, ResCfg<LN, K>::MINB) k_resident(const ResJob J, const TConst c)
+// SOLO: a launch of one cluster, which needs no other resident beside it and
+// may use all registers (262k bits: 18.5 us per squaring against 19.5).
+template <int LN, int K, int PCK, bool SOLO>
+__global__ void __launch_bounds__(ResCfg<LN, K>::NT, SOLO ? 1 : ResCfg<LN, K>::MINB) k_resident(const ResJob J, const TConst c)
 {
 	using Cfg = ResCfg<LN, K>;
 	constexpr int KP = Cfg::KP;
-	constexpr u32 N = Cfg::N, W = Cfg::W, NC = Cfg::NC;
+	constexpr u32 N = Cfg::N, W = Cfg::W, G = Cfg::G;
 	extern __shared__ __align__(16) u32 sm[];
 	__shared__ int decision;
 	u32 * const xa = sm, * const xb = xa + W;               // transform step: xb -> xa
-	u32 * const op = xb + W, * const op2 = op + N;          // image of N^-1 / N; of the second factor
+	u32 * const op = xb + W;                                // image of N^-1 (R) or N (Q)
+	u32 * const op2 = op + N;                               // image of the second factor of a product
+	u32 * const mq = op2;                                   // m' of a CTA's range when N is sparse, planes of 4 Q words
 	uint2 * const w = reinterpret_cast<uint2 *>(op2 + N);
-	uint2 * const wi = w + N / 2;
-	u32 * const tq = reinterpret_cast<u32 *>(wi + N / 2);   // T_Q of this CTA's coefficients, three planes of 4 Q words
-	u32 * const mq = tq + Cfg::TQ;                          // m' likewise, when N is sparse
-	u32 * const cwr = mq + Cfg::TQ, * const cwq = cwr + Cfg::CWN;
+	uint2 * const wi = w + N / 2;                           // R CTAs
+	u32 * const tq = reinterpret_cast<u32 *>(wi);           // Q CTAs: T_Q of the CTA's range, planes of 4 Q2 words
+	u32 * const cw = reinterpret_cast<u32 *>(wi) + (N > Cfg::TQ ? N : Cfg::TQ);
 
 	const u32 rank = cluster_rank(), cand = blockIdx.y;
 	const u32 dom = rank / KP, k = rank - dom * KP;
 	const u32 tid = threadIdx.x, NT = Cfg::NT;
 	const u32 p = c.p[k], pinv = c.pinv[k];
-	// the last step that the slot takes part in; an idle slot's cluster leaves
-	__shared__ int last;
-	if (tid == 0) last = (J.mult != nullptr) ? -1 : J.steps - 1;
-	__syncthreads();
-	if (J.mult != nullptr)
-	{
-		for (int s = (int)tid; s < J.steps; s += (int)NT)
-			if (J.mult[(size_t)s * J.ctrl_stride + cand] != 0u) atomicMax(&last, s);
-		__syncthreads();
-		if (last < 0) return;
-	}
-
 	const size_t on = (size_t)cand * J.stride_norm, ot = (size_t)cand * J.stride_ntt;
 	u32 * const reg = J.reg + on;
 	const uint2 * const gw = (dom == 0 ? J.wr : J.wq) + (size_t)k * (N / 2);
@@ -240,6 +243,22 @@ __global__ void __launch_bounds__(ResCfg<LN, K>::NT, ResCfg<LN, K>::MINB) k_resi
 		uint4 * o4 = reinterpret_cast<uint4 *>(op);
 		for (u32 i = tid; i < N / 4; i += NT) o4[(i & 1) * (N / 8) + (i >> 1)] = __ldg(img + i);
 	}
+	__shared__ SparseN sp;
+	if (tid == 0) sp = J.cand[cand].sp;
+	const int wbits = PCK * J.cand[cand].lbase;
+	// above: tables and images, which no earlier work of the stream writes
+	griddep_wait();
+	// the last step that the slot takes part in; an idle slot's cluster leaves
+	__shared__ int last;
+	if (tid == 0) last = (J.mult != nullptr) ? -1 : J.steps - 1;
+	__syncthreads();
+	if (J.mult != nullptr)
+	{
+		for (int s = (int)tid; s < J.steps; s += (int)NT)
+			if (J.mult[(size_t)s * J.ctrl_stride + cand] != 0u) atomicMax(&last, s);
+		__syncthreads();
+		if (last < 0) return;
+	}
 	auto encode_all = [&](const u32 * src) {
 		for (u32 i = tid; i < N; i += NT) xb[rpad(i)] = encode_res(c, (int)k, split30(src[i], src[N + i], src[2 * N + i]));
 	};
@@ -253,17 +272,17 @@ __global__ void __launch_bounds__(ResCfg<LN, K>::NT, ResCfg<LN, K>::MINB) k_resi
 	encode_all(reg);
 	__syncthreads();
 
-	__shared__ SparseN sp;
-	if (tid == 0) sp = J.cand[cand].sp;
-	__syncthreads();
 	const bool sparse = (sp.nt != 0u);
-	const int wbits = PCK * J.cand[cand].lbase;
 	const Width wd = make_width(wbits);
 	const bool full = (wd.ws == DigitLimbs<PCK>::N - 1);
-	auto carry = [&](u32 t, u32 src, bool nega, u32 amul, const u32 * sub, int lower, const u32 * m, u32 * cw, u32 (&x)[AB_NW], u32 & e) {
-		return full ? res_carry<LN, K, PCK, true>(c, rank, t, src, nega, amul, sub, lower, wd, wbits, xa, &sp, m, cw, &decision, x, e)
-		            : res_carry<LN, K, PCK, false>(c, rank, t, src, nega, amul, sub, lower, wd, wbits, xa, &sp, m, cw, &decision, x, e);
+	auto carry = [&](const CarryRange & rg, u32 src, bool nega, u32 amul, const u32 * sub, int lower, const u32 * m, u32 (&x)[AB_NW], u32 & e) {
+		return full ? res_carry<LN, K, PCK, true>(c, rg, src, nega, amul, sub, lower, wd, wbits, xa, &sp, m, cw, &decision, x, e)
+		            : res_carry<LN, K, PCK, false>(c, rg, src, nega, amul, sub, lower, wd, wbits, xa, &sp, m, cw, &decision, x, e);
 	};
+	// the CTA's groups: of all carry steps but that of T_Q, and of T_Q (Q CTAs)
+	const u32 g0 = rank * Cfg::Q, cnt = (g0 >= G) ? 0u : (G - g0 < Cfg::Q) ? G - g0 : Cfg::Q;
+	const CarryRange own{ g0, cnt, (cnt == 0) ? 0u : (rank == 0) ? 2u : 1u };
+	const u32 q0 = (rank - dom * KP) * Cfg::Q2, qn = (q0 >= G) ? 0u : (G - q0 < Cfg::Q2) ? G - q0 : Cfg::Q2;
 	// residues of a coefficient into the CTAs of domain d
 	auto scatter = [&](const u32 (&x)[AB_NW], u32 e, bool r_dom, bool q_dom) {
 		const Pieces a = split30(x[0], x[1], x[2]);
@@ -276,42 +295,43 @@ __global__ void __launch_bounds__(ResCfg<LN, K>::NT, ResCfg<LN, K>::MINB) k_resi
 			if (q_dom) st_remote(remote(xb, (u32)(KP + q)) + o, v);
 		}
 	};
-	auto keep = [&](u32 * planes, const u32 (&x)[AB_NW], u32 e) {
-		const u32 i = e - 4 * rank * Cfg::Q;
-#pragma unroll
-		for (int l = 0; l < AB_NW; ++l) planes[l * 4 * Cfg::Q + i] = x[l];
-	};
-
 #pragma unroll 1
 	for (int s = 0; s < J.steps; ++s)
 	{
 		const u32 amul = (J.mult != nullptr) ? J.mult[(size_t)s * J.ctrl_stride + cand] : ((J.bits >> s) & 1) ? J.a : 1u;
 		if (amul == 0u) continue;                 // the slot rests in this step
+		if (s == last && gridDim.y == 1) griddep_launch();   // the next run may load its tables
 		u32 x[AB_NW], e;
 		// T_R = a x y mod R, T_Q = a x y mod Q
 		res_transform<LN>(xb, xa, op2, (J.y != nullptr) ? BOTTOM_MUL : BOTTOM_SQUARE, tw, p, pinv);
 		cluster_sync();
-		if constexpr (Cfg::BOTH)
-		{
-			// the second half of the threads takes domain Q
-			const bool q = tid >= NC && tid < 2 * NC;
-			const u32 t = q ? tid - NC : tid;
-			const bool mine = carry((tid < 2 * NC) ? t : 4u * N, q ? (u32)KP : 0u, q, amul, nullptr, LOWER_NONE, nullptr, q ? cwq : cwr, x, e);
-			if (mine && q) keep(tq, x, e);
-			else if (mine) scatter(x, e, true, false);
-		}
+		if (carry(own, 0u, false, amul, nullptr, LOWER_NONE, nullptr, x, e)) scatter(x, e, true, false);
+		cluster_sync();
+		// m' = T_R N^-1 mod R, + 2; meanwhile the Q CTAs carry T_Q, which is only
+		// needed at the end
+		if (dom == 0) res_transform<LN>(xb, xa, op, BOTTOM_MUL, tw, p, pinv);
 		else
 		{
-			if (carry(tid, 0u, false, amul, nullptr, LOWER_NONE, nullptr, cwr, x, e)) scatter(x, e, true, false);
-			if (carry(tid, (u32)KP, true, amul, nullptr, LOWER_NONE, nullptr, cwq, x, e)) keep(tq, x, e);
+#pragma unroll 1
+			for (u32 i = 0; i < qn; i += Cfg::CH)
+			{
+				if (i != 0) __syncthreads();
+				const CarryRange rg{ q0 + i, (qn - i < Cfg::CH) ? qn - i : Cfg::CH, 1u };
+				if (carry(rg, (u32)KP, true, amul, nullptr, LOWER_NONE, nullptr, x, e))
+				{
+#pragma unroll
+					for (int l = 0; l < AB_NW; ++l) tq[l * 4 * Cfg::Q2 + e - 4 * q0] = x[l];
+				}
+			}
 		}
 		cluster_sync();
-		// m' = T_R N^-1 mod R, + 2
-		if (dom == 0) res_transform<LN>(xb, xa, op, BOTTOM_MUL, tw, p, pinv);
-		cluster_sync();
-		if (carry(tid, 0u, false, 1u, nullptr, LOWER_R_ADD2, nullptr, cwr, x, e))
+		if (carry(own, 0u, false, 1u, nullptr, LOWER_R_ADD2, nullptr, x, e))
 		{
-			if (sparse) keep(mq, x, e);
+			if (sparse)
+			{
+#pragma unroll
+				for (int l = 0; l < AB_NW; ++l) mq[l * 4 * Cfg::Q + e - 4 * g0] = x[l];
+			}
 			else scatter(x, e, false, true);
 		}
 		cluster_sync();
@@ -322,7 +342,7 @@ __global__ void __launch_bounds__(ResCfg<LN, K>::NT, ResCfg<LN, K>::MINB) k_resi
 			cluster_sync();
 		}
 		const bool snap = (J.snap != nullptr) && J.snap[(size_t)s * J.ctrl_stride + cand] != 0u;
-		if (carry(tid, (u32)KP, true, 1u, tq, LOWER_Q, sparse ? mq : nullptr, cwr, x, e))
+		if (carry(own, (u32)KP, true, 1u, tq, LOWER_Q, sparse ? mq : nullptr, x, e))
 		{
 			scatter(x, e, true, true);
 #pragma unroll
@@ -336,8 +356,8 @@ __global__ void __launch_bounds__(ResCfg<LN, K>::NT, ResCfg<LN, K>::MINB) k_resi
 	}
 }
 
-template <int LN, int K, int PCK>
-cudaError_t resident_t(const ResJob & J, const TConst & c, cudaStream_t s, int ncand, bool * fits)
+template <int LN, int K, int PCK, bool SOLO>
+cudaError_t resident_v(const ResJob & J, const TConst & c, cudaStream_t s, int ncand, bool * fits)
 {
 	using Cfg = ResCfg<LN, K>;
 	static_assert(Cfg::NC <= 1024 && Cfg::NT <= 1024, "a lane per coefficient");
@@ -352,22 +372,26 @@ cudaError_t resident_t(const ResJob & J, const TConst & c, cudaStream_t s, int n
 	cfg.blockDim = dim3(Cfg::NT);
 	cfg.dynamicSmemBytes = Cfg::SMEM;
 	cfg.stream = s;
-	cudaLaunchAttribute attr[1];
+	cudaLaunchAttribute attr[2];
 	attr[0].id = cudaLaunchAttributeClusterDimension;
 	attr[0].val.clusterDim.x = Cfg::C;
 	attr[0].val.clusterDim.y = 1;
 	attr[0].val.clusterDim.z = 1;
+	attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	attr[1].val.programmaticStreamSerializationAllowed = 1;
 	cfg.attrs = attr;
-	cfg.numAttrs = 1;
+	// a run of several clusters starts after the one before: placed among its
+	// last ones, fewer clusters fit (16 x 262k bits: 57 us per step against 32)
+	cfg.numAttrs = (ncand == 1) ? 2 : 1;
 	if (!(done.load(std::memory_order_acquire) & bit))
 	{
-		e = cudaFuncSetAttribute(k_resident<LN, K, PCK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM);
+		e = cudaFuncSetAttribute(k_resident<LN, K, PCK, SOLO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM);
 		if (e != cudaSuccess) return e;
-		if (Cfg::C > 8) e = cudaFuncSetAttribute(k_resident<LN, K, PCK>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+		if (Cfg::C > 8) e = cudaFuncSetAttribute(k_resident<LN, K, PCK, SOLO>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
 		if (e != cudaSuccess) return e;
 		cfg.gridDim = dim3(Cfg::C, 1);
 		int clusters = 0;
-		e = cudaOccupancyMaxActiveClusters(&clusters, k_resident<LN, K, PCK>, &cfg);
+		e = cudaOccupancyMaxActiveClusters(&clusters, k_resident<LN, K, PCK, SOLO>, &cfg);
 		if (e != cudaSuccess) { cudaGetLastError(); clusters = 0; }
 		if (clusters > 0) ok.fetch_or(bit, std::memory_order_acq_rel);
 		done.fetch_or(bit, std::memory_order_acq_rel);
@@ -377,7 +401,23 @@ cudaError_t resident_t(const ResJob & J, const TConst & c, cudaStream_t s, int n
 	if (fits) *fits = can;
 	if (ncand == 0) return cudaSuccess;       // query and set-up only
 	if (!can) return cudaErrorNotSupported;
-	return cudaLaunchKernelEx(&cfg, k_resident<LN, K, PCK>, J, c);
+	return cudaLaunchKernelEx(&cfg, k_resident<LN, K, PCK, SOLO>, J, c);
+}
+
+template <int LN, int K, int PCK>
+cudaError_t resident_t(const ResJob & J, const TConst & c, cudaStream_t s, int ncand, bool * fits)
+{
+	if constexpr (LN >= 11)
+	{
+		if (ncand == 0)
+		{
+			// both set up before any capture
+			const cudaError_t e = resident_v<LN, K, PCK, true>(J, c, s, 0, fits);
+			if (e != cudaSuccess || (fits && !*fits)) return e;
+		}
+		if (ncand == 1) return resident_v<LN, K, PCK, true>(J, c, s, ncand, fits);
+	}
+	return resident_v<LN, K, PCK, false>(J, c, s, ncand, fits);
 }
 
 template <int K, int PCK>
