@@ -49,7 +49,7 @@ struct RowTw
 	u32 H;
 };
 
-template <int S, bool INV>
+template <int S, bool INV, int MIR>
 __device__ __forceinline__ void rp_radix(u32 (&v)[RP_EPT], u32 tid, u32 T, int b, int LB, const RowTw & tw,
 	u32 Hr, u32 p, u32 p2)
 {
@@ -67,7 +67,7 @@ __device__ __forceinline__ void rp_radix(u32 (&v)[RP_EPT], u32 tid, u32 T, int b
 			// CNT = 2^(S-1-s) adjacent pairs, aligned to them: 16-byte loads
 			uint2 wv[1 << (S - 1)];
 			const int CNT = 1 << (S - 1 - s);
-			const bool mirror = INV && tw.wi == nullptr;
+			const bool mirror = INV && (MIR < 0 ? tw.wi == nullptr : MIR != 0);
 			const uint2 * const wp = !INV ? tw.w + i0 : !mirror ? tw.wi + i0 : tw.w + (3u * (tw.H << t) - i0 - (u32)CNT);
 			if (CNT == 1) wv[0] = __ldg(wp);
 			else
@@ -169,7 +169,7 @@ __device__ __forceinline__ void rp_store_global(const u32 (&v)[RP_EPT], u32 * __
 // the inverse levels.
 // w1: the 8 twiddles of the thread pair's last forward level (just read by
 // the forward stage, so an L1 hit), which are the polynomials' c.
-__device__ __forceinline__ void rp_pointwise(u32 (&v)[RP_EPT], const u32 * __restrict__ xp, bool is_mul, u32 tid, u32 NT,
+__device__ __forceinline__ void rp_pointwise(u32 (&v)[RP_EPT], const u32 * __restrict__ xp, const bool is_mul, u32 tid, u32 NT,
 	const uint2 * __restrict__ w1, u32 p, u32 p2, u32 pinv)
 {
 	// tid: virtual thread (its 16 words are the last-stage elements
@@ -206,14 +206,16 @@ __device__ __forceinline__ void reduce_all(u32 (&v)[N], u32 p2)
 
 // Physical threads of a row-pass CTA: 16 words per virtual thread, at most
 // 256 threads, each running R / (16 * threads) rounds per stage.  The kernel
-// is compiled for 4 CTAs per SM (at most 64 registers), so that the Q- and
-// R-domain row passes, which run side by side on two streams, are resident
-// together.
+// is compiled for 3 CTAs per SM (80 registers, no spills): the grids of the
+// long lengths have 2.6 per SM (33.2M bits: 384), and 4 of them at 64 registers
+// measured the same there and slower below (us per squaring, 4 / 3: 33.2M bits
+// 150.2 / 150.4, 6.6M bits 51.4 / 48.2, 2M bits 29.9 / 26.9).  128 threads:
+// 185.5 at 33.2M bits; 512: 155.5.
 #ifndef AB_ROW_THREADS
 #define AB_ROW_THREADS 256
 #endif
 #ifndef AB_ROW_MINB
-#define AB_ROW_MINB 4
+#define AB_ROW_MINB 3
 #endif
 template <int LOG_R>
 struct RowCfg
@@ -254,7 +256,9 @@ __device__ __forceinline__ void rp_touch(u32 vt0, u32 lane, int LB, const RowTw 
 // threads (tid < P) sharing the padded row buffer sm.  When P exceeds the
 // row's virtual threads T, the threads above T only take part in the
 // barriers.  mask_nt: threads of the CTA, for the shuffle masks.
-template <int LOG_R, u32 P>
+// MODE, MIR: the job's RowMode and whether its inverse twiddles are the
+// mirrored forward ones (domain Q), or -1 where only the job knows.
+template <int LOG_R, u32 P, int MODE, int MIR>
 __device__ __forceinline__ void rowpass_body(const RowJob & J, const TConst & c, u32 cand, u32 bx, u32 tid, u32 * sm, u32 mask_nt)
 {
 	constexpr int LB = LOG_R - 1;
@@ -265,6 +269,7 @@ __device__ __forceinline__ void rowpass_body(const RowJob & J, const TConst & c,
 	constexpr int NS = (NL == 0) ? 0 : 1 + (NL - S0) / 4;        // stages above the last
 	constexpr int B0 = LB + 1 - S0;
 
+	const int mode = (MODE < 0) ? J.mode : MODE;
 	const size_t cofs = (size_t)cand * J.stride;
 	const u32 k = bx / c.HR, r = bx - k * c.HR;
 	const u32 p = c.p[k], p2 = 2 * p, pinv = c.pinv[k];
@@ -273,7 +278,7 @@ __device__ __forceinline__ void rowpass_body(const RowJob & J, const TConst & c,
 	tw.w = J.w + (size_t)k * (c.n >> 1);
 	tw.wi = (J.wi != nullptr) ? J.wi + (size_t)k * (c.n >> 1) : nullptr;
 	tw.H = c.HR;
-	const u32 * __restrict__ xp = (J.mode == ROW_MUL) ? J.xp + cofs + (size_t)k * c.n + (size_t)r * (1u << LOG_R) : nullptr;
+	const u32 * __restrict__ xp = (mode == ROW_MUL) ? J.xp + cofs + (size_t)k * c.n + (size_t)r * (1u << LOG_R) : nullptr;
 	const u32 Hr = c.HR + r;
 	// threads of a shuffle: with idle threads, only the first T of the first warp
 	const u32 mnt = (IDLE && T < 32) ? T : mask_nt;
@@ -290,11 +295,11 @@ __device__ __forceinline__ void rowpass_body(const RowJob & J, const TConst & c,
 			const u32 vt = tid + rr * NT;
 			if (IDLE && vt >= T) continue;
 			rp_load_global<4>(v, x, vt, T, 1);
-			rp_radix<4, false>(v, vt, T, 1, LB, tw, Hr, p, p2);
-			if (J.mode != ROW_FWD_ONLY)
+			rp_radix<4, false, MIR>(v, vt, T, 1, LB, tw, Hr, p, p2);
+			if (mode != ROW_FWD_ONLY)
 			{
-				rp_pointwise(v, xp, J.mode == ROW_MUL, vt, mnt, w1(vt), p, p2, pinv);
-				rp_radix<4, true>(v, vt, T, 1, LB, tw, Hr, p, p2);
+				rp_pointwise(v, xp, mode == ROW_MUL, vt, mnt, w1(vt), p, p2, pinv);
+				rp_radix<4, true, MIR>(v, vt, T, 1, LB, tw, Hr, p, p2);
 			}
 			else reduce_all(v, p2);
 			rp_store_global<4>(v, x, vt, T, 1);
@@ -310,7 +315,7 @@ __device__ __forceinline__ void rowpass_body(const RowJob & J, const TConst & c,
 			const u32 vt = tid + rr * NT;
 			if (IDLE && vt >= T) continue;
 			rp_load_global<S0>(v, x, vt, T, B0);
-			rp_radix<S0, false>(v, vt, T, B0, LB, tw, Hr, p, p2);
+			rp_radix<S0, false, MIR>(v, vt, T, B0, LB, tw, Hr, p, p2);
 			rp_store_smem<S0>(v, sm, vt, T, B0);
 		}
 		int b = B0;
@@ -325,11 +330,11 @@ __device__ __forceinline__ void rowpass_body(const RowJob & J, const TConst & c,
 				const u32 vt = tid + rr * NT;
 			if (IDLE && vt >= T) continue;
 				rp_load_smem<4>(v, sm, vt, T, b);
-				rp_radix<4, false>(v, vt, T, b, LB, tw, Hr, p, p2);
+				rp_radix<4, false, MIR>(v, vt, T, b, LB, tw, Hr, p, p2);
 				rp_store_smem<4>(v, sm, vt, T, b);
 			}
 		}
-		const bool ahead = (T >= 32) && J.mode != ROW_FWD_ONLY;
+		const bool ahead = (T >= 32) && mode != ROW_FWD_ONLY;
 		if (ahead && tid < T) rp_touch(tid & ~31u, tid & 31, LB, tw, Hr, xp);
 		__syncthreads();
 
@@ -341,18 +346,18 @@ __device__ __forceinline__ void rowpass_body(const RowJob & J, const TConst & c,
 			if (IDLE && vt >= T) continue;
 			if (ahead && vt + NT < T) rp_touch((vt + NT) & ~31u, tid & 31, LB, tw, Hr, xp);
 			rp_load_smem<4>(v, sm, vt, T, 1);
-			rp_radix<4, false>(v, vt, T, 1, LB, tw, Hr, p, p2);
-			if (J.mode == ROW_FWD_ONLY)
+			rp_radix<4, false, MIR>(v, vt, T, 1, LB, tw, Hr, p, p2);
+			if (mode == ROW_FWD_ONLY)
 			{
 				reduce_all(v, p2);
 				rp_store_global<4>(v, x, vt, T, 1);
 				continue;
 			}
-			rp_pointwise(v, xp, J.mode == ROW_MUL, vt, mnt, w1(vt), p, p2, pinv);
-			rp_radix<4, true>(v, vt, T, 1, LB, tw, Hr, p, p2);
+			rp_pointwise(v, xp, mode == ROW_MUL, vt, mnt, w1(vt), p, p2, pinv);
+			rp_radix<4, true, MIR>(v, vt, T, 1, LB, tw, Hr, p, p2);
 			rp_store_smem<4>(v, sm, vt, T, 1);
 		}
-		if (J.mode == ROW_FWD_ONLY) return;
+		if (mode == ROW_FWD_ONLY) return;
 
 		// ---- inverse: back up through smem, stage 0 to global
 		b = 1;
@@ -367,7 +372,7 @@ __device__ __forceinline__ void rowpass_body(const RowJob & J, const TConst & c,
 				const u32 vt = tid + rr * NT;
 			if (IDLE && vt >= T) continue;
 				rp_load_smem<4>(v, sm, vt, T, b);
-				rp_radix<4, true>(v, vt, T, b, LB, tw, Hr, p, p2);
+				rp_radix<4, true, MIR>(v, vt, T, b, LB, tw, Hr, p, p2);
 				rp_store_smem<4>(v, sm, vt, T, b);
 			}
 		}
@@ -378,20 +383,22 @@ __device__ __forceinline__ void rowpass_body(const RowJob & J, const TConst & c,
 			const u32 vt = tid + rr * NT;
 			if (IDLE && vt >= T) continue;
 			rp_load_smem<S0>(v, sm, vt, T, B0);
-			rp_radix<S0, true>(v, vt, T, B0, LB, tw, Hr, p, p2);
+			rp_radix<S0, true, MIR>(v, vt, T, B0, LB, tw, Hr, p, p2);
 			rp_store_global<S0>(v, x, vt, T, B0);
 		}
 	}
 }
 
-template <int LOG_R>
+template <int LOG_R, int MODE>
 __global__ void __launch_bounds__(RowCfg<LOG_R>::NT, RowCfg<LOG_R>::MINB) k_rowpass(const RowJobs jobs, const TConst c)
 {
 	extern __shared__ __align__(16) u32 sm[];
 	const RowJob J = (blockIdx.y == 0) ? jobs.j[0] : jobs.j[1];
 	const u32 cand = blockIdx.z;
 	if (J.active != nullptr && J.active[cand] == 0u) return;
-	rowpass_body<LOG_R, RowCfg<LOG_R>::NT>(J, c, cand, blockIdx.x, threadIdx.x, sm, RowCfg<LOG_R>::NT);
+	constexpr u32 NT = RowCfg<LOG_R>::NT;
+	if (J.wi != nullptr) rowpass_body<LOG_R, NT, MODE, 0>(J, c, cand, blockIdx.x, threadIdx.x, sm, NT);
+	else rowpass_body<LOG_R, NT, MODE, 1>(J, c, cand, blockIdx.x, threadIdx.x, sm, NT);
 }
 
 // ================================================================ column pass
@@ -472,11 +479,11 @@ struct ColStages
 
 // Inverse levels of every tile column, from global memory (x: plane 0, row 0)
 // into the tile.
-template <int LOG_H, int KP>
+template <int LOG_H, int KP, int NT>
 __device__ __forceinline__ void col_inverse(const u32 * __restrict__ x, u32 n, u32 R, u32 gc, bool live, u32 * tile, const uint2 * twk, const TConst & c)
 {
 	constexpr int SB = ColStages<LOG_H>::SB, ST = ColStages<LOG_H>::ST, PS = CW << LOG_H;
-	const int tid = (int)threadIdx.x, NT = (int)blockDim.x, u = tid & 31;
+	const int tid = (int)threadIdx.x, u = tid & 31;
 	for (int task = tid; task < (KP << (LOG_H - SB + 5)); task += NT)
 	{
 		const int o = (task >> 5) & ((1 << (LOG_H - SB)) - 1), k = task >> (LOG_H - SB + 5);
@@ -497,11 +504,11 @@ __device__ __forceinline__ void col_inverse(const u32 * __restrict__ x, u32 n, u
 }
 
 // Forward levels of the own columns, from the tile into global memory.
-template <int LOG_H, int KP>
+template <int LOG_H, int KP, int NT>
 __device__ __forceinline__ void col_forward(u32 * tile, u32 * __restrict__ x, u32 n, u32 R, u32 gc, bool own, const uint2 * twk, const TConst & c)
 {
 	constexpr int SB = ColStages<LOG_H>::SB, ST = ColStages<LOG_H>::ST, PS = CW << LOG_H;
-	const int tid = (int)threadIdx.x, NT = (int)blockDim.x, u = tid & 31;
+	const int tid = (int)threadIdx.x, u = tid & 31;
 	if constexpr (ST > 0)
 	{
 		for (int task = tid; task < (KP << (LOG_H - ST + 5)); task += NT)
@@ -572,7 +579,7 @@ __device__ __forceinline__ void carry_phase2(const Width & w, const Big<AB_NW> &
 	for (int i = 0; i < AB_NW; ++i) x[3][i] = g.l[i];
 }
 
-// The column pass of column group b of nb of candidate cand, by all threads
+// The column pass of column group b of nb of candidate cand, by the NT threads
 // of the CTA (a multiple of 32); sm: colpass_smem bytes of shared memory.
 //
 // Bound by the integer multiplier (butterflies 4 units each, CRT about 75 and
@@ -586,7 +593,7 @@ __device__ __forceinline__ void carry_phase2(const Width & w, const Big<AB_NW> &
 // WIDE: a thread per tile word (32 H threads) and the carry by 4 lanes per
 // group (carry.cuh), for launches that do not fill the GPU.  SPARSE: the source
 // is SRC_SPARSE (both jobs of the launch).
-template <int LOG_H, int K, int PCK, bool WIDE, bool SPARSE>
+template <int LOG_H, int K, int PCK, bool WIDE, bool SPARSE, int NT>
 __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 cand, int b, int nb, u32 * sm, int & decision)
 {
 	constexpr int KP = K + 1, L = K;             // transform primes, limbs of the carry
@@ -615,7 +622,7 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 	const int E = single ? 0 : (b == 0) ? 8 : 4;
 	const u32 c0 = (b == 0) ? 0u : 28u * (u32)b - 4u;                  // first own column
 	const int WU = min(CW, E + (int)(R - c0)), ng = WU / 4;            // live columns and groups of a row
-	const int tid = (int)threadIdx.x, NT = (int)blockDim.x;
+	const int tid = (int)threadIdx.x;
 	// global column of tile column u (CTA 0's predecessors end the previous row)
 	auto gcol = [&](int u) -> u32 { return c0 + (u32)(u - E) + ((b == 0 && u < E) ? R : 0u); };
 	const int lane = tid & 31;
@@ -674,7 +681,7 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 	{
 		// ---- inverse column levels
 		auto get_m = [&](u32 i, u32 & d0, u32 & d1, u32 & d2) { d0 = J.in[i]; d1 = J.in[n + i]; d2 = J.in[2 * (size_t)n + i]; };
-		if constexpr (!SPARSE) col_inverse<LOG_H, KP>(J.in, n, R, gcol(lane), lane < WU, tile, twc, c);
+		if constexpr (!SPARSE) col_inverse<LOG_H, KP, NT>(J.in, n, R, gcol(lane), lane < WU, tile, twc, c);
 
 		const Width w = make_width(wbits);
 		const bool full = (w.ws == ND - 1);
@@ -927,7 +934,7 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 			}
 		}
 		__syncthreads();
-		col_forward<LOG_H, KP>(tile, out, n, R, gcol(lane), own, twc + (1 + dom) * KP * H, c);
+		col_forward<LOG_H, KP, NT>(tile, out, n, R, gcol(lane), own, twc + (1 + dom) * KP * H, c);
 		in_tile = false;
 	}
 }
@@ -937,7 +944,7 @@ __global__ void __launch_bounds__(ColCfg<LOG_H, WIDE>::NT, ColCfg<LOG_H, WIDE>::
 {
 	extern __shared__ __align__(16) u32 sm[];
 	__shared__ int decision;
-	colpass_body<LOG_H, K, PCK, WIDE, SPARSE>((blockIdx.y == 0) ? jobs.j[0] : jobs.j[1], c, blockIdx.z, (int)blockIdx.x, (int)gridDim.x, sm, decision);
+	colpass_body<LOG_H, K, PCK, WIDE, SPARSE, ColCfg<LOG_H, WIDE>::NT>((blockIdx.y == 0) ? jobs.j[0] : jobs.j[1], c, blockIdx.z, (int)blockIdx.x, (int)gridDim.x, sm, decision);
 }
 
 // ================================================================ mixed-size passes
@@ -984,22 +991,22 @@ __global__ void __launch_bounds__(AB_FUSED_ROW_THREADS, 4) k_fused_rowpass(const
 	constexpr u32 P = AB_FUSED_ROW_THREADS;
 	switch (d->log_r[f.ci])
 	{
-	case 5: rowpass_body<5, P>(J, cs, f.cand, f.bx, threadIdx.x, sm, P); break;
-	case 6: rowpass_body<6, P>(J, cs, f.cand, f.bx, threadIdx.x, sm, P); break;
-	case 7: rowpass_body<7, P>(J, cs, f.cand, f.bx, threadIdx.x, sm, P); break;
-	case 8: rowpass_body<8, P>(J, cs, f.cand, f.bx, threadIdx.x, sm, P); break;
-	case 9: rowpass_body<9, P>(J, cs, f.cand, f.bx, threadIdx.x, sm, P); break;
-	case 10: rowpass_body<10, P>(J, cs, f.cand, f.bx, threadIdx.x, sm, P); break;
-	case 11: rowpass_body<11, P>(J, cs, f.cand, f.bx, threadIdx.x, sm, P); break;
-	case 12: rowpass_body<12, P>(J, cs, f.cand, f.bx, threadIdx.x, sm, P); break;
-	case 13: rowpass_body<13, P>(J, cs, f.cand, f.bx, threadIdx.x, sm, P); break;
-	case 14: rowpass_body<14, P>(J, cs, f.cand, f.bx, threadIdx.x, sm, P); break;
+	case 5: rowpass_body<5, P, -1, -1>(J, cs, f.cand, f.bx, threadIdx.x, sm, P); break;
+	case 6: rowpass_body<6, P, -1, -1>(J, cs, f.cand, f.bx, threadIdx.x, sm, P); break;
+	case 7: rowpass_body<7, P, -1, -1>(J, cs, f.cand, f.bx, threadIdx.x, sm, P); break;
+	case 8: rowpass_body<8, P, -1, -1>(J, cs, f.cand, f.bx, threadIdx.x, sm, P); break;
+	case 9: rowpass_body<9, P, -1, -1>(J, cs, f.cand, f.bx, threadIdx.x, sm, P); break;
+	case 10: rowpass_body<10, P, -1, -1>(J, cs, f.cand, f.bx, threadIdx.x, sm, P); break;
+	case 11: rowpass_body<11, P, -1, -1>(J, cs, f.cand, f.bx, threadIdx.x, sm, P); break;
+	case 12: rowpass_body<12, P, -1, -1>(J, cs, f.cand, f.bx, threadIdx.x, sm, P); break;
+	case 13: rowpass_body<13, P, -1, -1>(J, cs, f.cand, f.bx, threadIdx.x, sm, P); break;
+	case 14: rowpass_body<14, P, -1, -1>(J, cs, f.cand, f.bx, threadIdx.x, sm, P); break;
 	default: break;
 	}
 }
 
 #define AB_FUSED_COL(LH, KK, PP) \
-	case LH * 8 + KK: colpass_body<LH, KK, PP, false, false>(J, cs, f.cand, (int)f.bx, (int)d->nbx[f.ci], sm, decision); break;
+	case LH * 8 + KK: colpass_body<LH, KK, PP, false, false, COL_THREADS>(J, cs, f.cand, (int)f.bx, (int)d->nbx[f.ci], sm, decision); break;
 #define AB_FUSED_COL_K(LH) AB_FUSED_COL(LH, 2, 1) AB_FUSED_COL(LH, 3, 2) AB_FUSED_COL(LH, 4, 2) AB_FUSED_COL(LH, 5, 4)
 
 __global__ void __launch_bounds__(COL_THREADS, 2) k_fused_colpass(const FusedColPass * __restrict__ d, const TConst * __restrict__ tcs)
@@ -1206,16 +1213,36 @@ static cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t 
 	return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
 }
 
-template <int LOG_R>
-static cudaError_t rowpass_t(const Geometry & g, const TConst & c, const RowJobs & jobs, int njobs, cudaStream_t s, int ncand)
+template <int LOG_R, int MODE>
+static cudaError_t rowpass_m(const Geometry & g, const TConst & c, const RowJobs & jobs, int njobs, cudaStream_t s, int ncand)
 {
 	const size_t smem = RowCfg<LOG_R>::SMEM;
 	static std::atomic<unsigned long long> attr_done{0};
-	const cudaError_t e = allow_dynamic_smem(k_rowpass<LOG_R>, smem, attr_done);
+	const cudaError_t e = allow_dynamic_smem(k_rowpass<LOG_R, MODE>, smem, attr_done);
 	if (e != cudaSuccess) return e;
 	if (ncand == 0) return cudaSuccess;      // set-up only (before a stream capture)
 	const dim3 grid((unsigned)(c.KP * g.HR), (unsigned)njobs, (unsigned)ncand);
-	return launch_pdl(k_rowpass<LOG_R>, grid, dim3(RowCfg<LOG_R>::NT), smem, s, jobs, c);
+	return launch_pdl(k_rowpass<LOG_R, MODE>, grid, dim3(RowCfg<LOG_R>::NT), smem, s, jobs, c);
+}
+
+// The jobs of a launch have one mode.
+template <int LOG_R>
+static cudaError_t rowpass_t(const Geometry & g, const TConst & c, const RowJobs & jobs, int njobs, cudaStream_t s, int ncand)
+{
+	if (ncand == 0)
+	{
+		cudaError_t e = rowpass_m<LOG_R, ROW_FWD_ONLY>(g, c, jobs, njobs, s, 0);
+		if (e == cudaSuccess) e = rowpass_m<LOG_R, ROW_SQUARE>(g, c, jobs, njobs, s, 0);
+		return (e != cudaSuccess) ? e : rowpass_m<LOG_R, ROW_MUL>(g, c, jobs, njobs, s, 0);
+	}
+	if (njobs > 1 && jobs.j[1].mode != jobs.j[0].mode) return cudaErrorInvalidValue;
+	switch (jobs.j[0].mode)
+	{
+	case ROW_FWD_ONLY: return rowpass_m<LOG_R, ROW_FWD_ONLY>(g, c, jobs, njobs, s, ncand);
+	case ROW_SQUARE: return rowpass_m<LOG_R, ROW_SQUARE>(g, c, jobs, njobs, s, ncand);
+	case ROW_MUL: return rowpass_m<LOG_R, ROW_MUL>(g, c, jobs, njobs, s, ncand);
+	default: return cudaErrorInvalidValue;
+	}
 }
 
 cudaError_t launch_rowpass(const Geometry & g, const TConst & c, const RowJobs & jobs, int njobs, cudaStream_t s, int ncand)
