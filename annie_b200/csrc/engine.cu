@@ -303,7 +303,7 @@ struct ab_transform
 	u32 * b(int i) const { return bufp[i]; }
 	static size_t words_of(int i, int K, size_t n)
 	{
-		if (i == XW) return (size_t)K * n;
+		if (i == XW) return (size_t)2 * K * n;
 		if (i == WR || i == WRI || i == WQ) return (size_t)(K + 1) * n;        // n/2 pairs per prime
 		if (i == WC) return (size_t)4 * (K + 1) * COLTW * 2;
 		return (i < NSLOT && normal_buf(i)) ? (size_t)AB_NW * n : (size_t)(K + 1) * n;
@@ -741,7 +741,9 @@ struct ab_transform
 
 	void upload(int buf, const u32 * src)
 	{
-		CK(cudaMemcpyAsync(b(buf), src, words_of(buf) * 4, cudaMemcpyHostToDevice, st));
+		// XW has room for two registers' words, an upload is one register
+		const size_t words = (buf == XW) ? (size_t)prm.K * n : words_of(buf);
+		CK(cudaMemcpyAsync(b(buf), src, words * 4, cudaMemcpyHostToDevice, st));
 		CK(cudaStreamSynchronize(st));
 	}
 	void download(int buf, u32 * dst, size_t words)
@@ -750,23 +752,24 @@ struct ab_transform
 		CK(cudaStreamSynchronize(st));
 	}
 
-	// the reference's register words (K planes) of a normal-form buffer, into XW
-	void export_words(int buf)
+	// the reference's register words (K planes) of a normal-form buffer, into XW;
+	// of two, with interleaved planes, as a checkpoint has them
+	void export_words(int buf, int buf1 = -1)
 	{
-		CK(launch_export(rc, b(buf), b(XW), (u32)n, st));
+		CK(launch_export(rc, b(buf), (buf1 < 0) ? nullptr : b(buf1), b(XW), (u32)n, st));
 		++launches;
 	}
-	// XW (the reference's register words) into a normal-form buffer; returns
-	// false when they are not a normal-form register
-	bool import_words(int buf)
+	// XW (the reference's register words) into one normal-form buffer or two;
+	// returns false when they are not normal-form registers
+	bool import_words(int buf, int buf1 = -1)
 	{
 		CK(cudaMemsetAsync(d_flag, 0, sizeof(u32), st));
-		CK(launch_import(rc, b(XW), b(buf), (u32)n, d_flag, st));
+		CK(launch_import(rc, b(XW), b(buf), (buf1 < 0) ? nullptr : b(buf1), (u32)n, d_flag, st));
 		++launches;
 		u32 bad = 0;
 		CK(cudaMemcpyAsync(&bad, d_flag, sizeof(u32), cudaMemcpyDeviceToHost, st));
 		CK(cudaStreamSynchronize(st));
-		if (buf == REG0) prefwd = false;
+		if (buf == REG0 || buf1 == REG0) prefwd = false;
 		return bad == 0;
 	}
 
@@ -1252,13 +1255,9 @@ int ab_save_checkpoint(ab_transform * h, void * buf, size_t cap, size_t * writte
 		u32 * o = static_cast<u32 *>(buf);
 		o[0] = (u32)K; o[1] = (u32)n;
 		// per prime k: plane k of Reg0 then plane k of Reg1 (transformGPU.h:626-641),
-		// the reference's register words
-		for (int r = 0; r < 2; ++r)
-		{
-			h->export_words(r == 0 ? ab_transform::REG0 : ab_transform::REG1);
-			for (size_t k = 0; k < K; ++k)
-				CK(cudaMemcpyAsync(o + 2 + 2 * k * n + r * n, h->b(ab_transform::XW) + k * n, n * 4, cudaMemcpyDeviceToHost, h->st));
-		}
+		// the reference's register words: one conversion, one copy
+		h->export_words(ab_transform::REG0, ab_transform::REG1);
+		CK(cudaMemcpyAsync(o + 2, h->b(ab_transform::XW), 2 * K * n * 4, cudaMemcpyDeviceToHost, h->st));
 		CK(cudaStreamSynchronize(h->st));
 		if (written) *written = need;
 	});
@@ -1272,13 +1271,8 @@ int ab_read_checkpoint(ab_transform * h, const void * buf, size_t size)
 		if (buf == nullptr || size < 8) throw ab_error(AB_E_CHECKPOINT, "checkpoint too short");
 		const u32 * in = static_cast<const u32 *>(buf);
 		if (in[0] != K || in[1] != n || size < ab_checkpoint_size(h)) throw ab_error(AB_E_CHECKPOINT, "checkpoint does not match K or n");
-		bool ok = true;
-		for (int r = 0; r < 2; ++r)
-		{
-			for (size_t k = 0; k < K; ++k)
-				CK(cudaMemcpyAsync(h->b(ab_transform::XW) + k * n, in + 2 + 2 * k * n + r * n, n * 4, cudaMemcpyHostToDevice, h->st));
-			ok = h->import_words(r == 0 ? ab_transform::REG0 : ab_transform::REG1) && ok;
-		}
+		CK(cudaMemcpyAsync(h->b(ab_transform::XW), in + 2, 2 * K * n * 4, cudaMemcpyHostToDevice, h->st));
+		const bool ok = h->import_words(ab_transform::REG0, ab_transform::REG1);
 		h->prefwd = false;
 		if (!ok) throw ab_error(AB_E_CHECKPOINT, "checkpoint registers are not in normal form");
 	});
@@ -1400,11 +1394,11 @@ int ab_square_mul_noalloc(ab_transform * h, uint32_t * reg, int32_t a)
 		// static scratch, then back to the caller's register words.  Each
 		// scratch word is written before it is read within the call, so
 		// nothing needs clearing between calls.
-		CK(launch_import(h->rc, reg, x, (u32)n, flag, h->st));
+		CK(launch_import(h->rc, reg, x, nullptr, (u32)n, flag, h->st));
 		if (h->resident)
 		{
 			h->run_resident(x, nullptr, 1, 1, (u32)a);
-			CK(launch_export(h->rc, x, reg, (u32)n, h->st));
+			CK(launch_export(h->rc, x, nullptr, reg, (u32)n, h->st));
 			h->launches += 2;
 			return;
 		}
@@ -1428,7 +1422,7 @@ int ab_square_mul_noalloc(ab_transform * h, uint32_t * reg, int32_t a)
 			j2 = h->cj_tr(aq1, true, 1, tq, LOWER_Q);
 		}
 		j2.out_norm = x; h->cols(j2);
-		CK(launch_export(h->rc, x, reg, (u32)n, h->st));
+		CK(launch_export(h->rc, x, nullptr, reg, (u32)n, h->st));
 		h->launches += 2;
 	});
 }

@@ -1041,10 +1041,16 @@ __device__ __forceinline__ u32 ref_mont(u32 a, u32 b, u32 p, u32 q)
 
 __device__ __forceinline__ u32 ref_add(u32 a, u32 b, u32 p) { return ref_sub(a, p - b, p); }
 
-__global__ void k_export(const RefConst rc, const u32 * __restrict__ norm, u32 * __restrict__ words, u32 n)
+// Both conversions take one register, or two with interleaved planes of words
+// (plane k of the second after plane k of the first: a checkpoint's payload),
+// blockIdx.y the register, ws the words between planes.
+__global__ void k_export(const RefConst rc, const u32 * __restrict__ norm0, const u32 * __restrict__ norm1, u32 * __restrict__ words, u32 n, u32 ws)
 {
 	const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+	griddep_wait();
 	if (i >= n) return;
+	const u32 * __restrict__ norm = (blockIdx.y == 0) ? norm0 : norm1;
+	words += blockIdx.y * n;
 	u32 d0 = norm[i], d1 = norm[n + i], d2 = norm[2 * (size_t)n + i];
 	const bool neg = (i32)d2 < 0;
 	if (neg)
@@ -1061,22 +1067,25 @@ __global__ void k_export(const RefConst rc, const u32 * __restrict__ norm, u32 *
 		const u32 a2 = ref_mont(ref_mont(d2, r2, p, q), r2, p, q);   // d2 2^64
 		u32 r = ref_add(ref_add(a0, a1, p), a2, p);
 		if (neg && r != 0) r = p - r;
-		words[(size_t)k * n + i] = r;
+		words[(size_t)k * ws + i] = r;
 	}
 }
 
 // Exact signed value from the K residues (mixed-radix Garner, leading digit
 // balanced; kernel.cl:1231-1470), checked against the 96-bit normal form.
 template <int K>
-__global__ void k_import(const RefConst rc, const u32 * __restrict__ words, u32 * __restrict__ norm, u32 n, u32 * bad)
+__global__ void k_import(const RefConst rc, const u32 * __restrict__ words, u32 * __restrict__ norm0, u32 * __restrict__ norm1, u32 n, u32 ws, u32 * bad)
 {
 	const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+	griddep_wait();
 	if (i >= n) return;
+	u32 * __restrict__ norm = (blockIdx.y == 0) ? norm0 : norm1;
+	words += blockIdx.y * n;
 	u32 u[K];
 #pragma unroll
 	for (int ii = K - 1; ii >= 0; --ii)
 	{
-		u32 v = words[(size_t)ii * n + i];
+		u32 v = words[(size_t)ii * ws + i];
 #pragma unroll
 		for (int j = K - 1; j > ii; --j) v = ref_mont_c(ref_sub(v, u[j], rc.p[ii]), rc.gm[ii][j], rc.gmq[ii][j], rc.p[ii]);
 		u[ii] = v;
@@ -1391,26 +1400,31 @@ cudaError_t launch_fused_colpass(const FusedColPass * d, const TConst * tcs, u32
 	return launch_pdl(k_fused_colpass, dim3(ctas), dim3(COL_THREADS), smem, s, d, tcs);
 }
 
-cudaError_t launch_export(const RefConst & rc, const u32 * norm, u32 * words, u32 n, cudaStream_t s)
+cudaError_t launch_export(const RefConst & rc, const u32 * norm0, const u32 * norm1, u32 * words, u32 n, cudaStream_t s)
 {
 	if (n == 0) return cudaSuccess;
-	k_export<<<(n + 255) / 256, 256, 0, s>>>(rc, norm, words, n);
-	return cudaGetLastError();
+	const u32 regs = (norm1 != nullptr) ? 2 : 1;
+	return launch_pdl(k_export, dim3((n + 255) / 256, regs), dim3(256), 0, s, rc, norm0, norm1, words, n, regs * n);
 }
 
-cudaError_t launch_import(const RefConst & rc, const u32 * words, u32 * norm, u32 n, u32 * bad, cudaStream_t s)
+template <int K>
+static cudaError_t import_t(const RefConst & rc, const u32 * words, u32 * norm0, u32 * norm1, u32 n, u32 * bad, cudaStream_t s)
+{
+	const u32 regs = (norm1 != nullptr) ? 2 : 1;
+	return launch_pdl(k_import<K>, dim3((n + 255) / 256, regs), dim3(256), 0, s, rc, words, norm0, norm1, n, regs * n, bad);
+}
+
+cudaError_t launch_import(const RefConst & rc, const u32 * words, u32 * norm0, u32 * norm1, u32 n, u32 * bad, cudaStream_t s)
 {
 	if (n == 0) return cudaSuccess;
-	const unsigned nb = (n + 255) / 256;
 	switch (rc.K)
 	{
-	case 2: k_import<2><<<nb, 256, 0, s>>>(rc, words, norm, n, bad); break;
-	case 3: k_import<3><<<nb, 256, 0, s>>>(rc, words, norm, n, bad); break;
-	case 4: k_import<4><<<nb, 256, 0, s>>>(rc, words, norm, n, bad); break;
-	case 5: k_import<5><<<nb, 256, 0, s>>>(rc, words, norm, n, bad); break;
+	case 2: return import_t<2>(rc, words, norm0, norm1, n, bad, s);
+	case 3: return import_t<3>(rc, words, norm0, norm1, n, bad, s);
+	case 4: return import_t<4>(rc, words, norm0, norm1, n, bad, s);
+	case 5: return import_t<5>(rc, words, norm0, norm1, n, bad, s);
 	default: return cudaErrorInvalidValue;
 	}
-	return cudaGetLastError();
 }
 
 } // namespace ab

@@ -160,10 +160,11 @@ bool resident_fits(const TConst & c);
 cudaError_t launch_resident(const ResJob & J, const TConst & c, cudaStream_t s, int ncand = 1);
 
 // Register words of the reference (K planes of residues mod its primes) from
-// the normal form, and back.  The import sets *bad when a coefficient's value
-// does not fit the 96-bit normal form (the words are not a normal-form
-// register).
-cudaError_t launch_export(const RefConst & rc, const u32 * norm, u32 * words, u32 n, cudaStream_t s);
-cudaError_t launch_import(const RefConst & rc, const u32 * words, u32 * norm, u32 n, u32 * bad, cudaStream_t s);
+// the normal form, and back.  With norm1, two registers in one launch, plane k
+// of the second after plane k of the first.  The import sets *bad when a
+// coefficient's value does not fit the 96-bit normal form (the words are not a
+// normal-form register).
+cudaError_t launch_export(const RefConst & rc, const u32 * norm0, const u32 * norm1, u32 * words, u32 n, cudaStream_t s);
+cudaError_t launch_import(const RefConst & rc, const u32 * words, u32 * norm0, u32 * norm1, u32 n, u32 * bad, cudaStream_t s);
 
 } // namespace ab
