@@ -260,7 +260,14 @@ __global__ void __launch_bounds__(ResCfg<LN, K>::NT, SOLO ? 1 : ResCfg<LN, K>::M
 		if (last < 0) return;
 	}
 	auto encode_all = [&](const u32 * src) {
-		for (u32 i = tid; i < N; i += NT) xb[rpad(i)] = encode_res(c, (int)k, split30(src[i], src[N + i], src[2 * N + i]));
+		const uint4 * s0 = reinterpret_cast<const uint4 *>(src), * s1 = s0 + N / 4, * s2 = s1 + N / 4;
+		for (u32 i = tid; i < N / 4; i += NT)
+		{
+			const uint4 a = s0[i], b = s1[i], d = s2[i];
+			*reinterpret_cast<uint4 *>(xb + rpad(4 * i)) = make_uint4(
+				encode_res(c, (int)k, split30(a.x, b.x, d.x)), encode_res(c, (int)k, split30(a.y, b.y, d.y)),
+				encode_res(c, (int)k, split30(a.z, b.z, d.z)), encode_res(c, (int)k, split30(a.w, b.w, d.w)));
+		}
 	};
 	if (J.y != nullptr)
 	{
