@@ -1168,12 +1168,13 @@ bool make_geometry(int ln, int lb_override, Geometry & g)
 {
 	if (ln < 6 || ln > 22) return false;
 	const int L = ln - 1;
-	// default split, measured on B200 for single transforms (us per squaring
-	// over every split, ln 9..19): the row pass gets L - 2 levels up to 2^12
-	// points, then 11 levels, and the column pass takes the rest (at most 6);
-	// above 2^20 the row and column passes are full (13 and 6 levels) and the
-	// mid pass takes the 1 or 2 levels left
-	static const int DEFAULT_LB[23] = {0, 0, 0, 0, 0, 0, 4, 4, 5, 6, 7, 8, 9, 10, 10, 11, 11, 11, 11, 12, 13, 13, 13};
+	// default split, measured on B200 over every split (ln 13..20, single
+	// transforms; batches agree): us per squaring, e.g. ln 13 LB 9 / 10: 20.7 /
+	// 21.0 and, 32 slots, 51.8 / 62.2 per step; ln 15 LB 10 / 11: 28.2 / 26.9; ln 17
+	// LB 10 / 11: 48.4 / 48.1; ln 18 LB 11 / 12: 82.6 / 90.8.  Above 2^20 the row
+	// and column passes are full (13 and 6 levels) and the mid pass takes the 1
+	// or 2 levels left.
+	static const int DEFAULT_LB[23] = {0, 0, 0, 0, 0, 0, 4, 4, 5, 6, 7, 8, 9, 9, 10, 11, 11, 11, 11, 12, 13, 13, 13};
 	int LB = (lb_override > 0) ? lb_override : DEFAULT_LB[ln];
 	if (lb_override <= 0 && L - LB > 6 && ln <= 20) LB = L - 6;
 	if (LB < 4 || LB > 13 || LB > L - 1) return false;
