@@ -1,12 +1,11 @@
-// Butterfly levels of one transform (or one row of a longer one) of 2^LN words
-// held in shared memory, shared by the row pass (kernels.cu) and the resident
-// kernel (resident.cu).
+// Butterfly levels of a transform of 2^LN words held in shared memory
+// (resident.cu).
 //
 // 8 words per thread: stages of 3 levels, the top one taking the remainder,
 // and a bottom step of two levels, the pointwise product and two inverse
 // levels.  A stage costs a shared-memory round trip and a barrier, about the
-// same as its three levels; 16 words per thread would save one stage of a
-// row, but halves the warps that hide each other's latency.
+// same as its three levels; 16 words per thread would save one stage, but
+// halves the warps that hide each other's latency.
 #pragma once
 #include "kernels.h"
 
@@ -18,55 +17,53 @@ namespace ab
 // words stay 16-byte aligned.
 __host__ __device__ constexpr u32 rpad(u32 e) { return e + ((e >> 5) << 2); }
 
-// Twiddles of the 2^LN words: the level with 2^t polynomials at w + (wb << t)
-// + j, as Shoup pairs; -w^-1 of the inverse levels at wi + (ib << t) + j, or
-// mirrored, wi + (ib << t) + 2^t - 1 - j (domain Q, where that is the forward
-// table of the mirrored row).  GLOBAL: tables in global memory, else shared.
+// Twiddles of the 2^LN words in shared memory, as Shoup pairs: the level with
+// 2^t polynomials at w[2^t + j]; -w^-1 of the inverse levels at wi[2^t + j], or
+// mirrored, w[2^t + 2^t - 1 - j] (domain Q).
 struct LevelTw
 {
 	const uint2 * w, * wi;
-	u32 wb, ib;
 	bool mirror;
 };
 
 // CNT adjacent pairs from p (aligned to them)
-template <int CNT, bool GLOBAL>
+template <int CNT>
 __device__ __forceinline__ void load_pairs(const uint2 * p, uint2 (&v)[CNT])
 {
-	if constexpr (CNT == 1) v[0] = GLOBAL ? __ldg(p) : *p;
+	if constexpr (CNT == 1) v[0] = *p;
 	else
 	{
 #pragma unroll
 		for (int i = 0; i < CNT / 2; ++i)
 		{
-			const uint4 q = GLOBAL ? __ldg(reinterpret_cast<const uint4 *>(p) + i) : reinterpret_cast<const uint4 *>(p)[i];
+			const uint4 q = reinterpret_cast<const uint4 *>(p)[i];
 			v[2 * i] = make_uint2(q.x, q.y); v[2 * i + 1] = make_uint2(q.z, q.w);
 		}
 	}
 }
 
 // The twiddles j = x .. x + CNT - 1 of level t (CNT divides x).
-template <int CNT, bool INV, bool GLOBAL>
+template <int CNT, bool INV>
 __device__ __forceinline__ void level_tw(const LevelTw & tw, int t, u32 x, uint2 (&v)[CNT])
 {
-	if (!INV) load_pairs<CNT, GLOBAL>(tw.w + (tw.wb << t) + x, v);
-	else if (!tw.mirror) load_pairs<CNT, GLOBAL>(tw.wi + (tw.ib << t) + x, v);
+	if (!INV) load_pairs<CNT>(tw.w + (1u << t) + x, v);
+	else if (!tw.mirror) load_pairs<CNT>(tw.wi + (1u << t) + x, v);
 	else
 	{
 		uint2 r[CNT];
-		load_pairs<CNT, GLOBAL>(tw.wi + (tw.ib << t) + (1u << t) - x - CNT, r);
+		load_pairs<CNT>(tw.w + (2u << t) - x - CNT, r);
 #pragma unroll
 		for (int i = 0; i < CNT; ++i) v[i] = r[CNT - 1 - i];
 	}
 }
 
 // One level of a group's 2^S words: on group bit s, level t = LN - 1 - (B + s).
-template <int LN, int S, int B, bool INV, bool GLOBAL, int SB>
+template <int LN, int S, int B, bool INV, int SB>
 __device__ __forceinline__ void level(u32 (&v)[1 << S], const LevelTw & tw, u32 ohi, u32 p, u32 p2)
 {
 	constexpr int CNT = 1 << (S - 1 - SB);
 	uint2 wv[CNT];
-	level_tw<CNT, INV, GLOBAL>(tw, LN - 1 - (B + SB), ohi << (S - 1 - SB), wv);
+	level_tw<CNT, INV>(tw, LN - 1 - (B + SB), ohi << (S - 1 - SB), wv);
 #pragma unroll
 	for (int jh = 0; jh < CNT; ++jh)
 #pragma unroll
@@ -78,11 +75,9 @@ __device__ __forceinline__ void level(u32 (&v)[1 << S], const LevelTw & tw, u32 
 		}
 }
 
-// Levels on index bits B..B+S-1: forward from the top one, inverse from the
-// bottom one.  SRC / DST: the words lie in shared memory (padded) or, for the
-// outer end of a row, in global memory (plain).
-enum Where { IN_SHARED, IN_GLOBAL };
-template <int LN, int S, int B, bool INV, bool GLOBAL, Where SRC, Where DST>
+// Levels on index bits B..B+S-1 of the words at src into dst: forward from the
+// top one, inverse from the bottom one.
+template <int LN, int S, int B, bool INV>
 __device__ __forceinline__ void level_stage(const u32 * src, u32 * dst, const LevelTw & tw, u32 tid, u32 NT, u32 p, u32 p2)
 {
 	constexpr u32 N = 1u << LN;
@@ -90,29 +85,23 @@ __device__ __forceinline__ void level_stage(const u32 * src, u32 * dst, const Le
 	{
 		u32 v[1 << S];
 		const u32 ohi = o >> B;
-		const u32 e0 = (o & ((1u << B) - 1)) | (ohi << (B + S)), a0 = rpad(e0);
+		const u32 a0 = rpad((o & ((1u << B) - 1)) | (ohi << (B + S)));
 #pragma unroll
-		for (int g = 0; g < (1 << S); ++g) v[g] = (SRC == IN_GLOBAL) ? src[e0 + ((u32)g << B)] : src[a0 + rpad((u32)g << B)];
+		for (int g = 0; g < (1 << S); ++g) v[g] = src[a0 + rpad((u32)g << B)];
 		if constexpr (INV)
 		{
-			level<LN, S, B, true, GLOBAL, 0>(v, tw, ohi, p, p2);
-			if constexpr (S > 1) level<LN, S, B, true, GLOBAL, 1>(v, tw, ohi, p, p2);
-			if constexpr (S > 2) level<LN, S, B, true, GLOBAL, 2>(v, tw, ohi, p, p2);
-			if constexpr (S > 3) level<LN, S, B, true, GLOBAL, 3>(v, tw, ohi, p, p2);
+			level<LN, S, B, true, 0>(v, tw, ohi, p, p2);
+			if constexpr (S > 1) level<LN, S, B, true, 1>(v, tw, ohi, p, p2);
+			if constexpr (S > 2) level<LN, S, B, true, 2>(v, tw, ohi, p, p2);
 		}
 		else
 		{
-			if constexpr (S > 3) level<LN, S, B, false, GLOBAL, 3>(v, tw, ohi, p, p2);
-			if constexpr (S > 2) level<LN, S, B, false, GLOBAL, 2>(v, tw, ohi, p, p2);
-			if constexpr (S > 1) level<LN, S, B, false, GLOBAL, 1>(v, tw, ohi, p, p2);
-			level<LN, S, B, false, GLOBAL, 0>(v, tw, ohi, p, p2);
+			if constexpr (S > 2) level<LN, S, B, false, 2>(v, tw, ohi, p, p2);
+			if constexpr (S > 1) level<LN, S, B, false, 1>(v, tw, ohi, p, p2);
+			level<LN, S, B, false, 0>(v, tw, ohi, p, p2);
 		}
 #pragma unroll
-		for (int g = 0; g < (1 << S); ++g)
-		{
-			if (DST == IN_GLOBAL) dst[e0 + ((u32)g << B)] = v[g];
-			else dst[a0 + rpad((u32)g << B)] = v[g];
-		}
+		for (int g = 0; g < (1 << S); ++g) dst[a0 + rpad((u32)g << B)] = v[g];
 	}
 }
 
@@ -137,7 +126,7 @@ enum BottomMode { BOTTOM_SQUARE = 0, BOTTOM_MUL = 1, BOTTOM_FORWARD = 2 };
 // (BOTTOM_FORWARD) the last two levels only, the words in [0, 2p) to out.
 // op(o, a, b) gives the other factor's words 8 o .. 8 o + 7, out(o, a, b) takes
 // the image.
-template <int LN, bool GLOBAL, typename Op, typename Out>
+template <int LN, typename Op, typename Out>
 __device__ __forceinline__ void level_bottom(u32 * x, int mode, const LevelTw & tw, u32 tid, u32 NT, u32 p, u32 p2, u32 pinv, Op op, Out out)
 {
 	constexpr u32 N = 1u << LN;
@@ -151,8 +140,8 @@ __device__ __forceinline__ void level_bottom(u32 * x, int mode, const LevelTw & 
 		a = xp[0]; b = xp[1];
 		v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 		uint2 w0[1], w1[2];
-		level_tw<1, false, GLOBAL>(tw, LN - 3, o, w0);
-		level_tw<2, false, GLOBAL>(tw, LN - 2, 2 * o, w1);
+		level_tw<1, false>(tw, LN - 3, o, w0);
+		level_tw<2, false>(tw, LN - 2, 2 * o, w1);
 #pragma unroll
 		for (int i = 0; i < 4; ++i) fwd_bf(v[i], v[i + 4], w0[0].x, w0[0].y, p, p2);
 #pragma unroll
@@ -169,8 +158,8 @@ __device__ __forceinline__ void level_bottom(u32 * x, int mode, const LevelTw & 
 			continue;
 		}
 		pointwise4(v, y, mode == BOTTOM_MUL, w1[0], w1[1], p, p2, pinv);
-		level_tw<2, true, GLOBAL>(tw, LN - 2, 2 * o, w1);
-		level_tw<1, true, GLOBAL>(tw, LN - 3, o, w0);
+		level_tw<2, true>(tw, LN - 2, 2 * o, w1);
+		level_tw<1, true>(tw, LN - 3, o, w0);
 #pragma unroll
 		for (int i = 0; i < 2; ++i)
 		{
@@ -184,30 +173,28 @@ __device__ __forceinline__ void level_bottom(u32 * x, int mode, const LevelTw & 
 	}
 }
 
-// A whole transform step: the words at src (shared, padded, or global) through
-// all forward levels, the pointwise product and all inverse levels into dst,
-// working in x (shared).  src may be x, dst may be x.  The caller's barrier
-// makes src and the tables visible; on return the words of dst are written but
-// not yet ordered for other threads.
-template <int LN, bool GLOBAL, Where SRC, Where DST, typename Op, typename Out>
-__device__ __forceinline__ void level_transform(const u32 * src, u32 * x, u32 * dst, int mode, const LevelTw & tw, u32 tid, u32 NT,
+// A whole transform step: the words at src through all forward levels, the
+// pointwise product and all inverse levels into x.  The caller's barrier makes
+// src and the tables visible; on return the words of x are written but not yet
+// ordered for other threads.
+template <int LN, typename Op, typename Out>
+__device__ __forceinline__ void level_transform(const u32 * src, u32 * x, int mode, const LevelTw & tw, u32 tid, u32 NT,
 	u32 p, u32 pinv, Op op, Out out)
 {
 	const u32 p2 = 2 * p;
 	constexpr int REM = (LN - 3) % 3;
-	constexpr int TOP = (REM == 0) ? 3 : (REM == 1 && LN >= 13) ? 4 : REM, BT = LN - TOP;    // the top stage: bits BT..LN-1
-	level_stage<LN, TOP, BT, false, GLOBAL, SRC, IN_SHARED>(src, x, tw, tid, NT, p, p2);
+	constexpr int TOP = (REM == 0) ? 3 : REM, BT = LN - TOP;    // the top stage: bits BT..LN-1
+	static_assert(LN >= 6 && LN <= 12, "stages above bit 9 are the top one");
+	level_stage<LN, TOP, BT, false>(src, x, tw, tid, NT, p, p2);
 	__syncthreads();
-	if constexpr (BT >= 12) { level_stage<LN, 3, 9, false, GLOBAL, IN_SHARED, IN_SHARED>(x, x, tw, tid, NT, p, p2); __syncthreads(); }
-	if constexpr (BT >= 9) { level_stage<LN, 3, 6, false, GLOBAL, IN_SHARED, IN_SHARED>(x, x, tw, tid, NT, p, p2); __syncthreads(); }
-	if constexpr (BT >= 6) { level_stage<LN, 3, 3, false, GLOBAL, IN_SHARED, IN_SHARED>(x, x, tw, tid, NT, p, p2); __syncthreads(); }
-	level_bottom<LN, GLOBAL>(x, mode, tw, tid, NT, p, p2, pinv, op, out);
+	if constexpr (BT >= 9) { level_stage<LN, 3, 6, false>(x, x, tw, tid, NT, p, p2); __syncthreads(); }
+	if constexpr (BT >= 6) { level_stage<LN, 3, 3, false>(x, x, tw, tid, NT, p, p2); __syncthreads(); }
+	level_bottom<LN>(x, mode, tw, tid, NT, p, p2, pinv, op, out);
 	if (mode == BOTTOM_FORWARD) return;
 	__syncthreads();
-	if constexpr (BT >= 6) { level_stage<LN, 3, 3, true, GLOBAL, IN_SHARED, IN_SHARED>(x, x, tw, tid, NT, p, p2); __syncthreads(); }
-	if constexpr (BT >= 9) { level_stage<LN, 3, 6, true, GLOBAL, IN_SHARED, IN_SHARED>(x, x, tw, tid, NT, p, p2); __syncthreads(); }
-	if constexpr (BT >= 12) { level_stage<LN, 3, 9, true, GLOBAL, IN_SHARED, IN_SHARED>(x, x, tw, tid, NT, p, p2); __syncthreads(); }
-	level_stage<LN, TOP, BT, true, GLOBAL, IN_SHARED, DST>(x, dst, tw, tid, NT, p, p2);
+	if constexpr (BT >= 6) { level_stage<LN, 3, 3, true>(x, x, tw, tid, NT, p, p2); __syncthreads(); }
+	if constexpr (BT >= 9) { level_stage<LN, 3, 6, true>(x, x, tw, tid, NT, p, p2); __syncthreads(); }
+	level_stage<LN, TOP, BT, true>(x, x, tw, tid, NT, p, p2);
 }
 
 } // namespace ab

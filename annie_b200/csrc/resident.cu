@@ -96,7 +96,7 @@ __device__ __forceinline__ void res_transform(const u32 * xb, u32 * xa, u32 * op
 {
 	uint4 * const q = reinterpret_cast<uint4 *>(op);
 	constexpr u32 N8 = (1u << LN) / 8;
-	level_transform<LN, false, IN_SHARED, IN_SHARED>(xb, xa, xa, mode, tw, threadIdx.x, blockDim.x, p, pinv,
+	level_transform<LN>(xb, xa, mode, tw, threadIdx.x, blockDim.x, p, pinv,
 		[&](u32 o, uint4 & a, uint4 & b) { a = q[o]; b = q[N8 + o]; },
 		[&](u32 o, uint4 a, uint4 b) { q[o] = a; q[N8 + o] = b; });
 }
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(ResCfg<LN, K>::NT, SOLO ? 1 : ResCfg<LN, K>::M
 		w[i] = __ldg(gw + i);
 		if (dom == 0) wi[i] = __ldg(J.wri + (size_t)k * (N / 2) + i);
 	}
-	const LevelTw tw{ w, (dom == 0) ? wi : w, 1u, 1u, dom != 0 };
+	const LevelTw tw{ w, wi, dom != 0 };
 	{
 		const uint4 * img = reinterpret_cast<const uint4 *>((dom == 0 ? J.nir : J.nq) + ot + (size_t)k * N);
 		uint4 * o4 = reinterpret_cast<uint4 *>(op);
