@@ -11,7 +11,10 @@
 // steps: six per squaring, where the row and column passes need six dependent
 // kernel launches and the L2 between them.  Those short launches cost 3 to
 // 5 us each whatever the length; the cluster's steps cost what their longest
-// dependency chain costs.
+// dependency chain costs.  B200, us per squaring, passes then / resident: 2,500
+// bits 22.6 / 5.9, 20k 25.3 / 7.3, 60k 33.3 / 10.0, 100k 28.5 / 12.1, 262k 34.7 /
+// 18.5 (the passes as they are now: 262k 21.9).  At 2^12 words a transform step
+// takes 7 k to 8 k clocks (multiplier floor 3.5 k) and a carry step 4.5 k.
 //
 // The arithmetic is that of the passes (kernels.cu): the same primes, twiddle
 // positions, products, CRT and carry rule, so the registers are the same.
