@@ -1,6 +1,6 @@
 // The carry of one group of 4 coefficients by 4 adjacent lanes, a lane per
 // coefficient (j = 0..3 its place).  One thread per group does the same with
-// fewer instructions (kernels.cu); the lanes shorten the chain of dependent
+// fewer instructions (columns.cuh); the lanes shorten the chain of dependent
 // ones to about a third, which is what bounds a launch too small to fill the
 // GPU.  All lanes of a warp call these together.
 #pragma once

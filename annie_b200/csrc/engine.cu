@@ -266,7 +266,7 @@ struct ab_transform
 	bool split = false;                  // without overlap: still one launch per domain
 	CandConst cand{};                    // digit size and sparse N, as on the device at d_cand
 	const CandConst * d_cand = nullptr;
-	bool resident = false;               // short length: runs of squarings in one launch (resident.cu)
+	bool resident = false;               // short length: runs of squarings in one launch (resident.cuh)
 	ab_params prm{};
 	int KP = 0;                          // transform primes
 	size_t n = 0;
@@ -901,7 +901,7 @@ struct ab_transform
 	}
 };
 
-// Slots of a batch up to which a chunk runs resident (resident.cu) and not as
+// Slots of a batch up to which a chunk runs resident (resident.cuh) and not as
 // passes.  Measured on B200, 64 squarings, us per step of the whole batch
 // (resident / passes with their best split): ln 9 (K = 3) 256 slots 36.1 / 58.6;
 // ln 10 (K = 5) 256 slots 87.9 / 107.8; ln 11 (K = 5) 32 slots 33.2 / 38.5, 64
@@ -943,7 +943,7 @@ struct ab_batch
 	int g_steps = 0;
 	bool g_sparse = false;             // gexec takes every N as sparse
 	uint64_t g_kernels = 0;
-	bool resident = false;             // short length: a chunk is one launch (resident.cu)
+	bool resident = false;             // short length: a chunk is one launch (resident.cuh)
 	int zl = 0;                        // slots the graph launches (grid.z): a power of two covering every live slot
 	uint64_t launches = 0;
 

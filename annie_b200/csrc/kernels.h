@@ -134,7 +134,7 @@ cudaError_t launch_fused_rowpass(const FusedRowPass * d, const TConst * tcs, u32
 cudaError_t launch_fused_colpass(const FusedColPass * d, const TConst * tcs, u32 ctas, size_t smem, cudaStream_t s);
 
 // Runs of squarings of short transforms (lengths up to 2^12), one launch for
-// the whole run: a thread-block cluster per candidate (resident.cu).
+// the whole run: a thread-block cluster per candidate (resident.cuh).
 struct ResJob
 {
 	u32 * reg;                 // normal-form register, replaced by the result of the last step

@@ -1,5 +1,5 @@
 // Butterfly levels of a transform of 2^LN words held in shared memory
-// (resident.cu).
+// (resident.cuh).
 //
 // 8 words per thread: stages of 3 levels, the top one taking the remainder,
 // and a bottom step of two levels, the pointwise product and two inverse

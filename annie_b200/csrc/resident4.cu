@@ -1,0 +1,12 @@
+// Resident runs of the classes with 4 reference primes.
+#include "resident.cuh"
+
+namespace ab
+{
+
+cudaError_t launch_resident4(const ResJob & J, const TConst & c, cudaStream_t s, int ncand, bool * fits)
+{
+	return resident_k<4, 2>(J, c, s, ncand, fits);
+}
+
+} // namespace ab
