@@ -87,7 +87,7 @@ __device__ __forceinline__ void inv_bf(u32 & x0, u32 & x1, u32 v, u32 vs, u32 p,
 struct TConst
 {
 	u32 p[AB_MAXKP], pinv[AB_MAXKP];
-	u32 enc[AB_MAXKP][3];                // s_k 2^(30 j) 2^32 mod p: encoding weights of a value's 30-bit pieces (encode_res)
+	u32 enc[AB_MAXKP][3];                // s_k 2^(32 j) 2^32 mod p: encoding weights of a value's limbs (encode_res)
 	u32 mk[AB_MAXKP][AB_MAXK];           // e_k M/p_k in radix 2^30, the top entry holding 32 bits (crt)
 	u32 mkh[AB_MAXKP];                   // bits above those 32
 	u32 negm[AB_MAXK], negmh;            // -M mod 2^(32 K) in the same form
@@ -298,27 +298,16 @@ __device__ __forceinline__ Big<L> sparse_product(const SparseN & s, u32 e, u32 n
 	return v;
 }
 
-// The 30-bit pieces of an exact value (three limbs, |v| < 2^91): v = a0 +
-// 2^30 a1 + 2^60 a2, a2 signed.
-struct Pieces
-{
-	u32 a0, a1;
-	i32 a2;
-};
-__device__ __forceinline__ Pieces split30(u32 d0, u32 d1, u32 d2)
-{
-	constexpr u32 M30 = (1u << 30) - 1;
-	return Pieces{ d0 & M30, __funnelshift_r(d0, d1, 30) & M30, (i32)__funnelshift_r(d1, d2, 28) };
-}
-
-// s_k v mod p_k in (0, 3p): one Montgomery reduction of the 64-bit sum of the
-// weighted pieces (its high word lies in (-p/2, p)).
-__device__ __forceinline__ u32 encode_res(const TConst & c, int k, const Pieces & a)
+// s_k v mod p_k in (0, 4p) for any exact value v (three limbs): one Montgomery
+// reduction of the 64-bit sum of the weighted limbs, the top one signed.  The
+// sign of s_k is chosen so that enc[0] + enc[1] + enc[2] / 2 <= 2p
+// (encode_weights), so the sum's high word lies in [-p/2, 2p).
+__device__ __forceinline__ u32 encode_res(const TConst & c, int k, u32 d0, u32 d1, u32 d2)
 {
 	const u32 p = c.p[k];
-	u64 s = (u64)a.a0 * c.enc[k][0];
-	s += (u64)a.a1 * c.enc[k][1];
-	s += (u64)((i64)a.a2 * (i32)c.enc[k][2]);
+	u64 s = (u64)d0 * c.enc[k][0];
+	s += (u64)d1 * c.enc[k][1];
+	s += (u64)((i64)(i32)d2 * (i32)c.enc[k][2]);
 	return (u32)(s >> 32) - __umulhi((u32)s * c.pinv[k], p) + 2 * p;
 }
 

@@ -256,19 +256,19 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 	// a group's exact values: normal form out, residues into the tile
 	const bool fwd = (J.out_fwd[0] != nullptr) || (J.out_fwd[1] != nullptr);
 	auto encode = [&](int row, int u4, const u32 (&x)[4][AB_NW]) {
-		Pieces a[4];
-#pragma unroll
-		for (int j = 0; j < 4; ++j) a[j] = split30(x[j][0], x[j][1], x[j][2]);
 #pragma unroll
 		for (int k = 0; k < KP; ++k)
-			*reinterpret_cast<uint4 *>(tile + k * PS + row * CW + 4 * u4) =
-				make_uint4(encode_res(c, k, a[0]), encode_res(c, k, a[1]), encode_res(c, k, a[2]), encode_res(c, k, a[3]));
+		{
+			u32 r[4];
+#pragma unroll
+			for (int j = 0; j < 4; ++j) r[j] = encode_res(c, k, x[j][0], x[j][1], x[j][2]);
+			*reinterpret_cast<uint4 *>(tile + k * PS + row * CW + 4 * u4) = make_uint4(r[0], r[1], r[2], r[3]);
+		}
 	};
 	// the same for the thread's own word of a WIDE tile
 	auto encode1 = [&](const u32 (&x)[AB_NW]) {
-		const Pieces a = split30(x[0], x[1], x[2]);
 #pragma unroll
-		for (int k = 0; k < KP; ++k) tile[k * PS + tid] = encode_res(c, k, a);
+		for (int k = 0; k < KP; ++k) tile[k * PS + tid] = encode_res(c, k, x[0], x[1], x[2]);
 	};
 	auto finalize = [&](int row, int u4, const u32 (&x)[4][AB_NW]) {
 		const size_t o = (size_t)row * R + gcol(4 * u4);

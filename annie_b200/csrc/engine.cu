@@ -332,13 +332,15 @@ struct ab_transform
 		mpz_clears(N, factor, nullptr);
 	}
 
-	// The weights of encode_res for prime k and image factor s: s 2^(30 j), times
-	// 2^32 for its Montgomery reduction.
-	static void encode_weights(TConst & tc, int k, u32 s)
+	// The weights of encode_res for prime k and image factor s: s 2^(32 j), times
+	// 2^32 for its Montgomery reduction.  Returns whether they are in its range
+	// (of s and -s, one is: their sums add up to 2.5 p).
+	static bool encode_weights(TConst & tc, int k, u32 s)
 	{
 		const TZp z(TPRIMES[k]);
-		u32 x = z.mul(s, (u32)(((u64)1 << 32) % z.p));
-		for (int j = 0; j < 3; ++j) { tc.enc[k][j] = x; x = z.mul(x, (u32)(((u64)1 << 30) % z.p)); }
+		const u32 c32 = (u32)(((u64)1 << 32) % z.p);
+		for (int j = 0; j < 3; ++j) tc.enc[k][j] = s = z.mul(s, c32);
+		return (u64)2 * tc.enc[k][0] + (u64)2 * tc.enc[k][1] + tc.enc[k][2] <= (u64)4 * z.p;
 	}
 
 	// Constants of the transform primes (TConst) and of the reference primes
@@ -378,7 +380,8 @@ struct ab_transform
 			const u32 cw = z.mul(z.mul(z.inv((u32)((n / 2) % p)), (u32)(((u64)1 << 32) % p)), z.inv((u32)mpz_fdiv_ui(Mk, p)));
 			u32 e = 1;
 			while (!z.is_square(z.mul(cw, z.inv(e)))) ++e;
-			encode_weights(tc, k, z.sqrt(z.mul(cw, z.inv(e))));
+			const u32 s = z.sqrt(z.mul(cw, z.inv(e)));
+			if (!encode_weights(tc, k, s) && !encode_weights(tc, k, p - s)) throw ab_error(AB_E_ARG, "encoding weights out of range");
 			mpz_mul_ui(Mk, Mk, e);
 			columns(Mk, tc.mk[k], tc.mkh[k]);
 			// the top column of the CRT sum must fit 64 bits, and its operands 32
@@ -1452,7 +1455,8 @@ int ab_diag_forward(ab_transform * h, int domain, const uint32_t * in, uint32_t 
 		if (!h->import_words(T::TMP)) throw ab_error(AB_E_ARG, "input is not a normal-form register");
 		// plain residues: the engine's own images carry a factor per prime
 		const TConst scaled = h->tc;
-		for (int k = 0; k < h->KP; ++k) T::encode_weights(h->tc, k, 1u);
+		for (int k = 0; k < h->KP; ++k)
+			if (!T::encode_weights(h->tc, k, 1u)) { h->tc = scaled; throw ab_error(AB_E_ARG, "encoding weights out of range"); }
 		try
 		{
 			if (domain) h->full_forward(h->b(T::TMP), h->b(T::AQ1), nullptr);

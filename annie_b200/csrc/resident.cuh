@@ -269,8 +269,8 @@ __global__ void __launch_bounds__(ResCfg<LN, K>::NT, SOLO ? 1 : ResCfg<LN, K>::M
 		{
 			const uint4 a = s0[i], b = s1[i], d = s2[i];
 			*reinterpret_cast<uint4 *>(xb + rpad(4 * i)) = make_uint4(
-				encode_res(c, (int)k, split30(a.x, b.x, d.x)), encode_res(c, (int)k, split30(a.y, b.y, d.y)),
-				encode_res(c, (int)k, split30(a.z, b.z, d.z)), encode_res(c, (int)k, split30(a.w, b.w, d.w)));
+				encode_res(c, (int)k, a.x, b.x, d.x), encode_res(c, (int)k, a.y, b.y, d.y),
+				encode_res(c, (int)k, a.z, b.z, d.z), encode_res(c, (int)k, a.w, b.w, d.w));
 		}
 	};
 	if (J.y != nullptr)
@@ -296,12 +296,11 @@ __global__ void __launch_bounds__(ResCfg<LN, K>::NT, SOLO ? 1 : ResCfg<LN, K>::M
 	const u32 q0 = (rank - dom * KP) * Cfg::Q2, qn = (q0 >= G) ? 0u : (G - q0 < Cfg::Q2) ? G - q0 : Cfg::Q2;
 	// residues of a coefficient into the CTAs of domain d
 	auto scatter = [&](const u32 (&x)[AB_NW], u32 e, bool r_dom, bool q_dom) {
-		const Pieces a = split30(x[0], x[1], x[2]);
 		const u32 o = (u32)sizeof(u32) * rpad(e);
 #pragma unroll
 		for (int q = 0; q < KP; ++q)
 		{
-			const u32 v = encode_res(c, q, a);
+			const u32 v = encode_res(c, q, x[0], x[1], x[2]);
 			if (r_dom) st_remote(remote(xb, (u32)q) + o, v);
 			if (q_dom) st_remote(remote(xb, (u32)(KP + q)) + o, v);
 		}
