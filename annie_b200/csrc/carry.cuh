@@ -36,30 +36,51 @@ __device__ __forceinline__ void lane_digits(Big<L> & f, const Width & w, u32 j, 
 	split_digit<FULL, L, ND>(f, w, d);
 }
 
+// Limbs that hold every sum of phase 2.  The carry into the second coefficient
+// of a group is below 2^(32 L - 1 - 2 W) in magnitude: with FULL (W >= 32 (ND - 1))
+// below 2^63, so two limbs pass it on and three hold the sums; other digit sizes
+// take all L.
+template <bool FULL, int L>
+struct CarryLimbs
+{
+	static constexpr int N = (FULL || L < AB_NW) ? AB_NW : L, PASS = FULL ? 2 : N;
+};
+
+// v as a sum of phase 2 (sign-extended)
+template <int CL, int L>
+__device__ __forceinline__ Big<CL> carry_extend(const Big<L> & v)
+{
+	Big<CL> r;
+#pragma unroll
+	for (int i = 0; i < CL; ++i) r.l[i] = (i < L) ? v.l[i % L] : (u32)((i32)v.l[L - 1] >> 31);
+	return r;
+}
+
 // Phase 2: cin = the previous group's carry-out (lane 0; 0 in the others), d =
 // the digits; x = the exact value: balanced in lanes 0..2, lane 3 absorbs the
-// rest.  half: 2^(W-1).  Past lane 0 the carry is below 2^55, two limbs.
+// rest.  half: 2^(W-1).
 template <bool FULL, int L, int ND>
 __device__ __forceinline__ void lane_balance(const Big<L> & cin, const u32 (&d)[ND], const Width & w, const Big<AB_NW> & half, u32 j, u32 (&x)[AB_NW])
 {
+	constexpr int CL = CarryLimbs<FULL, L>::N;
 	u32 hd[ND], dd[ND];
 #pragma unroll
 	for (int i = 0; i < ND; ++i) hd[i] = half.l[i];
 	Big<L> v = add_digit<L, ND>(add_digit<L, ND>(cin, d), hd);
 	split_digit<FULL, L, ND>(v, w, dd);
-	Big<AB_NW> c, t;
+	Big<CL> c = carry_extend<CL, L>(v), t;
 #pragma unroll
-	for (int i = 0; i < AB_NW; ++i) { c.l[i] = (i < L) ? v.l[i % L] : (u32)((i32)v.l[L - 1] >> 31); t.l[i] = (i < ND) ? d[i % ND] : 0u; }
+	for (int i = 0; i < CL; ++i) t.l[i] = (i < ND) ? d[i % ND] : 0u;
 #pragma unroll
 	for (int r = 1; r < 4; ++r)
 	{
-		const Big<AB_NW> up = shfl_up4<AB_NW, 2>(c);
-		if (j == (u32)r) t = big_add<AB_NW>(t, up);
+		const Big<CL> up = shfl_up4<CL, CarryLimbs<FULL, L>::PASS>(c);
+		if (j == (u32)r) t = big_add<CL>(t, up);
 		if (r < 3)
 		{
 			u32 e[ND];
-			c = big_add<AB_NW>(t, half);
-			split_digit<FULL, AB_NW, ND>(c, w, e);
+			c = add_digit<CL, ND>(t, hd);
+			split_digit<FULL, CL, ND>(c, w, e);
 			if (j == (u32)r)
 			{
 #pragma unroll

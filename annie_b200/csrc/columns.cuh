@@ -149,17 +149,17 @@ __device__ __forceinline__ void exact_add(u32 (&x)[AB_NW], __int128 d)
 // Second carry phase for one group of 4 coefficients (kernel.cl:1582-1613):
 // f = carry-in, d = the group's unsigned W-bit digits.  The first three become
 // balanced, v in [-2^(W-1), 2^(W-1)) with the carry (f + d + 2^(W-1)) >> W;
-// the last one absorbs the rest.  x: exact values (three limbs each).  After
-// the first step the carry is below 2^55, so three limbs hold every sum.
+// the last one absorbs the rest.  x: exact values (three limbs each); the sums
+// past the first have CarryLimbs limbs.
 template <bool FULL, int L, int PCK>
 __device__ __forceinline__ void carry_phase2(const Width & w, const Big<AB_NW> & half, const Big<L> & f, const u32 (&d)[4][DigitLimbs<PCK>::N],
 	u32 (&x)[4][AB_NW])
 {
-	constexpr int ND = DigitLimbs<PCK>::N;
+	constexpr int ND = DigitLimbs<PCK>::N, CL = CarryLimbs<FULL, L>::N;
 	u32 hd[ND];
 #pragma unroll
 	for (int i = 0; i < ND; ++i) hd[i] = half.l[i];
-	Big<AB_NW> g;
+	Big<CL> g;
 	auto balanced = [&](const u32 (&e)[ND], u32 (&v)[AB_NW]) {
 		Big<AB_NW> a;
 #pragma unroll
@@ -170,22 +170,20 @@ __device__ __forceinline__ void carry_phase2(const Width & w, const Big<AB_NW> &
 	};
 	{
 		Big<L> t = add_digit<L, ND>(add_digit<L, ND>(f, d[0]), hd);
-		const u32 s = (u32)((i32)t.l[L - 1] >> 31);
 		u32 e[ND];
 		split_digit<FULL, L, ND>(t, w, e);
 		balanced(e, x[0]);
-#pragma unroll
-		for (int i = 0; i < AB_NW; ++i) g.l[i] = (i < L) ? t.l[i % L] : s;
+		g = carry_extend<CL, L>(t);
 	}
 #pragma unroll
 	for (int j = 1; j < 3; ++j)
 	{
-		g = add_digit<AB_NW, ND>(add_digit<AB_NW, ND>(g, d[j]), hd);
+		g = add_digit<CL, ND>(add_digit<CL, ND>(g, d[j]), hd);
 		u32 e[ND];
-		split_digit<FULL, AB_NW, ND>(g, w, e);
+		split_digit<FULL, CL, ND>(g, w, e);
 		balanced(e, x[j]);
 	}
-	g = add_digit<AB_NW, ND>(g, d[3]);
+	g = add_digit<CL, ND>(g, d[3]);
 #pragma unroll
 	for (int i = 0; i < AB_NW; ++i) x[3][i] = g.l[i];
 }
