@@ -615,9 +615,10 @@ struct ab_transform
 		}
 	}
 
-	void prefwd_reg0()
+	// want_q: the caller takes AQ0 as it is, so a pending one is computed too
+	void prefwd_reg0(bool want_q = false)
 	{
-		if (!prefwd) { ColJob j = cj_norm(b(REG0)); set_fwd(j, b(AQ0), b(AR0)); cols(j); q_pending = false; }
+		if (!prefwd || (want_q && q_pending)) { ColJob j = cj_norm(b(REG0)); set_fwd(j, b(AQ0), b(AR0)); cols(j); q_pending = false; }
 	}
 
 	// `steps` squarings (multiplier a where bit s of bits is set, else 1) of the
@@ -655,6 +656,9 @@ struct ab_transform
 				CK(cudaEventRecord(mult_done[i], st));
 			}
 		}
+		// AR0, and AQ0 unless the graph's first step computes it (before the
+		// capture, which runs through the marks of a squaring)
+		prefwd_reg0(!overlap);
 		if (gexec == nullptr)
 		{
 			RowJobs rjs{}; ColJobs cjs{};
@@ -679,7 +683,6 @@ struct ab_transform
 			cudaGraphDestroy(g);
 			CK(ei);
 		}
-		prefwd_reg0();                           // AR0 (and AQ0, recomputed by the graph's first step)
 		const int hi = mult_i;
 		CK(cudaEventSynchronize(mult_done[hi]));
 		std::memcpy(h_mult[hi], mults, G * sizeof(u32));
