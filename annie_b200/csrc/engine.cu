@@ -573,7 +573,7 @@ struct ab_transform
 		const bool q_chain = overlap || split;   // the Q chain has launches of its own
 		if (want_prefwd) set_fwd(j2, q_chain ? nullptr : b(AQ0), b(AR0));
 		cols(j2);
-		q_pending = want_prefwd && q_chain;
+		if (want_prefwd) q_pending = q_chain;    // else AR0 and AQ0 are left as they are
 	}
 
 	// First product of squareMMGW / mulMMGW (transformGPU.h:540-568):

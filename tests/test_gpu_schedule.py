@@ -61,3 +61,22 @@ def test_overlap_switched_between_squarings(K, lbase):
     t.square_mul(3)
     t.square_mul_bits(bits, 64, 3)
     assert np.array_equal(got, t.read_register(0)), "profiled step"
+
+
+@pytest.mark.parametrize("overlap", [True, False])
+@pytest.mark.parametrize("K,lbase", [(2, 14), (4, 27), (5, 17)])
+def test_get_between_squarings(K, lbase, overlap):
+    # reading a register, by value or by its words, leaves the next squaring alone
+    params = (K, PCK[K], 13, lbase)
+    N = _number(params, K + 10)
+    t = A.Transform(N, 3, params=params)
+    t.set_overlap(overlap)
+    t.set1()
+    t.copy(1, 0)
+    e = 0
+    for i, a in enumerate((3, 1, 3, 3, 1)):
+        t.square_mul(a)
+        e = 2 * e + (a == 3)
+        t.get(i % 2)
+        t.read_register(0)
+    assert t.get(0) == pow(3, e, N)
