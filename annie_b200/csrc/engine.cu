@@ -702,14 +702,15 @@ struct ab_transform
 		apply_geometry(tc, g);
 	}
 
-	// row/column split of the transform (the register layouts do not depend on it)
+	// row/column split of the transform (the register layouts do not depend on
+	// it); 0: the default split, and resident runs where the length has them
 	void set_geometry(int lb)
 	{
 		Geometry g;
 		if (!make_geometry(prm.ln, lb, g)) throw ab_error(AB_E_ARG, "geometry not available for this length");
 		CK(cudaStreamSynchronize(st));
 		use_geometry(g);
-		resident = false;                        // the caller wants the passes, with this split
+		resident = (lb <= 0) && resident_fits(tc);   // a split of the caller's is for the passes
 		prefwd = false;                          // AQ0/AR0 hold levels of the old split
 		if (gexec) { cudaGraphExecDestroy(gexec); gexec = nullptr; }
 	}
@@ -1881,9 +1882,9 @@ int ab_batch_set_geometry(ab_batch * b, int lb)
 		CK(cudaStreamSynchronize(b->st));
 		b->geo = g;
 		++b->geo_version;
-		b->resident = false;                     // the caller wants the passes, with this split
 		apply_geometry(b->tc, g);
-		for (ab_transform * v : b->views) if (v) { v->use_geometry(g); v->resident = false; v->prefwd = false; }
+		b->resident = (lb <= 0) && resident_fits(b->tc);   // a split of the caller's is for the passes
+		for (ab_transform * v : b->views) if (v) { v->use_geometry(g); v->resident = b->resident; v->prefwd = false; }
 		RowJobs rjs{}; ColJobs cjs{};
 		CK(launch_rowpass(b->geo, b->tc, rjs, 1, b->st, 0));
 		CK(launch_colpass(b->geo, b->tc, cjs, 1, b->st, 0));

@@ -107,8 +107,9 @@ int ab_square_mul_bits(ab_transform * h, const uint64_t * bits, size_t count, in
    contents are kept.  The reference fixes its split per length at compile
    time (transformGPU.h:403-470, forward/backward kernel choice); here it is
    a run-time choice for the autotuner.  A handle of length up to 2^12 that has
-   been given a split squares by the row and column passes.  AB_E_ARG if the
-   split is not available for the length. */
+   been given a split squares by the row and column passes; row_levels = 0
+   restores the default split, and with it the one-launch runs of those lengths.
+   AB_E_ARG if the split is not available for the length. */
 int ab_set_geometry(ab_transform * h, int row_levels);
 int ab_get_geometry(const ab_transform * h, int * row_levels, int * col_levels);
 

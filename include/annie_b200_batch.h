@@ -67,7 +67,9 @@ int ab_batch_steps(ab_batch * b, int steps, const uint32_t * mult, const uint8_t
    flight), 0 when it would wait, < 0 on error. */
 int ab_batch_ready(const ab_batch * b);
 int ab_batch_gl_mul(ab_batch * b, int slot);
-/* Row levels per row pass (0 = default split); used by the autotuner. */
+/* Row levels per row pass.  A batch of length up to 2^12 that has been given a
+   split squares by the row and column passes; 0 restores the default split, and
+   with it the one-launch chunks of those lengths. */
 int ab_batch_set_geometry(ab_batch * b, int lb);
 /* Autotuner: times `steps` batched squarings for every admissible row/column
    split of the class, with copies of slot `src` in the empty slots (released

@@ -80,3 +80,51 @@ def test_get_between_squarings(K, lbase, overlap):
         t.get(i % 2)
         t.read_register(0)
     assert t.get(0) == pow(3, e, N)
+
+
+@pytest.mark.parametrize("bits", [2450, 60000, 262144])
+def test_default_split_restores_resident_runs(bits):
+    rng = Xoshiro256ss(bits)
+    N = rng.random_odd(bits)
+    while A.probe(N, 3)[1]:
+        N = rng.random_odd(bits)
+    t = A.Transform(N, 3)
+    split = t.geometry()
+
+    def launches(f):
+        l0 = t.launch_count()
+        f()
+        return t.launch_count() - l0
+
+    def step():
+        t.square_mul_bits(5, 16, 3)
+    t.set1()
+    assert launches(step) == 1
+    t.set_geometry(split[0])
+    passes = launches(step)
+    assert passes > 1
+    t.set_geometry(0)
+    assert t.geometry() == split and launches(step) == 1
+    t.set1()
+    for _ in range(3):
+        step()
+    exp = t.read_register(0)
+
+    b = A.Batch((t.K, t.pck, t.ln, t.lbase), capacity=2, max_steps=16)
+    assert not b.load(0, N, 3)
+    b.slot(0).set1()
+    m = np.array([[3 if (5 >> i) & 1 else 1, 0] for i in range(16)], dtype=np.uint32)
+    counts = []
+    for lb in (None, split[0], 0):
+        if lb is not None:
+            b.set_geometry(lb)
+        l0 = b.launch_count()
+        b.steps(m)
+        counts.append(b.launch_count() - l0)
+    assert counts[0] == counts[2] == 1 and counts[1] > 1
+    assert np.array_equal(b.slot(0).read_register(0), exp)
+    # the slot's own view squares resident again too
+    v = b.slot(0)
+    l0 = v.launch_count()
+    v.square_mul_bits(5, 16, 3)
+    assert v.launch_count() - l0 == 1
