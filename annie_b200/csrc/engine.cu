@@ -628,6 +628,7 @@ struct ab_transform
 		ResJob j; std::memset(&j, 0, sizeof(j));
 		j.reg = x; j.y = y; j.nir = b(NIR); j.nq = b(NQ); j.wr = wf(false); j.wri = wv(false); j.wq = wf(true);
 		j.steps = steps; j.bits = bits; j.a = a; j.cand = d_cand;
+		mark();
 		CK(launch_resident(j, tc, st));
 		++launches;
 	}
@@ -635,7 +636,7 @@ struct ab_transform
 	// squareMMGW (transformGPU.h:556-568)
 	void square_mul(u32 a)
 	{
-		if (resident && !split) { run_resident(b(REG0), nullptr, 1, 1, a); prefwd = false; return; }
+		if (resident) { run_resident(b(REG0), nullptr, 1, 1, a); prefwd = false; return; }
 		prefwd_reg0();
 		first_product(a, nullptr, nullptr, nullptr, q_pending);
 		reduce_tail(b(TQ), b(REG0), true, overlap);

@@ -132,7 +132,7 @@ int ab_launch_count(const ab_transform * h, uint64_t * count);
    returns each launch's device time (ms, launch order) in ms[0..*count).
    The launches are those of the overlapped schedule (one per domain: row
    and column pass of Q, of R, then the reduction), serialised on one
-   stream so that each is timed alone. */
+   stream so that each is timed alone; or the one launch of a short length. */
 int ab_profile_square(ab_transform * h, int32_t a, float * ms, int cap, int * count);
 
 /* Overwrites a device buffer of `bytes` (allocated on first use) on the

@@ -128,3 +128,24 @@ def test_default_split_restores_resident_runs(bits):
     l0 = v.launch_count()
     v.square_mul_bits(5, 16, 3)
     assert v.launch_count() - l0 == 1
+
+
+@pytest.mark.parametrize("bits,resident", [(20000, True), (262144, True), (400000, False)])
+def test_profile_times_the_launches_of_a_squaring(bits, resident):
+    rng = Xoshiro256ss(bits + 1)
+    N = rng.random_odd(bits)
+    while A.probe(N, 3)[1]:
+        N = rng.random_odd(bits)
+    t, u = A.Transform(N, 3), A.Transform(N, 3)
+    for x in (t, u):
+        x.set1()
+        x.square_mul(3)
+    ms = t.profile_square(3)
+    l0 = u.launch_count()
+    u.square_mul(3)
+    assert len(ms) == u.launch_count() - l0 and (len(ms) == 1) == resident
+    assert all(0.0 < x < 5.0 for x in ms)
+    assert np.array_equal(t.read_register(0), u.read_register(0))
+    # a handle that was given a split is profiled by its passes
+    t.set_geometry(t.geometry()[0])
+    assert len(t.profile_square(3)) > 1
