@@ -1893,11 +1893,12 @@ int ab_batch_set_geometry(ab_batch * b, int lb)
 	});
 }
 
-// Splits chosen by ab_batch_autotune in this process, by (K, ln, capacity).
+// Splits chosen by ab_batch_autotune in this process, by (K, ln, capacity) and
+// the schedule they were timed with (all N sparse: no product by N).
 namespace
 {
 std::mutex g_tune_mu;
-std::map<std::tuple<int, int, int>, int> g_tuned;
+std::map<std::tuple<int, int, int, bool>, int> g_tuned;
 
 void ok_or_throw(int rc) { if (rc != AB_OK) throw ab_error(rc, ab_last_error()); }
 }
@@ -1907,7 +1908,7 @@ int ab_batch_autotune(ab_batch * b, int src, int steps, int * row_levels)
 	return guarded([&] {
 		if (b == nullptr || src < 0 || src >= b->cap || b->views[src] == nullptr || b->views[src]->failed || steps < 1 || steps > b->max_steps)
 			throw ab_error(AB_E_ARG, "bad arguments");
-		const auto key = std::make_tuple(b->cls.K, b->cls.ln, b->cap);
+		const auto key = std::make_tuple(b->cls.K, b->cls.ln, b->cap, b->all_sparse());
 		int best = 0;
 		{
 			std::lock_guard<std::mutex> lock(g_tune_mu);

@@ -74,8 +74,10 @@ int ab_batch_set_geometry(ab_batch * b, int lb);
 /* Autotuner: times `steps` batched squarings for every admissible row/column
    split of the class, with copies of slot `src` in the empty slots (released
    afterwards; the loaded slots are not touched), keeps the fastest split and
-   remembers it for the process by (K, ln, capacity).  The reference picks its
-   kernel split per length at compile time (transformGPU.h:403-470). */
+   remembers it for the process by (K, ln, capacity) and whether every loaded N
+   is sparse (k 2^m + 1: a shorter squaring).  A batch whose chunks are always one
+   launch keeps its split.  The reference picks its kernel split per length at
+   compile time (transformGPU.h:403-470). */
 int ab_batch_autotune(ab_batch * b, int src, int steps, int * row_levels);
 int ab_batch_synchronize(ab_batch * b);
 int ab_batch_launch_count(const ab_batch * b, uint64_t * count);

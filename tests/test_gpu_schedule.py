@@ -149,3 +149,36 @@ def test_profile_times_the_launches_of_a_squaring(bits, resident):
     # a handle that was given a split is profiled by its passes
     t.set_geometry(t.geometry()[0])
     assert len(t.profile_square(3)) > 1
+
+
+def _numbers(bits):
+    """A dense N and a sparse one (k 2^m + 1) of one class."""
+    rng = Xoshiro256ss(bits)
+
+    def number(draw):
+        while True:
+            N = draw()
+            if not A.probe(N, 3)[1]:
+                return N
+    dense = number(lambda: rng.random_odd(bits))
+    sparse = number(lambda: proth(rng.uniform(1 << 19, 1 << 20) | 1, bits - 20))
+    assert A.probe(dense, 3)[0][:3] == A.probe(sparse, 3)[0][:3]
+    return dense, sparse
+
+
+def test_remembered_split_is_that_of_the_schedule():
+    # a split tuned with sparse N (a squaring without the last product's
+    # transform) is not taken for dense N, and the reverse
+    cap, steps = 7, 4
+    numbers = _numbers(500020)
+    tuned = []
+    for i in (1, 0, 1, 0):
+        b = A.Batch(A.probe(numbers[i], 3)[0], capacity=cap, max_steps=steps)
+        assert not b.load(0, numbers[i], 3)
+        b.slot(0).set1()
+        lb = b.autotune(0, steps)
+        assert lb == b.slot(0).geometry()[0]
+        tuned.append((b.launch_count() > 0, lb))
+        b.close()
+    assert [x[0] for x in tuned] == [True, True, False, False]
+    assert tuned[0][1] == tuned[2][1] and tuned[1][1] == tuned[3][1]
