@@ -947,18 +947,22 @@ struct ab_batch
 	int ctrl_i = 0;
 	cudaEvent_t chunk_done = nullptr;  // the last chunk has completed
 	std::vector<ab_transform *> views;
-	cudaGraphExec_t gexec = nullptr;
-	int g_steps = 0;
-	bool g_sparse = false;             // gexec takes every N as sparse
-	uint64_t g_kernels = 0;
+	// the captured chunk of each schedule: N of any form, all N sparse
+	struct ChunkGraph
+	{
+		cudaGraphExec_t exec = nullptr;
+		int steps = 0, zl = 0;
+		uint64_t kernels = 0;
+		void drop() { if (exec) { cudaGraphExecDestroy(exec); exec = nullptr; } }
+	} graphs[2];
 	bool resident = false;             // short length: a chunk is one launch (resident.cuh)
-	int zl = 0;                        // slots the graph launches (grid.z): a power of two covering every live slot
+	int zl = 0;                        // slots that rows()/cols() launch (grid.z): a power of two covering every live slot
 	uint64_t launches = 0;
 
 	~ab_batch()
 	{
 		for (ab_transform * v : views) delete v;
-		if (gexec) cudaGraphExecDestroy(gexec);
+		for (ChunkGraph & g : graphs) g.drop();
 		if (mem) cudaFree(mem);
 		if (d_cand) cudaFree(d_cand);
 		if (d_ctrl) cudaFree(d_ctrl);
@@ -1850,9 +1854,10 @@ int ab_batch_steps(ab_batch * b, int steps, const uint32_t * mult, const uint8_t
 			return;
 		}
 		const bool sparse = b->all_sparse();
-		if (b->gexec == nullptr || b->g_steps != steps || b->zl != zl || b->g_sparse != sparse)
+		ab_batch::ChunkGraph & cg = b->graphs[sparse ? 1 : 0];
+		if (cg.exec == nullptr || cg.steps != steps || cg.zl != zl)
 		{
-			if (b->gexec) { cudaGraphExecDestroy(b->gexec); b->gexec = nullptr; }
+			cg.drop();
 			b->zl = zl;
 			cudaGraph_t g = nullptr;
 			b->recorded = 0;
@@ -1860,16 +1865,16 @@ int ab_batch_steps(ab_batch * b, int steps, const uint32_t * mult, const uint8_t
 			try { b->record_steps(steps, sparse); }
 			catch (...) { cudaStreamEndCapture(b->st, &g); if (g) cudaGraphDestroy(g); throw; }
 			CK(cudaStreamEndCapture(b->st, &g));
-			const cudaError_t e = cudaGraphInstantiate(&b->gexec, g, 0);
+			const cudaError_t e = cudaGraphInstantiate(&cg.exec, g, 0);
 			cudaGraphDestroy(g);
 			CK(e);
-			b->g_steps = steps;
-			b->g_sparse = sparse;
-			b->g_kernels = b->recorded;
+			cg.steps = steps;
+			cg.zl = zl;
+			cg.kernels = b->recorded;
 		}
-		CK(cudaGraphLaunch(b->gexec, b->st));
+		CK(cudaGraphLaunch(cg.exec, b->st));
 		CK(cudaEventRecord(b->chunk_done, b->st));
-		b->launches += b->g_kernels;                  // kernels of the graph
+		b->launches += cg.kernels;                    // kernels of the graph
 		for (ab_transform * v : b->views) if (v) v->prefwd = false;
 	});
 }
@@ -1889,7 +1894,7 @@ int ab_batch_set_geometry(ab_batch * b, int lb)
 		RowJobs rjs{}; ColJobs cjs{};
 		CK(launch_rowpass(b->geo, b->tc, rjs, 1, b->st, 0));
 		CK(launch_colpass(b->geo, b->tc, cjs, 1, b->st, 0));
-		if (b->gexec) { cudaGraphExecDestroy(b->gexec); b->gexec = nullptr; }
+		for (ab_batch::ChunkGraph & cg : b->graphs) cg.drop();
 	});
 }
 

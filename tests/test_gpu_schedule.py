@@ -1,5 +1,7 @@
 """Calls that change a handle's or a batch's schedule between squarings: the
 registers do not depend on them, and the default path comes back."""
+import time
+
 import numpy as np
 import pytest
 
@@ -182,3 +184,34 @@ def test_remembered_split_is_that_of_the_schedule():
         b.close()
     assert [x[0] for x in tuned] == [True, True, False, False]
     assert tuned[0][1] == tuned[2][1] and tuned[1][1] == tuned[3][1]
+
+
+def test_schedules_of_a_batch_keep_their_graphs():
+    # a dense slot that comes and goes changes the batch's schedule; each
+    # schedule's graph is captured once
+    dense, sparse = _numbers(500020)
+    steps = 64
+    b = A.Batch(A.probe(sparse, 3)[0], capacity=2, max_steps=steps)
+    t = A.Transform(sparse, 3)
+    t.set1()
+    assert not b.load(0, sparse, 3)
+    b.slot(0).set1()
+    m = np.zeros((steps, 2), dtype=np.uint32)
+    m[:, 0] = [3 if i % 3 == 0 else 1 for i in range(steps)]
+    bits = sum(1 << i for i in range(0, steps, 3))
+    cost = []
+    for i in range(16):
+        if i % 2:
+            assert not b.load(1, dense, 3)
+        else:
+            b.release(1)
+        b.synchronize()
+        t0 = time.perf_counter()
+        b.steps(m)
+        cost.append(time.perf_counter() - t0)
+        b.synchronize()
+        t.square_mul_bits(bits, steps, 3)
+    assert np.array_equal(b.slot(0).read_register(0), t.read_register(0))
+    # host time of a chunk: capturing 64 squarings against a launch
+    assert min(cost[2:]) < 0.5 * min(cost[:2]), cost
+    assert sorted(cost[2:])[len(cost[2:]) // 2] < 0.5 * min(cost[:2]), cost
