@@ -331,8 +331,9 @@ template <int PCK>
 struct DigitLimbs { static constexpr int N = (PCK == 1) ? 1 : (PCK == 2) ? 2 : 3; };
 
 // d = the low W bits of f (unsigned), f >>= W (arithmetic).  FULL: W reaches
-// into the last of the ND limbs (ws = ND - 1), as the parameter rule's digit
-// sizes do for every class; other (forced) sizes take the general form.
+// into the last of the ND limbs (ws = ND - 1), as the digit sizes of the
+// parameter rule do for bases up to 100; smaller sizes (larger bases, forced
+// parameters) take the general form.
 template <bool FULL, int L, int ND>
 __device__ __forceinline__ void split_digit(Big<L> & f, const Width & w, u32 (&d)[ND])
 {

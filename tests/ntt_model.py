@@ -1,11 +1,11 @@
 """Bit-exact numpy model of the engine's own transform arithmetic (not the
 reference's): the transform primes, the Shoup twiddle tables, the lazily
-reduced butterflies, the Montgomery pointwise product and the CRT with its
-fixed-point quotient estimate, level by level.  Every element goes through the
-same operations in the same order as in the CUDA passes (only the grouping of
-butterflies into passes differs), so the model reproduces the device's lazy
-words; it is the reference for the forward-transform kernel test and, on the
-CPU, checks the design against exact big-integer convolutions.
+reduced butterflies, the summed Montgomery pointwise products, the image factors
+and the radix-2^30 CRT with its 32-bit quotient estimate, level by level.  Every
+element goes through the same operations in the same order as in the CUDA passes
+(only the grouping of butterflies into passes differs), so the model reproduces
+the device's lazy words; it is the reference for the forward-transform kernel test
+and, on the CPU, checks the design against exact big-integer convolutions.
 """
 import numpy as np
 
@@ -85,12 +85,13 @@ def shoup(x, w, ws, p):
     return _u(x * _u(w) - q * np.uint64(p))
 
 
-def mont(a, b, p):
+def redc(t, p, add=1):
+    """t 2^-32 mod p of a 64-bit sum: its high word less that of m p, plus `add` p."""
     pinv = pow(p, -1, 1 << 32)
-    t = _u(a) * _u(b)
+    t = np.asarray(t, dtype=np.uint64)
     lo, hi = t & np.uint64(M32), t >> np.uint64(32)
     m = _u(lo * np.uint64(pinv))
-    return _u(hi - ((m * np.uint64(p)) >> np.uint64(32)) + np.uint64(p))
+    return _u(hi - ((m * np.uint64(p)) >> np.uint64(32)) + np.uint64(add * p))
 
 
 def red2(x, p):
@@ -108,21 +109,22 @@ def exact_limbs(exact):
     return d0, d1, d2
 
 
-def encode(exact, k, limbs=None):
-    """Residues in [0, 3p) of exact values (python ints, |v| < 2^95), as the column pass."""
+def encode_weights(k, s=1):
+    """Weights of the three limbs for image factor s (encode_weights of the engine),
+    and whether they are in the encoder's range."""
+    p = TPRIMES[k]
+    w = [s * pow(2, 32 * (j + 1), p) % p for j in range(3)]
+    return w, 2 * w[0] + 2 * w[1] + w[2] <= 4 * p
+
+
+def encode(exact, k, limbs=None, s=1):
+    """Residues in (0, 4p) of s times exact values (python ints, 96 bits), as the column pass."""
     p = TPRIMES[k]
     d0, d1, d2 = exact_limbs(exact) if limbs is None else limbs
-    d2u = d2 ^ np.uint64(0x80000000)
-    one_s = (1 << 32) // p
-    a = _u(d0 - ((d0 * np.uint64(one_s)) >> np.uint64(32)) * np.uint64(p))
-    c32 = (1 << 32) % p
-    c64 = c32 * c32 % p
-    b = shoup(d1, c32, shoup_const(c32, p), p)
-    e = shoup(d2u, c64, shoup_const(c64, p), p)
-    s = red2(a + b, p)
-    s = red2(s + e, p)
-    k95 = (p - (c64 * ((1 << 31) % p)) % p) % p
-    return _u(s + np.uint64(k95))
+    w, ok = encode_weights(k, s)
+    assert ok
+    top = np.where(d2 >> np.uint64(31) != 0, d2 | np.uint64(M32 << 32), d2)   # sign-extended
+    return redc(d0 * np.uint64(w[0]) + d1 * np.uint64(w[1]) + top * np.uint64(w[2]), p, 2)
 
 
 def forward(x, ln, k, domain_q, reduce_out=False):
@@ -145,26 +147,27 @@ def forward(x, ln, k, domain_q, reduce_out=False):
     return red2(x, p) if reduce_out else x
 
 
+def poly_product(x0, x1, y0, y1, mul, cm, p):
+    """(x0 + x1 X)(y0 + y1 X) 2^-32 mod (X^2 - c), cm = c 2^32 mod p; words in [0, 2p)."""
+    x0, x1, y0, y1, cm = _u(x0), _u(x1), _u(y0), _u(y1), _u(cm)
+    t = redc(x1 * y1, p)
+    r0 = redc(x0 * y0 + t * cm, p)
+    r1 = redc(x0 * y1 + x1 * y0 if mul else (x0 + x0) * x1, p)
+    return red2(r0, p), red2(r1, p)
+
+
 def pointwise(x, ln, k, domain_q, y=None):
     """Degree-1 products mod (x^2 -+ c), c = w[n/4 + m/2] (Montgomery, outputs [0, 2p))."""
     p = TPRIMES[k]
-    w, ws, _, _ = tables(ln, k, domain_q)
+    _, ws, _, _ = tables(ln, k, domain_q)
     n = 1 << ln
     m = np.arange(n // 2)
-    c, cs = w[n // 4 + (m >> 1)], ws[n // 4 + (m >> 1)]
+    cm = _u(np.uint64(0) - ws[n // 4 + (m >> 1)] * np.uint64(p))     # w 2^32 mod p from its Shoup quotient
+    cm = np.where((m & 1) == 0, cm, np.uint64(p) - cm)
     x0, x1 = red2(x[0::2], p), red2(x[1::2], p)
-    if y is None:
-        t = shoup(mont(x1, x1, p), c, cs, p)
-        y1 = mont(red2(x0 + x0, p), x1, p)
-        y0 = mont(x0, x0, p)
-    else:
-        p0, p1 = _u(y[0::2]), _u(y[1::2])
-        t = shoup(mont(x1, p1, p), c, cs, p)
-        y1 = red2(mont(x0, p1, p) + mont(x1, p0, p), p)
-        y0 = mont(x0, p0, p)
-    y0 = np.where((m & 1) == 0, red2(y0 + t, p), red2(y0 - t + np.uint64(2 * p), p))
+    y0, y1 = (x0, x1) if y is None else (y[0::2], y[1::2])
     out = np.empty(n, dtype=np.uint64)
-    out[0::2], out[1::2] = y0, y1
+    out[0::2], out[1::2] = poly_product(x0, x1, y0, y1, y is not None, cm, p)
     return out
 
 
@@ -193,39 +196,109 @@ def inverse(x, ln, k, domain_q):
     return x
 
 
+def _sqrt(x, p):
+    """A square root of the square x mod p (Tonelli-Shanks, as the engine)."""
+    q, m = p - 1, 0
+    while q % 2 == 0:
+        q, m = q // 2, m + 1
+    g = 2
+    while pow(g, (p - 1) // 2, p) == 1:
+        g += 1
+    c, t, r = pow(g, q, p), pow(x, q, p), pow(x, (q + 1) // 2, p)
+    while t != 1:
+        i, y = 0, t
+        while y != 1:
+            i, y = i + 1, y * y % p
+        b = pow(c, 1 << (m - i - 1), p)
+        m, c = i, b * b % p
+        t, r = t * c % p, r * b % p
+    return r
+
+
+class Consts:
+    """The class's image factors and CRT constants (build_consts of the engine)."""
+
+    def __init__(self, ln, K):
+        KP, M30 = K + 1, (1 << 30) - 1
+        M = 1
+        for p in TPRIMES[:KP]:
+            M *= p
+
+        def columns(v):
+            c = [(v >> (30 * j)) & M30 for j in range(K - 1)] + [(v >> (30 * (K - 1))) & M32]
+            return c, v >> (30 * (K - 1) + 32)
+        self.K, self.M, self.s, self.e, self.mk, self.mkh = K, M, [], [], [], []
+        total = 0
+        for k in range(KP):
+            p = TPRIMES[k]
+            cw = pow((1 << ln) // 2, -1, p) * ((1 << 32) % p) % p * pow(M // p % p, -1, p) % p
+            e = 1
+            while pow(cw * pow(e, -1, p) % p, (p - 1) // 2, p) != 1:
+                e += 1
+            s = _sqrt(cw * pow(e, -1, p) % p, p)
+            self.s.append(s if encode_weights(k, s)[1] else p - s)
+            assert encode_weights(k, self.s[k])[1]
+            self.e.append(e)
+            c, h = columns(M // p * e)
+            assert h == 0 or (K == 4 and k == 3)
+            self.mk.append(c)
+            self.mkh.append(h)
+            total += M // p * e * 2 * p
+        assert (total >> (30 * (K - 1))).bit_length() <= 64
+        self.tsh = 0
+        while True:
+            self.tsh += 1
+            t = (1 << (64 + 30 * (K - 1) + self.tsh)) // M
+            if t.bit_length() >= 31:
+                break
+        self.tinv = t
+        assert t.bit_length() <= 32
+        self.negm, self.negmh = columns(-M % (1 << (32 * K)))
+
+
+def crt_limbs(c, y):
+    """The engine's crt: K limbs of V from the K+1 lazy CRT coordinates."""
+    L, u = c.K, np.uint64
+    y = [_u(v) for v in y]
+    col = []
+    for j in range(L):
+        a = y[0] * u(c.mk[0][j])
+        for k in range(1, L + 1):
+            a = a + y[k] * u(c.mk[k][j])
+        col.append(a)
+    if L == 4:
+        col[L - 1] = col[L - 1] + (_u(y[3] * u(c.mkh[3])) << u(32))
+    hi = _u((col[L - 1] + (col[L - 2] >> u(30))) >> u(32))
+    t = (((hi * u(c.tinv)) >> u(32)) + u(1 << (c.tsh - 1))) >> u(c.tsh)
+    for j in range(L):
+        col[j] = col[j] + t * u(c.negm[j])
+    col[L - 1] = col[L - 1] + (_u(t * u(c.negmh)) << u(32))
+    for j in range(1, L):
+        col[j] = col[j] + (col[j - 1] >> u(30))
+    limbs = []
+    for i in range(L - 1):
+        pair = (_u(col[i]) << u(2) & u(M32)) | (_u(col[i + 1]) << u(32))
+        limbs.append(_u(pair >> u(2 + 2 * i)))
+    limbs.append(_u(col[L - 1] >> u(2 * (L - 1))))
+    return limbs
+
+
 def crt(res, ln, K):
-    """Exact signed values from the K+1 planes (each [0, 2p), holding (n/2) 2^-32 V)."""
-    KP = K + 1
-    M = 1
-    for p in TPRIMES[:KP]:
-        M *= p
-    n = 1 << ln
-    L = 32 * K
+    """Exact signed values from the K+1 planes of inverse outputs (each [0, 2p))."""
+    limbs = crt_limbs(Consts(ln, K), res)
     out = []
-    ys = []
-    for k in range(KP):
-        p = TPRIMES[k]
-        Mk = M // p
-        c = pow(n // 2, -1, p) * ((1 << 32) % p) % p * pow(Mk % p, -1, p) % p
-        y = shoup(res[k], c, shoup_const(c, p), p)
-        ys.append(np.where(y >= p, y - np.uint64(p), y))
-    fl = [(1 << 60) // p for p in TPRIMES[:KP]]
-    for i in range(len(ys[0])):
-        est = sum(int(ys[k][i]) * fl[k] for k in range(KP)) & ((1 << 64) - 1)
-        t = (est + (1 << 59)) >> 60
-        v = (sum(int(ys[k][i]) * (M // TPRIMES[k]) for k in range(KP)) - t * M) % (1 << L)
-        if v >> (L - 1):
-            v -= 1 << L
-        out.append(v)
+    for i in range(len(limbs[0])):
+        v = sum(int(l[i]) << (32 * j) for j, l in enumerate(limbs))
+        out.append(v - (1 << (32 * K)) if v >> (32 * K - 1) else v)
     return out
 
 
 def product(xe, ye, ln, K, domain_q):
     """Exact coefficients of x*y mod (x^n -+ 1) (ye None: x^2) through the model."""
-    res = []
+    res, c = [], Consts(ln, K)
     for k in range(K + 1):
-        fx = forward(encode(xe, k), ln, k, domain_q)
-        fy = None if ye is None else forward(encode(ye, k), ln, k, domain_q, reduce_out=True)
+        fx = forward(encode(xe, k, s=c.s[k]), ln, k, domain_q)
+        fy = None if ye is None else forward(encode(ye, k, s=c.s[k]), ln, k, domain_q, reduce_out=True)
         res.append(inverse(pointwise(fx, ln, k, domain_q, fy), ln, k, domain_q))
     return crt(res, ln, K)
 
