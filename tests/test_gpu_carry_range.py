@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 import annie_b200 as A
+from helpers import PRIMES
 from test_gpu_exact_range import _words
 from test_gpu_resident import PCK, _number
 
@@ -76,3 +77,69 @@ def test_product_with_large_coefficients_resident(K, lbase, bits):
         t.write_register(1, _words(K, y))
         t.mul(0, 1)
         assert t.get(0) == (v * y0 << W * i) * pow(half, -2, N) % N, "coefficient %d" % i
+
+
+def _square(x, B, nega):
+    """Coefficients of x^2 mod x^n -+ 1, below 2^(B-1) in magnitude (by one product
+    of integers with B bits per coefficient)."""
+    n, half = len(x), 1 << (B - 1)
+    X = sum(v << B * i for i, v in enumerate(x))
+    p, c = X * X, []
+    for _ in range(2 * n):
+        d = ((p + half) & ((1 << B) - 1)) - half
+        c.append(d)
+        p = (p - d) >> B
+    return [c[i] - c[i + n] if nega else c[i] + c[i + n] for i in range(n)]
+
+
+# K, lbase, ln inside the parameter rule
+EXTREME = [(2, 14, 10), (3, 21, 9), (3, 20, 12), (4, 28, 10), (4, 27, 11), (5, 18, 10), (5, 17, 11)]
+
+
+def _extreme(K, lbase, ln):
+    """Registers of extreme digits: all-maximal, the most negative balanced ones,
+    both beside each other; and the largest multiplier that they leave room for."""
+    W, n, P = PCK[K] * lbase, 1 << ln, 1
+    for p in PRIMES[:K]:
+        P *= p
+    big, low = (1 << W) - 1, -(1 << (W - 1))
+    a = min((1 << 31) - 1, P // 2 >> (ln + 2 * W))
+    assert a >= 3
+    return [[big] * n, [low] * n, [low, big] * (n // 2), [low] * (n - 1) + [big], [big] + [low] * (n - 1)], a
+
+
+@pytest.mark.parametrize("rows", [5, 3, 1])
+@pytest.mark.parametrize("K,lbase,ln", EXTREME)
+def test_extreme_digits(K, lbase, ln, rows):
+    # 32 rows (a thread per group), 8 and 2 rows (four lanes per group)
+    params, W = (K, PCK[K], ln, lbase), PCK[K] * lbase
+    t = A.Transform(_number(params, 3 * ln), 3, params=params)
+    if ln - 1 - rows < 4:
+        rows = ln - 5
+    t.set_geometry(ln - 1 - rows)
+    regs, amax = _extreme(K, lbase, ln)
+    for x in regs:
+        for dom in (0, 1):
+            V = _square(x, 2 * W + ln + 3, dom == 1)
+            for a in (1, amax):
+                got = t.diag_product(_words(K, x), dom, a)
+                assert np.array_equal(got, _words(K, _carry([a * v for v in V], W, dom == 1))), "domain %d, a = %d" % (dom, a)
+
+
+@pytest.mark.parametrize("K,lbase,ln", EXTREME)
+def test_extreme_digits_resident(K, lbase, ln):
+    # up to about half of R, as a register of a number within the rule
+    params, W, n = (K, PCK[K], ln, lbase), PCK[K] * lbase, 1 << ln
+    N = _number(params, 3 * ln)
+    t = A.Transform(N, 3, params=params)
+    scale = pow((pow(2, W * n, N) - 1) * pow(2, -1, N), -2, N)
+    regs, a = _extreme(K, lbase, ln)
+    for x in regs:
+        x = x[:n // 2] + [0] * (n - n // 2)
+        X = sum(v << W * i for i, v in enumerate(x))
+        t.write_register(0, _words(K, x))
+        t.write_register(1, _words(K, x))
+        t.square_mul(a)
+        assert t.get(0) == a * X * X * scale % N
+        t.mul(1, 1)
+        assert t.get(1) == X * X * scale % N
