@@ -27,18 +27,13 @@ __host__ __device__ constexpr u32 col_ctas(u32 RC) { return (RC <= 32) ? 1u : 1u
 // Threads of a column-pass CTA: the carry phases have 8 groups of 4 columns
 // per row, the butterfly stages KP / 8 times 32 tasks per row, so the thread
 // count follows the number of rows.
-#ifndef AB_COL_TPR
-#define AB_COL_TPR 8
-#endif
-#ifndef AB_COL_REGT
-#define AB_COL_REGT 1024
-#endif
+constexpr int COL_ROW_THREADS = 8, COL_SM_THREADS = 1024;   // per row; per SM (64 registers each)
 constexpr int COL_THREADS = 384;                       // fused kernels: every split in one launch
 template <int LOG_H, bool WIDE>
 struct ColCfg
 {
-	static constexpr int NT = WIDE ? 32 << LOG_H : ((AB_COL_TPR << LOG_H) < 64) ? 64 : (AB_COL_TPR << LOG_H);
-	static constexpr int MINB = (AB_COL_REGT / NT < 16) ? AB_COL_REGT / NT : 16;
+	static constexpr int NT = WIDE ? 32 << LOG_H : ((COL_ROW_THREADS << LOG_H) < 64) ? 64 : (COL_ROW_THREADS << LOG_H);
+	static constexpr int MINB = (COL_SM_THREADS / NT < 16) ? COL_SM_THREADS / NT : 16;
 };
 
 // One radix-2^S step of the column transform (levels on row bits b..b+S-1)
@@ -136,14 +131,6 @@ __device__ __forceinline__ void col_forward(u32 * tile, u32 * __restrict__ x, u3
 		const u32 p = c.p[k];
 		if (own) col_step<SB, false>(tile + k * PS + u, CW, x + (size_t)k * n + gc, R, LOG_H, 0, (u32)o, twk + (k << LOG_H), p, 2 * p);
 	}
-}
-
-// Adds d to an exact value (three limbs).
-__device__ __forceinline__ void exact_add(u32 (&x)[AB_NW], __int128 d)
-{
-	const unsigned __int128 v = ((unsigned __int128)x[0] | ((unsigned __int128)x[1] << 32) | ((unsigned __int128)x[2] << 64)) +
-	                            (unsigned __int128)d;
-	x[0] = (u32)v; x[1] = (u32)(v >> 32); x[2] = (u32)(v >> 64);
 }
 
 // Second carry phase for one group of 4 coefficients (kernel.cl:1582-1613):
@@ -298,216 +285,212 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 		const bool full = (w.ws == ND - 1);
 		const bool adjust = (J.lower != LOWER_NONE);
 		const bool edges = adjust && (b == 0 || b == nb - 1);
-	if constexpr (WIDE)
-	{
-		// a thread per tile word: row tid / 32, column lane
-		const int row = tid >> 5, u4 = lane >> 2;
-		const u32 j = (u32)lane & 3u;
-		const size_t o = (size_t)row * R + gcol(lane);
-		Big<L> f = big_zero<L>();
-		if (lane < WU)
+		if constexpr (WIDE)
 		{
-			u32 sv[AB_NW] = {};
-			if (J.sub != nullptr)
-			{
-#pragma unroll
-				for (int l = 0; l < AB_NW; ++l) sv[l] = J.sub[(size_t)l * n + o];
-			}
-			if constexpr (SPARSE) f = sparse_product<L>(J.cand[cand].sp, (u32)o, n, get_m);
-			else
-			{
-				u32 y[KP];
-#pragma unroll
-				for (int k = 0; k < KP; ++k) y[k] = tile[k * PS + tid];
-				f = crt<L>(c, y);
-			}
-			if (amul != 1u) f = big_mul_u32<L>(f, amul);
-			if (J.sub != nullptr) f = big_sub<L>(f, big_from_exact<L>(sv[0], sv[1], sv[2]));
-		}
-		u32 d[ND], x[AB_NW];
-		if (full) lane_digits<true, L, ND>(f, w, j, d);
-		else lane_digits<false, L, ND>(f, w, j, d);
-		if (lane < WU && j == 3)
-		{
-#pragma unroll
-			for (int l = 0; l < L; ++l) cw[(tid >> 2) * L + l] = f.l[l];
-		}
-		__syncthreads();
-		const bool mine = (lane >= E && lane < WU);
-		const bool top0 = adjust && E == 8 && row == H - 1 && u4 == 1;
-		Big<L> cin = big_zero<L>();
-		if (j == 0 && (mine || top0))
-		{
-			int prow = row, pu4 = u4 - 1;
-			bool neg = false;
-			if (b == 0 && lane == E)
-			{
-				// first group of a row: its predecessor ends the previous row
-				if (E == 0) pu4 = ng - 1;
-				if (row > 0) prow = row - 1;
-				else { prow = H - 1; neg = (J.nega != 0); }
-			}
-#pragma unroll
-			for (int l = 0; l < L; ++l) cin.l[l] = cw[(prow * 8 + pu4) * L + l];
-			if (neg) cin = big_neg<L>(cin);
-		}
-		if (full) lane_balance<true, L, ND>(cin, d, w, half_of(wbits), j, x);
-		else lane_balance<false, L, ND>(cin, d, w, half_of(wbits), j, x);
-		if (edges)
-		{
-			// mod R (+2) / mod Q on the top and bottom coefficients (kernel.cl:1653-1683);
-			// CTA 0 re-derives the last coefficient of the register from its
-			// predecessor columns
-			const bool last = (b == nb - 1) && row == H - 1 && lane == WU - 1;
-			if ((last || (top0 && j == 3)) && reaches_width(x, w)) decision = 1;
-			__syncthreads();
-			if (last && decision) exact_add(x, -((__int128)1 << wbits));
-			if (b == 0 && row == 0 && lane == E)
-			{
-				int dv = 0;
-				if (decision) dv += (J.lower == LOWER_Q) ? -1 : 1;
-				if (J.lower == LOWER_R_ADD2) dv += 2;
-				exact_add(x, (__int128)dv);
-			}
-		}
-		if (mine)
-		{
-#pragma unroll
-			for (int l = 0; l < AB_NW; ++l)
-			{
-				if (J.out_norm) J.out_norm[(size_t)l * n + o] = x[l];
-				if (J.out_snap) J.out_snap[(size_t)l * n + o] = x[l];
-			}
-			if (fwd) encode1(x);
-		}
-	}
-	else
-	{
-		// ---- carry phase 1: per group, exact values (CRT), x a, - sub,
-		// unsigned digits + carry-out
-		for (int idx = tid; idx < H * 8; idx += NT)
-		{
-			const int row = idx >> 3, u4 = idx & 7;
-			if (u4 >= ng) continue;
-			u32 xv[KP][4];
-			if constexpr (!SPARSE)
-#pragma unroll
-			for (int k = 0; k < KP; ++k)
-			{
-				const uint4 t = *reinterpret_cast<const uint4 *>(tile + k * PS + row * CW + 4 * u4);
-				xv[k][0] = t.x; xv[k][1] = t.y; xv[k][2] = t.z; xv[k][3] = t.w;
-			}
-			u32 sv[4][AB_NW];
-			if (J.sub != nullptr) load_norm(J.sub, row, u4, sv);
+			// a thread per tile word: row tid / 32, column lane
+			const int row = tid >> 5, u4 = lane >> 2;
+			const u32 j = (u32)lane & 3u;
+			const size_t o = (size_t)row * R + gcol(lane);
 			Big<L> f = big_zero<L>();
-			u32 dg[4][ND];
-			auto digits = [&](auto is_full) {
-#pragma unroll
-				for (int j = 0; j < 4; ++j)
+			if (lane < WU)
+			{
+				u32 sv[AB_NW] = {};
+				if (J.sub != nullptr)
 				{
-					Big<L> V;
-					if constexpr (SPARSE) V = sparse_product<L>(J.cand[cand].sp, (u32)row * R + gcol(4 * u4) + (u32)j, n, get_m);
-					else
-					{
-						u32 rr[KP];
 #pragma unroll
-						for (int k = 0; k < KP; ++k) rr[k] = xv[k][j];
-						V = crt<L>(c, rr);
-					}
-					if (amul != 1u) V = big_mul_u32<L>(V, amul);
-					if (J.sub != nullptr) V = big_sub<L>(V, big_from_exact<L>(sv[j][0], sv[j][1], sv[j][2]));
-					f = (j == 0) ? V : big_add<L>(f, V);
-					split_digit<decltype(is_full)::value, L, ND>(f, w, dg[j]);
+					for (int l = 0; l < AB_NW; ++l) sv[l] = J.sub[(size_t)l * n + o];
 				}
-			};
-			if (full) digits(std::true_type{});
-			else digits(std::false_type{});
-#pragma unroll
-			for (int l = 0; l < ND; ++l)
-				*reinterpret_cast<uint4 *>(tile + l * PS + row * CW + 4 * u4) = make_uint4(dg[0][l], dg[1][l], dg[2][l], dg[3][l]);
-#pragma unroll
-			for (int l = 0; l < L; ++l) cw[idx * L + l] = f.l[l];
-		}
-		__syncthreads();
-
-		// ---- carry phase 2: add the previous group's carry-out, balanced
-		// values; then the outputs of the group.  Each thread reads and writes
-		// only its own group of the tile.
-		const Big<AB_NW> half = half_of(wbits);
-		for (int idx = tid; idx < H * 8; idx += NT)
-		{
-			const int row = idx >> 3, u4 = idx & 7;
-			if (u4 >= ng) continue;
-			// CTA 0 re-derives the last coefficient of the register from its
-			// predecessor columns, for the mod R / mod Q decision
-			const bool top0 = adjust && E == 8 && row == H - 1 && u4 == 1;
-			if (4 * u4 < E && !top0) continue;
-			int prow = row, pu4 = u4 - 1;
-			bool neg = false;
-			if (b == 0 && 4 * u4 == E)
-			{
-				// first group of a row: its predecessor ends the previous row
-				if (E == 0) pu4 = ng - 1;
-				if (row > 0) prow = row - 1;
-				else { prow = H - 1; neg = (J.nega != 0); }
-			}
-			Big<L> f;
-#pragma unroll
-			for (int l = 0; l < L; ++l) f.l[l] = cw[(prow * 8 + pu4) * L + l];
-			if (neg) f = big_neg<L>(f);
-			u32 dg[4][ND];
-#pragma unroll
-			for (int l = 0; l < ND; ++l)
-			{
-				const uint4 t = *reinterpret_cast<const uint4 *>(tile + l * PS + row * CW + 4 * u4);
-				dg[0][l] = t.x; dg[1][l] = t.y; dg[2][l] = t.z; dg[3][l] = t.w;
-			}
-			u32 ex[4][AB_NW];
-			if (full) carry_phase2<true, L, PCK>(w, half, f, dg, ex);
-			else carry_phase2<false, L, PCK>(w, half, f, dg, ex);
-			const bool first = (b == 0) && row == 0 && 4 * u4 == E;
-			const bool last = (b == nb - 1) && row == H - 1 && u4 == ng - 1;
-			if (adjust && (first || last || top0))
-			{
-				if ((last || top0) && reaches_width(ex[3], w)) decision = 1;
-				if (!top0)
+				if constexpr (SPARSE) f = sparse_product<L>(J.cand[cand].sp, (u32)o, n, get_m);
+				else
 				{
+					u32 y[KP];
+#pragma unroll
+					for (int k = 0; k < KP; ++k) y[k] = tile[k * PS + tid];
+					f = crt<L>(c, y);
+				}
+				if (amul != 1u) f = big_mul_u32<L>(f, amul);
+				if (J.sub != nullptr) f = big_sub<L>(f, big_from_exact<L>(sv[0], sv[1], sv[2]));
+			}
+			u32 d[ND], x[AB_NW];
+			if (full) lane_digits<true, L, ND>(f, w, j, d);
+			else lane_digits<false, L, ND>(f, w, j, d);
+			if (lane < WU && j == 3)
+			{
+#pragma unroll
+				for (int l = 0; l < L; ++l) cw[(tid >> 2) * L + l] = f.l[l];
+			}
+			__syncthreads();
+			const bool mine = (lane >= E && lane < WU);
+			const bool top0 = adjust && E == 8 && row == H - 1 && u4 == 1;
+			Big<L> cin = big_zero<L>();
+			if (j == 0 && (mine || top0))
+			{
+				int prow = row, pu4 = u4 - 1;
+				bool neg = false;
+				if (b == 0 && lane == E)
+				{
+					// first group of a row: its predecessor ends the previous row
+					if (E == 0) pu4 = ng - 1;
+					if (row > 0) prow = row - 1;
+					else { prow = H - 1; neg = (J.nega != 0); }
+				}
+#pragma unroll
+				for (int l = 0; l < L; ++l) cin.l[l] = cw[(prow * 8 + pu4) * L + l];
+				if (neg) cin = big_neg<L>(cin);
+			}
+			if (full) lane_balance<true, L, ND>(cin, d, w, half_of(wbits), j, x);
+			else lane_balance<false, L, ND>(cin, d, w, half_of(wbits), j, x);
+			if (edges)
+			{
+				// mod R (+2) / mod Q on the top and bottom coefficients (kernel.cl:1653-1683);
+				// CTA 0 re-derives the last coefficient of the register from its
+				// predecessor columns
+				const bool last = (b == nb - 1) && row == H - 1 && lane == WU - 1;
+				if ((last || (top0 && j == 3)) && reaches_width(x, w)) decision = 1;
+				__syncthreads();
+				if (last && decision) exact_add(x, -((__int128)1 << wbits));
+				if (b == 0 && row == 0 && lane == E)
+				{
+					exact_add(x, lower_first(J.lower, decision != 0));
+				}
+			}
+			if (mine)
+			{
+#pragma unroll
+				for (int l = 0; l < AB_NW; ++l)
+				{
+					if (J.out_norm) J.out_norm[(size_t)l * n + o] = x[l];
+					if (J.out_snap) J.out_snap[(size_t)l * n + o] = x[l];
+				}
+				if (fwd) encode1(x);
+			}
+		}
+		else
+		{
+			// ---- carry phase 1: per group, exact values (CRT), x a, - sub,
+			// unsigned digits + carry-out
+			for (int idx = tid; idx < H * 8; idx += NT)
+			{
+				const int row = idx >> 3, u4 = idx & 7;
+				if (u4 >= ng) continue;
+				u32 xv[KP][4];
+				if constexpr (!SPARSE)
+				{
+#pragma unroll
+					for (int k = 0; k < KP; ++k)
+					{
+						const uint4 t = *reinterpret_cast<const uint4 *>(tile + k * PS + row * CW + 4 * u4);
+						xv[k][0] = t.x; xv[k][1] = t.y; xv[k][2] = t.z; xv[k][3] = t.w;
+					}
+				}
+				u32 sv[4][AB_NW];
+				if (J.sub != nullptr) load_norm(J.sub, row, u4, sv);
+				Big<L> f = big_zero<L>();
+				u32 dg[4][ND];
+				auto digits = [&](auto is_full) {
+#pragma unroll
+					for (int j = 0; j < 4; ++j)
+					{
+						Big<L> V;
+						if constexpr (SPARSE) V = sparse_product<L>(J.cand[cand].sp, (u32)row * R + gcol(4 * u4) + (u32)j, n, get_m);
+						else
+						{
+							u32 rr[KP];
+#pragma unroll
+							for (int k = 0; k < KP; ++k) rr[k] = xv[k][j];
+							V = crt<L>(c, rr);
+						}
+						if (amul != 1u) V = big_mul_u32<L>(V, amul);
+						if (J.sub != nullptr) V = big_sub<L>(V, big_from_exact<L>(sv[j][0], sv[j][1], sv[j][2]));
+						f = (j == 0) ? V : big_add<L>(f, V);
+						split_digit<decltype(is_full)::value, L, ND>(f, w, dg[j]);
+					}
+				};
+				if (full) digits(std::true_type{});
+				else digits(std::false_type{});
+#pragma unroll
+				for (int l = 0; l < ND; ++l)
+					*reinterpret_cast<uint4 *>(tile + l * PS + row * CW + 4 * u4) = make_uint4(dg[0][l], dg[1][l], dg[2][l], dg[3][l]);
+#pragma unroll
+				for (int l = 0; l < L; ++l) cw[idx * L + l] = f.l[l];
+			}
+			__syncthreads();
+
+			// ---- carry phase 2: add the previous group's carry-out, balanced
+			// values; then the outputs of the group.  Each thread reads and writes
+			// only its own group of the tile.
+			const Big<AB_NW> half = half_of(wbits);
+			for (int idx = tid; idx < H * 8; idx += NT)
+			{
+				const int row = idx >> 3, u4 = idx & 7;
+				if (u4 >= ng) continue;
+				// CTA 0 re-derives the last coefficient of the register from its
+				// predecessor columns, for the mod R / mod Q decision
+				const bool top0 = adjust && E == 8 && row == H - 1 && u4 == 1;
+				if (4 * u4 < E && !top0) continue;
+				int prow = row, pu4 = u4 - 1;
+				bool neg = false;
+				if (b == 0 && 4 * u4 == E)
+				{
+					// first group of a row: its predecessor ends the previous row
+					if (E == 0) pu4 = ng - 1;
+					if (row > 0) prow = row - 1;
+					else { prow = H - 1; neg = (J.nega != 0); }
+				}
+				Big<L> f;
+#pragma unroll
+				for (int l = 0; l < L; ++l) f.l[l] = cw[(prow * 8 + pu4) * L + l];
+				if (neg) f = big_neg<L>(f);
+				u32 dg[4][ND];
+#pragma unroll
+				for (int l = 0; l < ND; ++l)
+				{
+					const uint4 t = *reinterpret_cast<const uint4 *>(tile + l * PS + row * CW + 4 * u4);
+					dg[0][l] = t.x; dg[1][l] = t.y; dg[2][l] = t.z; dg[3][l] = t.w;
+				}
+				u32 ex[4][AB_NW];
+				if (full) carry_phase2<true, L, PCK>(w, half, f, dg, ex);
+				else carry_phase2<false, L, PCK>(w, half, f, dg, ex);
+				const bool first = (b == 0) && row == 0 && 4 * u4 == E;
+				const bool last = (b == nb - 1) && row == H - 1 && u4 == ng - 1;
+				if (adjust && (first || last || top0))
+				{
+					if ((last || top0) && reaches_width(ex[3], w)) decision = 1;
+					if (!top0)
+					{
+#pragma unroll
+						for (int j = 0; j < 4; ++j)
+#pragma unroll
+							for (int l = 0; l < AB_NW; ++l) edge[(last ? 12 : 0) + 3 * j + l] = ex[j][l];
+					}
+				}
+				else finalize(row, u4, ex);
+			}
+
+			// ---- mod R (+2) / mod Q on the top and bottom coefficients (kernel.cl:1653-1683)
+			if (edges)
+			{
+				__syncthreads();
+				if (tid < 2 && ((tid == 0) ? b == 0 : b == nb - 1))
+				{
+					u32 ex[4][AB_NW];
 #pragma unroll
 					for (int j = 0; j < 4; ++j)
 #pragma unroll
-						for (int l = 0; l < AB_NW; ++l) edge[(last ? 12 : 0) + 3 * j + l] = ex[j][l];
-				}
-			}
-			else finalize(row, u4, ex);
-		}
-
-		// ---- mod R (+2) / mod Q on the top and bottom coefficients (kernel.cl:1653-1683)
-		if (edges)
-		{
-			__syncthreads();
-			if (tid < 2 && ((tid == 0) ? b == 0 : b == nb - 1))
-			{
-				u32 ex[4][AB_NW];
-#pragma unroll
-				for (int j = 0; j < 4; ++j)
-#pragma unroll
-					for (int l = 0; l < AB_NW; ++l) ex[j][l] = edge[12 * tid + 3 * j + l];
-				if (tid == 0)
-				{
-					int d = 0;
-					if (decision) d += (J.lower == LOWER_Q) ? -1 : 1;
-					if (J.lower == LOWER_R_ADD2) d += 2;
-					exact_add(ex[0], (__int128)d);
-					finalize(0, E / 4, ex);
-				}
-				else
-				{
-					if (decision) exact_add(ex[3], -((__int128)1 << wbits));
-					finalize(H - 1, ng - 1, ex);
+						for (int l = 0; l < AB_NW; ++l) ex[j][l] = edge[12 * tid + 3 * j + l];
+					if (tid == 0)
+					{
+						exact_add(ex[0], lower_first(J.lower, decision != 0));
+						finalize(0, E / 4, ex);
+					}
+					else
+					{
+						if (decision) exact_add(ex[3], -((__int128)1 << wbits));
+						finalize(H - 1, ng - 1, ex);
+					}
 				}
 			}
 		}
-	}
 	}
 
 	// ---- the first LA forward levels of the result in one or two domains: the
@@ -535,13 +518,15 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 				}
 			}
 			else
-			for (int idx = tid; idx < H * 8; idx += NT)
 			{
-				const int row = idx >> 3, u4 = idx & 7;
-				if (4 * u4 < E || u4 >= ng) continue;
-				u32 x[4][AB_NW];
-				load_norm(src, row, u4, x);
-				encode(row, u4, x);
+				for (int idx = tid; idx < H * 8; idx += NT)
+				{
+					const int row = idx >> 3, u4 = idx & 7;
+					if (4 * u4 < E || u4 >= ng) continue;
+					u32 x[4][AB_NW];
+					load_norm(src, row, u4, x);
+					encode(row, u4, x);
+				}
 			}
 		}
 		__syncthreads();
@@ -582,14 +567,12 @@ static cudaError_t colpass_s(const Geometry & g, const TConst & c, const ColJobs
 	                                             : colpass_w<LOG_H, K, PCK, WIDE, false>(g, c, jobs, njobs, s, ncand);
 }
 
-// A thread per tile word (WIDE) up to 16 rows and AB_COL_WIDE_CTAS CTAs: where
+// A thread per tile word (WIDE) up to 16 rows and COL_WIDE_CTAS CTAs: where
 // the launch leaves SMs idle, the shorter chains win (us per squaring, grouped /
 // wide: 524k bits 28.6 / 23.1, 2M bits 34.2 / 31.1, 4M bits 41.7 / 38.4); with
 // 32 rows a CTA has 1,024 threads and costs more to start than it saves (6.6M
 // bits, 147 CTAs: 52.1 / 60.7).
-#ifndef AB_COL_WIDE_CTAS
-#define AB_COL_WIDE_CTAS 296
-#endif
+constexpr u32 COL_WIDE_CTAS = 296;
 template <int LOG_H, int K, int PCK>
 static cudaError_t colpass_t(const Geometry & g, const TConst & c, const ColJobs & jobs, int njobs, cudaStream_t s, int ncand)
 {
@@ -600,7 +583,7 @@ static cudaError_t colpass_t(const Geometry & g, const TConst & c, const ColJobs
 			const cudaError_t e = colpass_s<LOG_H, K, PCK, true>(g, c, jobs, njobs, s, 0);
 			if (e != cudaSuccess) return e;
 		}
-		else if (g.NC * (u32)njobs * (u32)ncand <= AB_COL_WIDE_CTAS) return colpass_s<LOG_H, K, PCK, true>(g, c, jobs, njobs, s, ncand);
+		else if (g.NC * (u32)njobs * (u32)ncand <= COL_WIDE_CTAS) return colpass_s<LOG_H, K, PCK, true>(g, c, jobs, njobs, s, ncand);
 	}
 	return colpass_s<LOG_H, K, PCK, false>(g, c, jobs, njobs, s, ncand);
 }

@@ -219,19 +219,14 @@ __device__ __forceinline__ void reduce_all(u32 (&v)[N], u32 p2)
 // measured the same there and slower below (us per squaring, 4 / 3: 33.2M bits
 // 150.2 / 150.4, 6.6M bits 51.4 / 48.2, 2M bits 29.9 / 26.9).  128 threads:
 // 185.5 at 33.2M bits; 512: 155.5.
-#ifndef AB_ROW_THREADS
-#define AB_ROW_THREADS 256
-#endif
-#ifndef AB_ROW_MINB
-#define AB_ROW_MINB 3
-#endif
+constexpr u32 ROW_THREADS = 256;
 template <int LOG_R>
 struct RowCfg
 {
 	static constexpr u32 T = (1u << LOG_R) / RP_EPT;             // virtual threads
-	static constexpr u32 NT = (T < AB_ROW_THREADS) ? T : AB_ROW_THREADS;   // physical threads
+	static constexpr u32 NT = (T < ROW_THREADS) ? T : ROW_THREADS;   // physical threads
 	static constexpr u32 RND = T / NT;
-	static constexpr int MINB = (AB_ROW_MINB * AB_ROW_THREADS > 2048) ? 2048 / AB_ROW_THREADS : AB_ROW_MINB;
+	static constexpr int MINB = 3;
 	static constexpr size_t SMEM = sizeof(u32) * ((1u << LOG_R) + (1u << LOG_R) / 16);   // padded row
 };
 
@@ -336,7 +331,7 @@ __device__ __forceinline__ void rowpass_body(const RowJob & J, const TConst & c,
 			for (u32 rr = 0; rr < RND; ++rr)
 			{
 				const u32 vt = tid + rr * NT;
-			if (IDLE && vt >= T) continue;
+				if (IDLE && vt >= T) continue;
 				rp_load_smem<4>(v, sm, vt, T, b);
 				rp_radix<4, false, MIR>(v, vt, T, b, LB, tw, Hr, p, p2);
 				rp_store_smem<4>(v, sm, vt, T, b);
@@ -378,7 +373,7 @@ __device__ __forceinline__ void rowpass_body(const RowJob & J, const TConst & c,
 			for (u32 rr = 0; rr < RND; ++rr)
 			{
 				const u32 vt = tid + rr * NT;
-			if (IDLE && vt >= T) continue;
+				if (IDLE && vt >= T) continue;
 				rp_load_smem<4>(v, sm, vt, T, b);
 				rp_radix<4, true, MIR>(v, vt, T, b, LB, tw, Hr, p, p2);
 				rp_store_smem<4>(v, sm, vt, T, b);

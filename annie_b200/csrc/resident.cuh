@@ -65,9 +65,7 @@ __device__ __forceinline__ void st_remote(u32 a, u32 v)
 	asm volatile("st.shared::cluster.u32 [%0], %1;" :: "r"(a), "r"(v) : "memory");
 }
 
-#ifndef AB_RES_REGT
-#define AB_RES_REGT 1024
-#endif
+constexpr u32 RES_THREADS = 1024;                       // of an SM that a kernel is compiled for (64 registers each)
 template <int LN, int K>
 struct ResCfg
 {
@@ -88,7 +86,7 @@ struct ResCfg
 	static constexpr size_t SMEM = sizeof(u32) * (2 * W + 3 * N + (N > TQ ? N : TQ) + CWN);
 	static_assert(MQ <= N, "m' in the second factor's place");
 	// CTAs per SM that the kernel is compiled for
-	static constexpr u32 BY_T = AB_RES_REGT / NT, BY_S = (u32)((size_t)227 * 1024 / (SMEM + 1024));
+	static constexpr u32 BY_T = RES_THREADS / NT, BY_S = (u32)((size_t)227 * 1024 / (SMEM + 1024));
 	static constexpr u32 MINB = (BY_T < BY_S ? BY_T : BY_S) < 1 ? 1 : (BY_T < BY_S ? BY_T : BY_S);
 };
 
@@ -184,28 +182,8 @@ __device__ __forceinline__ bool res_carry(const TConst & c, const CarryRange & r
 		// whether the last coefficient is 2^W or more
 		if ((mine || top0) && e == N - 1) *decision = reaches_width(x, w) ? 1 : 0;
 		__syncthreads();
-		if (mine && (e == 0 || e == N - 1))
-		{
-			Big<AB_NW> a, b;
-#pragma unroll
-			for (int i = 0; i < AB_NW; ++i) a.l[i] = x[i];
-			if (e == 0)
-			{
-				int dv = 0;
-				if (*decision) dv += (lower == LOWER_Q) ? -1 : 1;
-				if (lower == LOWER_R_ADD2) dv += 2;
-				b.l[0] = (u32)dv; b.l[1] = b.l[2] = (u32)(dv >> 31);
-				a = big_add<AB_NW>(a, b);
-			}
-			else if (*decision)
-			{
-#pragma unroll
-				for (int i = 0; i < AB_NW; ++i) b.l[i] = (i == (wbits >> 5)) ? 1u << (wbits & 31) : 0u;
-				a = big_sub<AB_NW>(a, b);
-			}
-#pragma unroll
-			for (int i = 0; i < AB_NW; ++i) x[i] = a.l[i];
-		}
+		if (mine && e == 0) exact_add(x, lower_first(lower, *decision != 0));
+		else if (mine && e == N - 1 && *decision) exact_add(x, -((__int128)1 << wbits));
 	}
 	return mine;
 }
