@@ -5,7 +5,6 @@
 // GPU.  All lanes of a warp call these together.
 #pragma once
 #include "arith.cuh"
-#include "kernels.h"
 
 namespace ab
 {
@@ -80,7 +79,7 @@ __device__ __forceinline__ void lane_balance(const Big<L> & cin, const u32 (&d)[
 		if (r < 3)
 		{
 			u32 e[ND];
-			c = add_digit<CL, ND>(t, hd);
+			c = big_add<CL>(t, carry_extend<CL, AB_NW>(half));
 			split_digit<FULL, CL, ND>(c, w, e);
 			if (j == (u32)r)
 			{
@@ -116,21 +115,6 @@ __device__ __forceinline__ bool reaches_width(const u32 (&x)[AB_NW], const Width
 	u32 e[AB_NW];
 	split_digit<false, AB_NW, AB_NW>(t, w, e);
 	return (i32)t.l[2] >= 0 && (t.l[0] | t.l[1] | t.l[2]) != 0u;
-}
-
-// Adds d to an exact value (three limbs).
-__device__ __forceinline__ void exact_add(u32 (&x)[AB_NW], __int128 d)
-{
-	const unsigned __int128 v = ((unsigned __int128)x[0] | ((unsigned __int128)x[1] << 32) | ((unsigned __int128)x[2] << 64)) +
-	                            (unsigned __int128)d;
-	x[0] = (u32)v; x[1] = (u32)(v >> 32); x[2] = (u32)(v >> 64);
-}
-
-// mod R (+2) / mod Q (kernel.cl:1653-1683): what the first coefficient of the
-// register takes; `reached`: the last one is 2^W or more, and then loses 2^W.
-__device__ __forceinline__ __int128 lower_first(int lower, bool reached)
-{
-	return (reached ? ((lower == LOWER_Q) ? -1 : 1) : 0) + ((lower == LOWER_R_ADD2) ? 2 : 0);
 }
 
 } // namespace ab

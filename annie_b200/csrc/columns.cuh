@@ -133,6 +133,14 @@ __device__ __forceinline__ void col_forward(u32 * tile, u32 * __restrict__ x, u3
 	}
 }
 
+// Adds d to an exact value (three limbs).
+__device__ __forceinline__ void exact_add(u32 (&x)[AB_NW], __int128 d)
+{
+	const unsigned __int128 v = ((unsigned __int128)x[0] | ((unsigned __int128)x[1] << 32) | ((unsigned __int128)x[2] << 64)) +
+	                            (unsigned __int128)d;
+	x[0] = (u32)v; x[1] = (u32)(v >> 32); x[2] = (u32)(v >> 64);
+}
+
 // Second carry phase for one group of 4 coefficients (kernel.cl:1582-1613):
 // f = carry-in, d = the group's unsigned W-bit digits.  The first three become
 // balanced, v in [-2^(W-1), 2^(W-1)) with the carry (f + d + 2^(W-1)) >> W;
@@ -185,7 +193,7 @@ __device__ __forceinline__ void carry_phase2(const Width & w, const Big<AB_NW> &
 // runtime amount), the residues are the CRT coordinates themselves (crt), the
 // exact values go from the carry to their residues in registers, and the first
 // and last butterfly stages read and write global memory directly.  B200, one
-// domain out, 33.2M bits: 36.9 -> 24.5 us (17.5 M -> 12.1 M warp instructions,
+// domain out, 33.2M bits: 37.6 -> 24.5 us (17.5 M -> 12.1 M warp instructions,
 // multiplier floor 8.6 us); a batch of 16 x 1.1M bits 164.8 -> 85.0 us per step.
 //
 // WIDE: a thread per tile word (32 H threads) and the carry by 4 lanes per
@@ -351,7 +359,10 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 				if (last && decision) exact_add(x, -((__int128)1 << wbits));
 				if (b == 0 && row == 0 && lane == E)
 				{
-					exact_add(x, lower_first(J.lower, decision != 0));
+					int dv = 0;
+					if (decision) dv += (J.lower == LOWER_Q) ? -1 : 1;
+					if (J.lower == LOWER_R_ADD2) dv += 2;
+					exact_add(x, (__int128)dv);
 				}
 			}
 			if (mine)
@@ -480,7 +491,10 @@ __device__ __forceinline__ void colpass_body(ColJob J, const TConst & c, u32 can
 						for (int l = 0; l < AB_NW; ++l) ex[j][l] = edge[12 * tid + 3 * j + l];
 					if (tid == 0)
 					{
-						exact_add(ex[0], lower_first(J.lower, decision != 0));
+						int d = 0;
+						if (decision) d += (J.lower == LOWER_Q) ? -1 : 1;
+						if (J.lower == LOWER_R_ADD2) d += 2;
+						exact_add(ex[0], (__int128)d);
 						finalize(0, E / 4, ex);
 					}
 					else

@@ -911,9 +911,18 @@ struct ab_transform
 
 // Slots of a batch up to which a chunk runs resident (resident.cuh) and not as
 // passes.  Measured on B200, 64 squarings, us per step of the whole batch
-// (resident / passes with their best split): ln 9 (K = 3) 256 slots 36.1 / 58.6;
-// ln 10 (K = 5) 256 slots 87.9 / 107.8; ln 11 (K = 5) 32 slots 33.2 / 38.5, 64
-// slots 59.1 / 53.5; ln 12 (K = 5) 16 slots 32.0 / 36.8, 32 slots 59.7 / 47.9.
+// (resident / passes with their best split), dense N, K = 3 and K = 5:
+//   ln 6, 256 slots: 19.4 / 27.6 and 34.7 / 34.6; 1,024: 71 / 64 and 133 / 90
+//   ln 8, 1,024 slots: 86 / 119 and 160 / 167
+//   ln 9, 512 slots: 54 / 95 and 94 / 133
+//   ln 10, 512 slots: 95 / 128 and 158 / 189
+//   ln 11, 32 slots: 17.2 / 29.8 and 25.8 / 37.3; 64: 33.7 / 38.0 and 47.9 / 52.2
+//   ln 12, 8 slots: 19.0 / 24.9 and 27.5 / 28.1; 16: 37.7 / 28.3 and 32.6 / 35.4
+//   (K = 4: 29.9 / 32.2); 32: 56 / 35 and 57 / 47
+// Sparse N shortens both sides, by 10 to 25 % (ln 12, 16 slots: 28.5 / 24.5 and
+// 25.2 / 30.0).  A cluster has 2 (K + 1) CTAs, so the crossover moves with K too;
+// the rule goes by the length alone and is on the slower side for hundreds of
+// slots at ln 6 and for 9 to 16 slots at ln 12 with K = 3.
 static int resident_slots(int ln)
 {
 	return (ln <= 10) ? 1 << 30 : (ln == 11) ? 32 : (ln == 12) ? 16 : 0;
@@ -1532,9 +1541,9 @@ int ab_batch_create(int device, const ab_params * cls, int capacity, int max_ste
 		b->n = (size_t)1 << cls->ln;
 		b->w_ntt = (size_t)(cls->K + 1) * b->n; b->w_norm = (size_t)AB_NW * b->n;
 		CK(cudaSetDevice(device));
-		// smaller classes at higher stream priority: their chunks are chains of
-		// short, latency-bound launches, which otherwise queue behind the large
-		// grids of the big classes sharing the GPU
+		// smaller classes at higher stream priority: their chunks (one launch of a
+		// few clusters, or a chain of short, latency-bound launches) otherwise queue
+		// behind the large grids of the big classes sharing the GPU
 		int least = 0, greatest = 0;
 		CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
 		const int prio = std::min(least, greatest + std::max(0, cls->ln - 12));

@@ -41,7 +41,7 @@ namespace ab
 // Bound by the integer multiplier (about 370 units of one IMAD per coefficient
 // of 6 primes, 10.4 us at 33.2M bits) and by latency: half of the pass is its
 // last stage, whose lines are touched ahead (rp_touch).  33.2M bits, multiply:
-// 34.8 -> 27.5 us.  8 words per thread with the row's twiddles in shared memory
+// 33.8 -> 26.6 us.  8 words per thread with the row's twiddles in shared memory
 // measured slower (33.2M bits 171 -> 177 us per squaring): more stages, more
 // shared-memory traffic.
 constexpr int RP_EPT = 16;
